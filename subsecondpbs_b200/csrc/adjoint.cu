@@ -226,7 +226,7 @@ struct AdjShape {
 // accumulators) and waits for the previous instance before it exits.
 template <int RLo, int RHi, int MinBlocks>
 __global__ void __launch_bounds__(kAdjThreads, MinBlocks)
-superpose_adjoint_kernel(BeamGeomDev g, const float* __restrict__ idd, const float* __restrict__ rsig,
+superpose_adjoint_kernel(BeamGeomDev g, const float2* __restrict__ sources,
                          const int4* __restrict__ work, BeamStateDev* __restrict__ beam, const float* __restrict__ gradBev,
                          float* __restrict__ rbar, int range) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -253,7 +253,7 @@ superpose_adjoint_kernel(BeamGeomDev g, const float* __restrict__ idd, const flo
         if (c >= sBlocks.total) break;
         if (t == 0) sItem[buf ^ 1] = atomicAdd(counter, 1);
         const int4 it = work[block_slot<RLo, RHi>(sBlocks, c)];
-        const int lc = it.x & 0xff, tile = it.y, zRel = it.z, R = it.w;
+        const int lc = (it.w >> 8) + __ffs(it.x) - 1, tile = it.y, zRel = it.z, R = it.w & 0xff;
         const int tx = tile % g.tilesX, ty = tile / g.tilesX;
         const int Ho = kTileY + 2 * R, Wo = kTileX + 2 * R;
         const float* src = gradBev + static_cast<size_t>(zRel) * bevPlane +
@@ -265,11 +265,12 @@ superpose_adjoint_kernel(BeamGeomDev g, const float* __restrict__ idd, const flo
         __syncthreads();
         const int sy = t >> 5, sx = t & 31;
         const int ry = ty * kTileY + sy, rx = tx * kTileX + sx;
-        const size_t s = lc * layerStride + zRel * padPlane + static_cast<size_t>(ry) * g.pitchX + rx;
-        const float dose = idd[s];
+        const size_t s = lc * layerStride + zRel * padPlane + static_cast<size_t>(tile) * kTileSources + t;
+        const float2 source = sources[s];
+        const float dose = source.x;
         const bool live = dose > 0.0f && ry < g.rayY && rx < g.rayX;
         if (R >= RLo && R <= RHi)
-            adjoint_dispatch<RLo, RHi>(R, tileG, eS + t * kAdjEStride, E4, P, dose, live ? rsig[s] : 0.0f,
+            adjoint_dispatch<RLo, RHi>(R, tileG, eS + t * kAdjEStride, E4, P, dose, live ? source.y : 0.0f,
                                        live ? rbar + lc * rayPlane + static_cast<size_t>(ry) * g.rayX + rx : nullptr,
                                        sy, sx);
         // Every thread is past the item (and has read sItem[buf]) before the next
@@ -281,7 +282,7 @@ superpose_adjoint_kernel(BeamGeomDev g, const float* __restrict__ idd, const flo
 }
 
 template <int RLo, int RHi, int MinBlocks>
-cudaError_t launch_adjoint_range(const BeamGeomDev& g, const float* idd, const float* rsigma, const int4* work,
+cudaError_t launch_adjoint_range(const BeamGeomDev& g, const float2* sources, const int4* work,
                                  BeamStateDev* beam, const float* gradBev, float* rbar, int numSMs, int range,
                                  bool overlap, cudaStream_t s) {
     auto k = superpose_adjoint_kernel<RLo, RHi, MinBlocks>;
@@ -298,7 +299,7 @@ cudaError_t launch_adjoint_range(const BeamGeomDev& g, const float* idd, const f
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = overlap ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k, g, idd, rsigma, work, beam, gradBev, rbar, range);
+    return cudaLaunchKernelEx(&cfg, k, g, sources, work, beam, gradBev, rbar, range);
 }
 
 // Resident CTAs per SM of the adjoint instances (radii 16..32, 8..15, 0..7).
@@ -318,18 +319,18 @@ cudaError_t launch_transfer_adjoint(const BeamGeomDev& g, const double* gradDose
     return cudaGetLastError();
 }
 
-cudaError_t launch_superpose_adjoint(const BeamGeomDev& g, const float* idd, const float* rsigma, const int4* work,
+cudaError_t launch_superpose_adjoint(const BeamGeomDev& g, const float2* sources, const int4* work,
                                      BeamStateDev* beam, const float* gradBev, float* rbar, int numSMs,
                                      cudaStream_t s) {
     cudaError_t e = launch_one_layer_list_view(beam, s);
     if (e != cudaSuccess) return e;
-    e = launch_adjoint_range<kSplitR + 1, kMaxR, kAdjWideBlocks>(g, idd, rsigma, work, beam, gradBev, rbar, numSMs,
+    e = launch_adjoint_range<kSplitR + 1, kMaxR, kAdjWideBlocks>(g, sources, work, beam, gradBev, rbar, numSMs,
                                                                  0, false, s);
     if (e != cudaSuccess) return e;
-    e = launch_adjoint_range<kSplitR2 + 1, kSplitR, kAdjMidBlocks>(g, idd, rsigma, work, beam, gradBev, rbar, numSMs,
+    e = launch_adjoint_range<kSplitR2 + 1, kSplitR, kAdjMidBlocks>(g, sources, work, beam, gradBev, rbar, numSMs,
                                                                    1, true, s);
     if (e != cudaSuccess) return e;
-    return launch_adjoint_range<0, kSplitR2, kAdjNarrowBlocks>(g, idd, rsigma, work, beam, gradBev, rbar, numSMs, 2,
+    return launch_adjoint_range<0, kSplitR2, kAdjNarrowBlocks>(g, sources, work, beam, gradBev, rbar, numSMs, 2,
                                                                true, s);
 }
 

@@ -50,10 +50,10 @@ __device__ __forceinline__ float step_let(const BioDev& m, float row, float weq)
 // One chunk of layers: out = idd * factor of `channel` at every computed step
 // (channel 0: alpha (LQ) or z1D (MKM), 1: sqrt(beta) (LQ), 2: LET).
 __global__ void __launch_bounds__(256)
-bio_channel_kernel(BeamGeomDev g, BioDev m, int layer0, int nLayers, const float* __restrict__ idd,
+bio_channel_kernel(BeamGeomDev g, BioDev m, int layer0, int nLayers, const float2* __restrict__ sources,
                    const float* __restrict__ wepl, const LayerStateDev* __restrict__ ls,
                    const BeamStateDev* __restrict__ beam, const float* __restrict__ layerRow, int channel,
-                   float* __restrict__ out) {
+                   float2* __restrict__ out) {
     const size_t padPlane = static_cast<size_t>(g.pitchX) * g.pitchY;
     const size_t layerStride = static_cast<size_t>(g.steps) * padPlane;
     const size_t rayPlane = static_cast<size_t>(g.rayX) * g.rayY;
@@ -64,12 +64,15 @@ bio_channel_kernel(BeamGeomDev g, BioDev m, int layer0, int nLayers, const float
         const size_t r = i - size_t(lc) * layerStride;
         const int zr = int(r / padPlane);
         const size_t p = r - size_t(zr) * padPlane;
-        const int y = int(p / g.pitchX), x = int(p - size_t(y) * g.pitchX);
+        const int tile = int(p) / kTileSources, src = int(p) % kTileSources;
+        const int y = tile / g.tilesX * kTileY + src / kTileX, x = tile % g.tilesX * kTileX + src % kTileX;
         const int l = layer0 + lc;
         const int k = first + zr;
-        float v = 0.0f;
+        float2 v = make_float2(0.0f, 0.0f);
         if (k < ls[l].afterLast && x < g.rayX && y < g.rayY) {
-            const float d = idd[i];
+            v = sources[i];
+            const float d = v.x;
+            v.x = 0.0f;
             if (d > 0.0f) {
                 const float weq = wepl[static_cast<size_t>(k) * rayPlane + static_cast<size_t>(y) * g.rayX + x];
                 const float let = step_let(m, layerRow[l], weq);
@@ -81,7 +84,7 @@ bio_channel_kernel(BeamGeomDev g, BioDev m, int layer0, int nLayers, const float
                     else
                         f = channel == 0 ? table_at(m.alpha, m.nLq, li) : sqrtf(fmaxf(table_at(m.beta, m.nLq, li), 0.0f));
                 }
-                v = d * f;
+                v.x = d * f;
             }
         }
         out[i] = v;
@@ -135,12 +138,12 @@ __global__ void bio_map_kernel(const double* __restrict__ dose, const double* __
 
 }  // namespace
 
-cudaError_t launch_bio_channel(const BeamGeomDev& g, const BioDev& m, int layer0, int nLayers, const float* idd,
+cudaError_t launch_bio_channel(const BeamGeomDev& g, const BioDev& m, int layer0, int nLayers, const float2* sources,
                                const float* wepl, const LayerStateDev* ls, const BeamStateDev* beam,
-                               const float* layerRow, int channel, float* out, cudaStream_t s) {
+                               const float* layerRow, int channel, float2* out, cudaStream_t s) {
     const size_t total = static_cast<size_t>(nLayers) * g.steps * g.pitchX * g.pitchY;
     const int blocks = int(std::min<size_t>((total + 255) / 256, 148 * 16));
-    bio_channel_kernel<<<blocks, 256, 0, s>>>(g, m, layer0, nLayers, idd, wepl, ls, beam, layerRow, channel, out);
+    bio_channel_kernel<<<blocks, 256, 0, s>>>(g, m, layer0, nLayers, sources, wepl, ls, beam, layerRow, channel, out);
     return cudaGetLastError();
 }
 

@@ -89,9 +89,9 @@ Context::~Context() {
     cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
     for (DevBuf* b : {&cidd, &density, &sp, &rrl, &ct, &ctQuad, &dose64, &dens, &wepl, &weplMin, &rayW, &interm, &lattice,
-                      &iddBuf, &rsBuf, &bev, &cpb, &subspots, &floatOut, &firstIn, &firstOut, &firstPassive, &codes,
-                      &work, &lp, &ls, &bs, &stats, &nucWeight, &nucSqSigma, &rayToNuc, &nucIddBuf, &nucRsBuf,
-                      &nucCodes, &nucWork, &nucBev, &bevFixed, &nucLs, &nucBs, &errWord, &gradDoseBuf, &bevGrad, &rbarBuf,
+                      &sources, &bev, &cpb, &subspots, &floatOut, &firstIn, &firstOut, &firstPassive, &codes, &tileRange,
+                      &work, &lp, &ls, &bs, &stats, &nucWeight, &nucSqSigma, &rayToNuc, &nucSources,
+                      &nucCodes, &nucRange, &nucWork, &nucBev, &bevFixed, &nucLs, &nucBs, &errWord, &gradDoseBuf, &bevGrad, &rbarBuf,
                       &gradInterm, &gradLattice, &weqBody, &opColPtr, &opBlockOff, &opRows, &opVals})
         b->release();
     staging.release();
@@ -743,8 +743,9 @@ BeamBuffers beam_buffers(const BeamPlan& P, size_t nSubspotData, int nuclear, lo
     z.rayW = L * rays * 4;
     z.bev = S * (pitchX + 2 * kMaxR) * (pitchY + 2 * kMaxR) * 4;
     z.codes = chunk * S * tiles;
+    z.range = chunk * S * tiles * sizeof(unsigned);
     z.work = chunk * S * tiles * sizeof(int4);
-    z.idd = z.rs = chunk * S * padPlane * 4;
+    z.sources = chunk * S * padPlane * sizeof(float2);
     z.firstPassive = chunk * rays * 4;
     z.lp = L * sizeof(LayerParamsDev);
     z.ls = L * sizeof(LayerStateDev);
@@ -761,8 +762,9 @@ BeamBuffers beam_buffers(const BeamPlan& P, size_t nSubspotData, int nuclear, lo
         const size_t nucY = (size_t(P.lattice.ny) + kTileY - 1) / kTileY * kTileY;
         const size_t nucPlane = nucX * nucY, nucTiles = nucPlane / (kTileX * kTileY);
         z.rayToNuc = rays * 4;
-        z.nucIdd = z.nucRs = chunk * S * nucPlane * 4;
+        z.nucSources = chunk * S * nucPlane * sizeof(float2);
         z.nucCodes = chunk * S * nucTiles;
+        z.nucRange = chunk * S * nucTiles * sizeof(unsigned);
         z.nucWork = chunk * S * nucTiles * sizeof(int4);
         z.nucBev = S * (nucX + 2 * kMaxR) * (nucY + 2 * kMaxR) * 4;
         z.nucLs = L * sizeof(LayerStateDev);
@@ -773,9 +775,9 @@ BeamBuffers beam_buffers(const BeamPlan& P, size_t nSubspotData, int nuclear, lo
 }
 
 size_t BeamBuffers::total(bool withTrace) const {
-    return (withTrace ? dens + wepl + weplMin + firstIn + firstOut : 0) + rayW + bev + codes + work + idd + rs +
-           firstPassive + lp + ls + bs + lattice + interm + subspots + cpb + rayToNuc + nucIdd + nucRs + nucCodes +
-           nucWork + nucBev + nucLs + nucBs + bevFixed;
+    return (withTrace ? dens + wepl + weplMin + firstIn + firstOut : 0) + rayW + bev + codes + range + work + sources +
+           firstPassive + lp + ls + bs + lattice + interm + subspots + cpb + rayToNuc + nucSources + nucCodes +
+           nucRange + nucWork + nucBev + nucLs + nucBs + bevFixed;
 }
 
 size_t trace_bytes(size_t steps, size_t rays) {
@@ -786,9 +788,9 @@ size_t trace_bytes(size_t steps, size_t rays) {
 
 void Context::use_stream_ordered_allocation() {
     for (DevBuf* b : {&cidd, &density, &sp, &rrl, &ct, &ctQuad, &dose64, &dens, &wepl, &weplMin, &rayW, &interm, &lattice,
-                      &iddBuf, &rsBuf, &bev, &cpb, &subspots, &floatOut, &firstIn, &firstOut, &firstPassive, &codes,
-                      &work, &lp, &ls, &bs, &stats, &nucWeight, &nucSqSigma, &rayToNuc, &nucIddBuf, &nucRsBuf,
-                      &nucCodes, &nucWork, &nucBev, &bevFixed, &nucLs, &nucBs, &gradDoseBuf, &bevGrad, &rbarBuf, &gradInterm,
+                      &sources, &bev, &cpb, &subspots, &floatOut, &firstIn, &firstOut, &firstPassive, &codes, &tileRange,
+                      &work, &lp, &ls, &bs, &stats, &nucWeight, &nucSqSigma, &rayToNuc, &nucSources,
+                      &nucCodes, &nucRange, &nucWork, &nucBev, &bevFixed, &nucLs, &nucBs, &gradDoseBuf, &bevGrad, &rbarBuf, &gradInterm,
                       &gradLattice, &weqBody, &opColPtr, &opBlockOff, &opRows, &opVals})
         if (!b->ptr) b->allocStream = stream;
 }
@@ -796,9 +798,9 @@ void Context::use_stream_ordered_allocation() {
 size_t Context::device_bytes() const {
     size_t n = 0;
     for (const DevBuf* b : {&cidd, &density, &sp, &rrl, &ct, &ctQuad, &dose64, &dens, &wepl, &weplMin, &rayW, &interm, &lattice,
-                            &iddBuf, &rsBuf, &bev, &cpb, &subspots, &floatOut, &firstIn, &firstOut, &firstPassive,
-                            &codes, &work, &lp, &ls, &bs, &stats, &nucWeight, &nucSqSigma, &rayToNuc, &nucIddBuf,
-                            &nucRsBuf, &nucCodes, &nucWork, &nucBev, &bevFixed, &nucLs, &nucBs, &errWord, &gradDoseBuf, &bevGrad,
+                            &sources, &bev, &cpb, &subspots, &floatOut, &firstIn, &firstOut, &firstPassive,
+                            &codes, &tileRange, &work, &lp, &ls, &bs, &stats, &nucWeight, &nucSqSigma, &rayToNuc, &nucSources,
+                            &nucCodes, &nucRange, &nucWork, &nucBev, &bevFixed, &nucLs, &nucBs, &errWord, &gradDoseBuf, &bevGrad,
                             &rbarBuf, &gradInterm, &gradLattice, &weqBody, &opColPtr, &opBlockOff, &opRows, &opVals,
                             &opNorm, &opVoxels, &colBev, &colFixed, &colDose})
         n += b->bytes;
@@ -807,9 +809,9 @@ size_t Context::device_bytes() const {
 
 void Context::release_beam_buffers() {
     join_side_work();
-    for (DevBuf* b : {&dens, &wepl, &weplMin, &rayW, &interm, &lattice, &iddBuf, &rsBuf, &bev, &cpb, &subspots,
-                      &floatOut, &firstIn, &firstOut, &firstPassive, &codes, &work, &rayToNuc, &nucIddBuf, &nucRsBuf,
-                      &nucCodes, &nucWork, &nucBev, &bevFixed, &gradDoseBuf, &bevGrad, &rbarBuf, &gradInterm, &gradLattice, &dose64,
+    for (DevBuf* b : {&dens, &wepl, &weplMin, &rayW, &interm, &lattice, &sources, &bev, &cpb, &subspots,
+                      &floatOut, &firstIn, &firstOut, &firstPassive, &codes, &tileRange, &work, &rayToNuc, &nucSources,
+                      &nucCodes, &nucRange, &nucWork, &nucBev, &bevFixed, &gradDoseBuf, &bevGrad, &rbarBuf, &gradInterm, &gradLattice, &dose64,
                       &weqBody, &opColPtr, &opBlockOff, &opRows, &opVals, &opNorm, &opVoxels, &colBev, &colFixed,
                       &colDose})
         b->release();
@@ -945,6 +947,7 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
     g.doseY = doseGrid.dims[1];
     g.doseZ = doseGrid.dims[2];
     g.compatBevZShift = compatBevZShift;
+    g.fillDeadTiles = keepDebug;
     g.errWord = static_cast<int*>(errWord.ptr);
     // Transport constants (idd_sigma.cu:102-121) and the nuclear halo grid.
     g.eRefSq = 198.81f;
@@ -1056,14 +1059,15 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
         trace.weplMin = static_cast<float*>(weplMin.ptr);
     }
     if ((rc = rayW.ensure(z.rayW)) || (rc = bev.ensure(z.bev)) || (rc = codes.ensure(z.codes)) ||
-        (rc = work.ensure(z.work)) || (rc = iddBuf.ensure(z.idd)) || (rc = rsBuf.ensure(z.rs)) ||
+        (rc = tileRange.ensure(z.range)) ||
+        (rc = work.ensure(z.work)) || (rc = sources.ensure(z.sources)) ||
         (rc = firstPassive.ensure(z.firstPassive)) || (rc = lp.ensure(z.lp)) || (rc = ls.ensure(z.ls)) ||
         (rc = bs.ensure(z.bs)))
         return rc;
     const size_t nucPlane = size_t(g.nucX) * g.nucY, nucTiles = nucPlane / (kTileX * kTileY);
     if (nuclear &&
-        ((rc = rayToNuc.ensure(z.rayToNuc)) || (rc = nucIddBuf.ensure(z.nucIdd)) || (rc = nucRsBuf.ensure(z.nucRs)) ||
-         (rc = nucCodes.ensure(z.nucCodes)) || (rc = nucWork.ensure(z.nucWork)) || (rc = nucBev.ensure(z.nucBev)) ||
+        ((rc = rayToNuc.ensure(z.rayToNuc)) || (rc = nucSources.ensure(z.nucSources)) ||
+         (rc = nucCodes.ensure(z.nucCodes)) || (rc = nucRange.ensure(z.nucRange)) || (rc = nucWork.ensure(z.nucWork)) || (rc = nucBev.ensure(z.nucBev)) ||
          (rc = nucLs.ensure(z.nucLs)) || (rc = nucBs.ensure(z.nucBs))))
         return rc;
     if (!adj) {
@@ -1106,7 +1110,7 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
                                                       b.energies[l]);
         const size_t bevN = S * size_t(g.bevX) * g.bevY;
         const int nCh = bioModel == PBS_BIO_LQ ? 3 : 2;
-        if ((rc = bioLayerRow.ensure(size_t(L) * 4)) || (rc = bioIdd.ensure(z.idd)) ||
+        if ((rc = bioLayerRow.ensure(size_t(L) * 4)) || (rc = bioSources.ensure(z.sources)) ||
             (rc = bioBev.ensure(size_t(nCh) * bevN * 4)))
             return rc;
         if ((rc = upload(bioLayerRow.ptr, rows.data(), size_t(L) * 4))) return rc;
@@ -1287,8 +1291,10 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
     if (smCount <= 0) PBS_CUDA(cudaDeviceGetAttribute(&smCount, cudaDevAttrMultiProcessorCount, device), "SM count");
     const int workCap = int(size_t(chunk) * S * tiles);
     const int nucWorkCap = int(size_t(chunk) * S * nucTiles);
-    float* dNucIdd = static_cast<float*>(nucIddBuf.ptr);
-    float* dNucRs = static_cast<float*>(nucRsBuf.ptr);
+    float2* dSources = static_cast<float2*>(sources.ptr);
+    float2* dNucSources = static_cast<float2*>(nucSources.ptr);
+    unsigned* dRange = static_cast<unsigned*>(tileRange.ptr);
+    unsigned* dNucRange = static_cast<unsigned*>(nucRange.ptr);
     LayerStateDev* dNucLs = static_cast<LayerStateDev*>(nucLs.ptr);
     BeamStateDev* dNucBs = static_cast<BeamStateDev*>(nucBs.ptr);
     if ((rc = join_side_work())) return rc;
@@ -1344,12 +1350,11 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
     };
     for (int l0 = 0; l0 < L; l0 += chunk) {
         const int nl = std::min(chunk, L - l0);
-        if (nuclear) PBS_CUDA(launch_nuc_prepare(nucGeom, nl, dNucIdd, dNucRs, stream), "nuc_prepare");
+        if (nuclear) PBS_CUDA(launch_nuc_prepare(nucGeom, nl, dNucSources, stream), "nuc_prepare");
         PBS_CUDA(launch_idd(g, luts, l0, nl, dDens, dWepl, dFi, dFo, dRayW, dlp, dls, dbs,
-                            static_cast<float*>(iddBuf.ptr), static_cast<float*>(rsBuf.ptr),
-                            static_cast<uint8_t*>(codes.ptr), static_cast<int*>(firstPassive.ptr),
-                            static_cast<const int*>(rayToNuc.ptr), static_cast<const float*>(lattice.ptr), dNucIdd,
-                            dNucRs, stream),
+                            dSources, dRange, static_cast<uint8_t*>(codes.ptr), static_cast<int*>(firstPassive.ptr),
+                            static_cast<const int*>(rayToNuc.ptr), static_cast<const float*>(lattice.ptr), dNucSources,
+                            stream),
                  "idd");
         if (l0 == 0 && (rc = mark(4))) return rc;
         PBS_CUDA(launch_bin_plan(g, l0, nl, static_cast<const uint8_t*>(codes.ptr), dls, dbs,
@@ -1357,7 +1362,7 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
                                  nullptr, stream),
                  "bin_plan");
         if (nuclear) {
-            PBS_CUDA(launch_nuc_codes(nucGeom, l0, nl, dNucIdd, dNucRs, dls, dbs, dNucLs,
+            PBS_CUDA(launch_nuc_codes(nucGeom, l0, nl, dNucSources, dls, dbs, dNucLs, dNucRange,
                                       static_cast<uint8_t*>(nucCodes.ptr), stream),
                      "nuc_codes");
             PBS_CUDA(launch_bin_plan(nucGeom, l0, nl, static_cast<const uint8_t*>(nucCodes.ptr), dNucLs, dNucBs,
@@ -1373,9 +1378,8 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
             // compacts the columns, then the volumes' live cells are cleared.
             float* cBev = static_cast<float*>(colBev.ptr);
             unsigned long long* cFixed = static_cast<unsigned long long*>(colFixed.ptr);
-            PBS_CUDA(launch_superpose_columns(g, static_cast<const float*>(iddBuf.ptr),
-                                              static_cast<const float*>(rsBuf.ptr), static_cast<const int4*>(work.ptr),
-                                              dbs, dls + l0, nl, cBev, cFixed, colCells, smCount, stream),
+            PBS_CUDA(launch_superpose_columns(g, dSources, dRange, static_cast<const int4*>(work.ptr), dbs, dls + l0, nl,
+                                              cBev, cFixed, colCells, smCount, stream),
                      "superpose_columns");
             PBS_CUDA(launch_column_transfer(g, cBev, colCells, dbs, dls + l0, nl, colBox,
                                             static_cast<double*>(colDose.ptr), stream),
@@ -1385,11 +1389,11 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
             continue;
         }
         bevFixedClean = false;
-        PBS_CUDA(launch_superpose(g, static_cast<const float*>(iddBuf.ptr), static_cast<const float*>(rsBuf.ptr),
-                                  static_cast<const int4*>(work.ptr), dbs, dBev, dFixed, 0, smCount, stream),
+        PBS_CUDA(launch_superpose(g, dSources, dRange, static_cast<const int4*>(work.ptr), dbs, dBev, dFixed, 0, smCount,
+                                  stream),
                  "superpose");
         if (nuclear)
-            PBS_CUDA(launch_superpose(nucGeom, dNucIdd, dNucRs, static_cast<const int4*>(nucWork.ptr), dNucBs,
+            PBS_CUDA(launch_superpose(nucGeom, dNucSources, dNucRange, static_cast<const int4*>(nucWork.ptr), dNucBs,
                                       static_cast<float*>(nucBev.ptr), dFixed, 0, smCount, stream),
                      "nuc_superpose");
         if (bio) {
@@ -1400,14 +1404,14 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
             int slot = 0;
             for (int c : channels) {
                 if (c == 1 && bioModel != PBS_BIO_LQ) continue;
-                PBS_CUDA(launch_bio_channel(g, bioDev, l0, nl, static_cast<const float*>(iddBuf.ptr), dWepl, dls, dbs,
+                PBS_CUDA(launch_bio_channel(g, bioDev, l0, nl, dSources, dWepl, dls, dbs,
                                             static_cast<const float*>(bioLayerRow.ptr), c,
-                                            static_cast<float*>(bioIdd.ptr), stream),
+                                            static_cast<float2*>(bioSources.ptr), stream),
                          "bio_channel");
                 PBS_CUDA(launch_reset_work_claims(dbs, stream), "reset work claims");
-                PBS_CUDA(launch_superpose(g, static_cast<const float*>(bioIdd.ptr),
-                                          static_cast<const float*>(rsBuf.ptr), static_cast<const int4*>(work.ptr),
-                                          dbs, static_cast<float*>(bioBev.ptr) + size_t(slot) * bevN, dFixed,
+                PBS_CUDA(launch_superpose(g, static_cast<const float2*>(bioSources.ptr), dRange,
+                                          static_cast<const int4*>(work.ptr), dbs,
+                                          static_cast<float*>(bioBev.ptr) + size_t(slot) * bevN, dFixed,
                                           bioShiftOffset[c], smCount, stream),
                          "bio_superpose");
                 ++slot;
@@ -1473,7 +1477,7 @@ int Context::finish_adjoint(const AdjointArgs& a, const PbsBeamDesc& b) {
     PBS_CUDA(cudaMemsetAsync(bevGrad.ptr, 0, bevN * 4, stream), "memset");
     PBS_CUDA(cudaMemsetAsync(rbarBuf.ptr, 0, L * rays * 4, stream), "memset");
     PBS_CUDA(launch_transfer_adjoint(g, a.gradDose, dbs, static_cast<float*>(bevGrad.ptr), stream), "transfer_adjoint");
-    PBS_CUDA(launch_superpose_adjoint(g, static_cast<const float*>(iddBuf.ptr), static_cast<const float*>(rsBuf.ptr),
+    PBS_CUDA(launch_superpose_adjoint(g, static_cast<const float2*>(sources.ptr),
                                       static_cast<const int4*>(work.ptr), dbs, static_cast<const float*>(bevGrad.ptr),
                                       static_cast<float*>(rbarBuf.ptr), smCount, stream),
              "superpose_adjoint");
@@ -1626,6 +1630,17 @@ int Context::stage_times(float* ms, int n) {
     return PBS_OK;
 }
 
+// One component of tile-major source planes (0: IDD, 1: rSigma) as plain [y][x] planes.
+static void untile_planes(const float2* tiled, int component, size_t planes, int nx, int ny, float* out) {
+    for (size_t z = 0; z < planes; ++z, tiled += size_t(nx) * ny)
+        for (int y = 0; y < ny; ++y)
+            for (int x = 0; x < nx; ++x) {
+                const float2 v = tiled[(size_t(y / kTileY) * (nx / kTileX) + x / kTileX) * kTileSources +
+                                       (y % kTileY) * kTileX + x % kTileX];
+                *out++ = component ? v.y : v.x;
+            }
+}
+
 int Context::debug_copy(int which, int layer, void* out, size_t bytes) {
     PBS_CUDA(cudaSetDevice(device), "cudaSetDevice");
     if (!lastBeamValid) {
@@ -1703,11 +1718,11 @@ int Context::debug_copy(int which, int layer, void* out, size_t bytes) {
             const float fill = which == PBS_DBG_IDD ? 0.0f : __builtin_inff();
             std::fill(o, o + S * padPlane, fill);
             const int nz = std::max(0, lh.afterLast - first);
-            const char* src = static_cast<const char*>(which == PBS_DBG_IDD ? iddBuf.ptr : rsBuf.ptr) +
-                              size_t(layer) * S * padPlane * 4;
-            if (nz > 0)
-                PBS_CUDA(cudaMemcpy(o + size_t(first) * padPlane, src, size_t(nz) * padPlane * 4, cudaMemcpyDeviceToHost),
-                         "debug D2H");
+            const float2* src = static_cast<const float2*>(sources.ptr) + size_t(layer) * S * padPlane;
+            std::vector<float2> tiled(size_t(nz) * padPlane);
+            PBS_CUDA(cudaMemcpy(tiled.data(), src, tiled.size() * sizeof(float2), cudaMemcpyDeviceToHost), "debug D2H");
+            untile_planes(tiled.data(), which == PBS_DBG_RSIGMA, size_t(nz), geom.pitchX, geom.pitchY,
+                          o + size_t(first) * padPlane);
             return PBS_OK;
         }
         case PBS_DBG_TILE_BINS: {
@@ -1763,12 +1778,18 @@ int Context::debug_copy(int which, int layer, void* out, size_t bytes) {
             }
             // The halo is computed over [first, afterLast); its codes over [first, calcPassive).
             const int nz = std::max(0, (bins ? lh.calcPassive : lh.afterLast) - first);
-            const void* srcBase = bins ? nucCodes.ptr : (which == PBS_DBG_NUC_IDD ? nucIddBuf.ptr : nucRsBuf.ptr);
-            const char* src = static_cast<const char*>(srcBase) + size_t(layer) * S * per * elem;
-            if (nz > 0)
-                PBS_CUDA(cudaMemcpy(static_cast<char*>(out) + size_t(first) * per * elem, src, size_t(nz) * per * elem,
+            if (bins) {
+                PBS_CUDA(cudaMemcpy(static_cast<char*>(out) + size_t(first) * per,
+                                    static_cast<const char*>(nucCodes.ptr) + size_t(layer) * S * per, size_t(nz) * per,
                                     cudaMemcpyDeviceToHost),
                          "debug D2H");
+            } else {
+                const float2* src = static_cast<const float2*>(nucSources.ptr) + size_t(layer) * S * per;
+                std::vector<float2> tiled(size_t(nz) * per);
+                PBS_CUDA(cudaMemcpy(tiled.data(), src, tiled.size() * sizeof(float2), cudaMemcpyDeviceToHost), "debug D2H");
+                untile_planes(tiled.data(), which == PBS_DBG_NUC_RSIGMA, size_t(nz), geom.nucX, geom.nucY,
+                              static_cast<float*>(out) + size_t(first) * per);
+            }
             return PBS_OK;
         }
         default:

@@ -37,9 +37,9 @@ struct PinnedBuf {
 // context's buffers grow to the largest beam they have run).
 struct BeamBuffers {
     int chunk = 1;
-    size_t dens = 0, wepl = 0, weplMin = 0, firstIn = 0, firstOut = 0, rayW = 0, bev = 0, codes = 0, work = 0, idd = 0,
-           rs = 0, firstPassive = 0, lp = 0, ls = 0, bs = 0, lattice = 0, interm = 0, subspots = 0, cpb = 0;
-    size_t rayToNuc = 0, nucIdd = 0, nucRs = 0, nucCodes = 0, nucWork = 0, nucBev = 0, nucLs = 0, nucBs = 0;
+    size_t dens = 0, wepl = 0, weplMin = 0, firstIn = 0, firstOut = 0, rayW = 0, bev = 0, codes = 0, range = 0, work = 0,
+           sources = 0, firstPassive = 0, lp = 0, ls = 0, bs = 0, lattice = 0, interm = 0, subspots = 0, cpb = 0;
+    size_t rayToNuc = 0, nucSources = 0, nucCodes = 0, nucRange = 0, nucWork = 0, nucBev = 0, nucLs = 0, nucBs = 0;
     size_t bevFixed = 0;  // int64 accumulator of the larger of the two BEV volumes
     size_t total(bool withTrace = true) const;
 };
@@ -134,7 +134,7 @@ struct Context {
     BioDev bioDev{};
     std::vector<float> bioLetEnergies;
     int bioShiftOffset[3] = {0, 0, 0};  // fixed-point exponent offset of channels 0, 1, 2
-    DevBuf bioTables, bioLayerRow, bioIdd, bioBev, bioAcc;
+    DevBuf bioTables, bioLayerRow, bioSources, bioBev, bioAcc;
     int set_bio_model(const PbsBioModel* m);
     int read_bio_map(int map, float* out, int onDevice);
     int clear_bio();
@@ -158,10 +158,10 @@ struct Context {
     DevBuf dose64;
 
     // Per-beam working set (grow-only).
-    DevBuf dens, wepl, weplMin, rayW, interm, lattice, iddBuf, rsBuf, bev, cpb, subspots, floatOut;
-    DevBuf firstIn, firstOut, firstPassive, codes, work, lp, ls, bs, stats;
+    DevBuf dens, wepl, weplMin, rayW, interm, lattice, sources, bev, cpb, subspots, floatOut;
+    DevBuf firstIn, firstOut, firstPassive, codes, tileRange, work, lp, ls, bs, stats;
     // Nuclear halo working set and the device word collecting error flags.
-    DevBuf rayToNuc, nucIddBuf, nucRsBuf, nucCodes, nucWork, nucBev, nucLs, nucBs, errWord;
+    DevBuf rayToNuc, nucSources, nucCodes, nucRange, nucWork, nucBev, nucLs, nucBs, errWord;
     // Fixed-point superposition accumulator; zero between superpositions unless a
     // run stopped between a superposition and its write-out (bevFixedClean false).
     DevBuf bevFixed;

@@ -35,6 +35,17 @@ __device__ __forceinline__ float float_from_order_key(unsigned k) {
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
+// A tile's range of rSigma as one word: the upper bound in the high half, the lower one
+// in the low half, each the top 16 bits of the positive float below its sign (2^-8
+// relative, rounded outwards); 0 is no depositing source. A depositing source without a
+// valid rSigma > 0 has the smallest upper and the largest lower bound.
+__device__ __forceinline__ unsigned range_hi(float r) { return r > 0.0f ? max((__float_as_uint(r) + 0x7fffu) >> 15, 1u) : 1u; }
+__device__ __forceinline__ unsigned range_lo(float r) { return r > 0.0f ? __float_as_uint(r) >> 15 : 0xffffu; }
+__device__ __forceinline__ unsigned merge_range(unsigned a, unsigned b) {
+    if (!a || !b) return a | b;
+    return max(a >> 16, b >> 16) << 16 | min(a & 0xffffu, b & 0xffffu);
+}
+
 // Same lookup on a table staged in shared memory.
 __device__ __forceinline__ float lut_linear_clamp_smem(const float* t, int n, float x) {
     const float xb = fminf(fmaxf(x - 0.5f, 0.0f), float(n - 1));

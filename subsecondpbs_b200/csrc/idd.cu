@@ -27,9 +27,10 @@ constexpr int kMaxChunkLayers = 64;
 // One CTA = one 32x8 tile of rays for one layer. Each thread walks its ray from the
 // beam's first-inside step to the layer's cut-off step (fillIddAndSigmaKernel,
 // idd_sigma.cu:46-259). After every step each warp reduces min(rSigmaEff) and
-// any(idd > 0) over its 32 rays into shared memory; once the walk is done the CTA
+// the largest rSigmaEff with idd > 0 over its 32 rays into shared memory; once the walk is done the CTA
 // turns the eight warp partials of every step into the tile's radius bucket
-// (tileRadCalc, complete_superposition.cu:198-255), stores the code and adds the
+// (tileRadCalc, complete_superposition.cu:198-255), stores the code and, for a live
+// tile, its range of rSigma (the superposition's interpolation range), and adds the
 // tile's bucket counts to the layer histogram.
 // Profile table value of channel c at a fractional depth and row index, both
 // already clamped to the table: the linear filter of the reference's profile
@@ -52,9 +53,9 @@ __global__ void __launch_bounds__(256)
 idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ density,
            const float* __restrict__ wepl, const int* __restrict__ firstInside, const int* __restrict__ firstOutside,
            const float* __restrict__ rayW, const LayerParamsDev* __restrict__ lp, LayerStateDev* __restrict__ ls,
-           const BeamStateDev* __restrict__ beam, float* __restrict__ iddOut, float* __restrict__ rsigOut,
+           const BeamStateDev* __restrict__ beam, float2* __restrict__ sources, unsigned* __restrict__ tileRange,
            uint8_t* __restrict__ codes, int* __restrict__ firstPassiveOut, const int* __restrict__ rayToNuc,
-           const float* __restrict__ lattice, float* __restrict__ nucIddOut, float* __restrict__ nucRsOut) {
+           const float* __restrict__ lattice, float2* __restrict__ nucSources) {
     extern __shared__ float smem[];
     float* ciddRow = smem;                                    // [nS]
     float* nucWRow = ciddRow + luts.nS;                       // [nS] with the nuclear halo
@@ -63,8 +64,8 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ de
     float* stepNum = rrlTab + luts.nRrl;                      // [steps] 0.5 (voxel width x + y)
     float* stepVolT = stepNum + g.steps;                      // [steps] step volume
     float* partMin = stepVolT + g.steps;                      // [steps][8]
-    int* partLive = reinterpret_cast<int*>(partMin + g.steps * 8);  // [steps][8]
-    __shared__ int shHist[kBuckets], shLive[kBuckets], shPassive[8];
+    unsigned* partRange = reinterpret_cast<unsigned*>(partMin + g.steps * 8);  // [steps][8]
+    __shared__ int shHist[kBuckets], shLive[kBuckets], shPassive[8], shEnd;
 
     // Longest walks first: the layers are dispatched from the end of the chunk whose
     // cut-off step is deeper, so that the long CTAs do not form the grid's tail.
@@ -123,6 +124,7 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ de
             shHist[tid] = 0;
             shLive[tid] = 0;
         }
+        if (tid == 0) shEnd = first;
     }
     __syncthreads();
 
@@ -130,8 +132,8 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ de
     const size_t rayPlane = static_cast<size_t>(g.rayX) * g.rayY;
     const size_t padPlane = static_cast<size_t>(g.pitchX) * g.pitchY;
     const size_t layerStride = static_cast<size_t>(g.steps) * padPlane;
-    float* iddL = iddOut + lc * layerStride;
-    float* rsL = rsigOut + lc * layerStride;
+    // This thread's source of the tile (tile-major planes).
+    float2* srcL = sources + lc * layerStride + static_cast<size_t>(ty * g.tilesX + tx) * kTileSources + tid;
     const size_t ridx = static_cast<size_t>(y) * g.rayX + x;
 
     int firstIn = 0;
@@ -153,16 +155,19 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ de
     // halo lattice cell carry a halo value; the cell's raw spot weight is its
     // weight. Every ray's primary dose keeps the (1 - nuclear weight) share.
     const bool nucOn = kNuclear && p.spotDist > 0.0f;
-    int nucIdx = -1;
+    int nucIdx = -1;  // the cell's source in the halo's tile-major planes
     float nucRayWeight = 0.0f;
     if (nucOn && real) {
-        nucIdx = rayToNuc[ridx];
-        if (nucIdx >= 0)
-            nucRayWeight = lattice[(static_cast<size_t>(l) * g.latNy + nucIdx / g.nucX) * g.latNx + nucIdx % g.nucX];
+        const int cell = rayToNuc[ridx];
+        if (cell >= 0) {
+            const int cx = cell % g.nucX, cy = cell / g.nucX;
+            nucRayWeight = lattice[(static_cast<size_t>(l) * g.latNy + cy) * g.latNx + cx];
+            nucIdx = ((cy / kTileY) * (g.nucX / kTileX) + cx / kTileX) * kTileSources + (cy % kTileY) * kTileX +
+                     cx % kTileX;
+        }
     }
     const size_t nucPlane = static_cast<size_t>(g.nucX) * g.nucY;
-    float* nucIddL = nucIddOut + lc * static_cast<size_t>(g.steps) * nucPlane;
-    float* nucRsL = nucRsOut + lc * static_cast<size_t>(g.steps) * nucPlane;
+    float2* nucL = nucSources + lc * static_cast<size_t>(g.steps) * nucPlane;
     const float spotDist = p.spotDist;
     const float entrySigmaSq = ls[l].entrySigmaSq;
     const float eRefSq = nucOn ? g.eRefSq : 198.81f;
@@ -297,37 +302,37 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ de
         }
         runMax = fmaxf(runMax, res);
         const int zr = stepNo - first;
-        const size_t o = static_cast<size_t>(zr) * padPlane + static_cast<size_t>(y) * g.pitchX + x;
-        iddL[o] = res;
-        rsL[o] = rSigmaEff;
-        if (nucIdx >= 0) {
-            nucIddL[static_cast<size_t>(zr) * nucPlane + nucIdx] = nucRes;
-            nucRsL[static_cast<size_t>(zr) * nucPlane + nucIdx] = nucRSigmaEff;
-        }
+        srcL[static_cast<size_t>(zr) * padPlane] = make_float2(res, rSigmaEff);
+        if (nucIdx >= 0) nucL[static_cast<size_t>(zr) * nucPlane + nucIdx] = make_float2(nucRes, nucRSigmaEff);
 
         // Warp minimum on order-preserving unsigned keys of the floats; the device's
         // canonical NaN maps above +inf and drops out, as it does under fminf.
         const unsigned mk = __reduce_min_sync(0xffffffffu, float_order_key(rSigmaEff));
-        const int anyLive = __any_sync(0xffffffffu, res > 0.0f);
+        // Range of rSigmaEff over the depositing sources. The smallest is the minimum above
+        // unless a ray without dose has a finite value too.
+        const bool deposits = res > 0.0f;
+        const unsigned hi = __reduce_max_sync(0xffffffffu, deposits ? range_hi(rSigmaEff) : 0u);
+        unsigned lo = range_lo(float_from_order_key(mk));
+        if (__any_sync(0xffffffffu, !deposits && rSigmaEff < __int_as_float(0x7f800000)))
+            lo = __reduce_min_sync(0xffffffffu, deposits ? range_lo(rSigmaEff) : 0xffffu);
         if (lane == 0) {
             partMin[zr * 8 + warp] = float_from_order_key(mk);
-            partLive[zr * 8 + warp] = anyLive;
+            partRange[zr * 8 + warp] = hi ? hi << 16 | lo : 0u;
         }
     }
-    // The row's remaining steps: no dose, rSigmaEff = +inf, nothing live.
-    for (int k = stepNo; k < afterLastL; ++k) {
-        const int zr = k - first;
-        const size_t o = static_cast<size_t>(zr) * padPlane + static_cast<size_t>(y) * g.pitchX + x;
-        iddL[o] = 0.0f;
-        rsL[o] = __int_as_float(0x7f800000);
-        if (nucIdx >= 0) {
-            nucIddL[static_cast<size_t>(zr) * nucPlane + nucIdx] = 0.0f;
-            nucRsL[static_cast<size_t>(zr) * nucPlane + nucIdx] = __int_as_float(0x7f800000);
-        }
-    }
+    // The row's remaining steps: no dose, rSigmaEff = +inf, nothing live. Past the tile's
+    // last walked step no tile is live and nothing reads its sources.
+    if (lane == 0) atomicMax(&shEnd, stepNo);
+    __syncthreads();
+    const int fillEnd = g.fillDeadTiles ? afterLastL : shEnd;
+    for (int k = stepNo; k < fillEnd; ++k)
+        srcL[static_cast<size_t>(k - first) * padPlane] = make_float2(0.0f, __int_as_float(0x7f800000));
+    if (nucIdx >= 0)
+        for (int k = stepNo; k < afterLastL; ++k)
+            nucL[static_cast<size_t>(k - first) * nucPlane + nucIdx] = make_float2(0.0f, __int_as_float(0x7f800000));
     for (int zr = stepNo - first + lane; zr < afterLastL - first; zr += 32) {
         partMin[zr * 8 + warp] = __int_as_float(0x7f800000);
-        partLive[zr * 8 + warp] = 0;
+        partRange[zr * 8 + warp] = 0;
     }
 
     {
@@ -346,14 +351,16 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ de
     const int tiles = g.tilesX * g.tilesY;
     for (int zr = tid; zr < nSteps; zr += 256) {
         float tm = partMin[zr * 8];
-        int tl = partLive[zr * 8];
+        unsigned tl = partRange[zr * 8];
 #pragma unroll
         for (int w = 1; w < 8; ++w) {
             tm = fminf(tm, partMin[zr * 8 + w]);
-            tl |= partLive[zr * 8 + w];
+            tl = merge_range(tl, partRange[zr * 8 + w]);
         }
         const int R = tile_radius_bucket(tm);
-        codeL[static_cast<size_t>(zr) * tiles + ty * g.tilesX + tx] = static_cast<uint8_t>(R | (tl ? 0x80 : 0));
+        const size_t ti = static_cast<size_t>(zr) * tiles + ty * g.tilesX + tx;
+        codeL[ti] = static_cast<uint8_t>(R | (tl ? 0x80 : 0));
+        if (tl) tileRange[static_cast<size_t>(lc) * g.steps * tiles + ti] = tl;
         atomicAdd(&shHist[R], 1);
         if (tl) atomicAdd(&shLive[R], 1);
     }
@@ -546,7 +553,7 @@ layer_plan_kernel(BeamGeomDev g, int layer0, int nLayers, LayerStateDev* __restr
 
 // One thread per (layer, step, tile) code of the chunk: live tiles are written to
 // their layer's radius group of the work list as one-layer items in the forward
-// superposition's format (x = the chunk layer in the low byte, 0xff above it). Each
+// superposition's format. Each
 // layer's box of the cells its items can write (LayerStateDev::liveLo/liveHi) is
 // reduced per warp (a warp's 32 consecutive codes span at most a few layers) before
 // its atomics.
@@ -574,7 +581,7 @@ __global__ void work_scatter_kernel(BeamGeomDev g, int layer0, int nLayers, cons
                 R = st.batchedR[c & 0x3f];
                 const int slot = st.offR[R] + atomicAdd(&st.curR[R], 1);
                 if (slot < workCapacity)
-                    work[slot] = make_int4(static_cast<int>(0xffffff00u | static_cast<unsigned>(lc)), tile, zr, R);
+                    work[slot] = make_int4(static_cast<int>(1u << (lc & 31)), tile, zr, R | ((lc & ~31) << 8));
                 key = lc;
             }
         }
@@ -607,22 +614,21 @@ __global__ void work_scatter_kernel(BeamGeomDev g, int layer0, int nLayers, cons
 // (R = 0: up to blockStart[kMaxR + 1], the item count). Merging only joins items of one
 // radius, so the merged items of R fit in the block its unmerged items occupy.
 __device__ __forceinline__ void emit_merged(BeamStateDev* beam, const int* blockStart, int4* work, unsigned layers,
-                                            int tile, int zr, int R) {
+                                            int base, int tile, int zr, int R) {
     const int begin = blockStart[R];
     const int end = R > 0 ? blockStart[R - 1] : blockStart[kMaxR + 1];
     const int slot = begin + atomicAdd(&beam->mergedR[R], 1);
-    if (slot < end) work[slot] = make_int4(static_cast<int>(layers), tile, zr, R);
+    if (slot < end) work[slot] = make_int4(static_cast<int>(layers), tile, zr, R | (base << 8));
 }
 
 // The forward superposition's work list: one warp per (step, tile) of the chunk,
 // a lane per chunk layer (two passes for chunks of more than 32 layers), takes the
 // tile's live items at that step (the same items, radii and step ranges as
-// work_scatter_kernel) and groups the layers with equal batched radius, in layer
-// order, into items of up to kMergeLayers layers (x = the chunk layers as bytes,
-// 0xff: none); radii above kSplitR stay one layer per item. Each item goes to the
-// block of its radius (so the superposition's CTAs run one radius at a time); the
-// order within a block is arbitrary, and the superposition's fixed-point BEV makes
-// the dose independent of it.
+// work_scatter_kernel) and makes one item of all layers with equal batched radius: the
+// superposition's convolutions are done once per item whatever its layers. Each item
+// goes to the block of its radius (so the superposition's warps run one radius at a
+// time); the order within a block is arbitrary, and the superposition's fixed-point BEV
+// makes the dose independent of it.
 __global__ void work_merge_kernel(BeamGeomDev g, int layer0, int nLayers, const uint8_t* __restrict__ codes,
                                   const LayerStateDev* __restrict__ ls, BeamStateDev* __restrict__ beam,
                                   int4* __restrict__ work) {
@@ -654,26 +660,9 @@ __global__ void work_merge_kernel(BeamGeomDev g, int layer0, int nLayers, const 
                 if (zr < st.afterLast - first && (c & 0x80)) R = st.batchedR[c & 0x3f];
             }
             rMax = max(rMax, R);
-            const bool merge = R >= 0 && R <= kSplitR;
-            const unsigned mergeLanes = __ballot_sync(0xffffffffu, merge);
-            if (R > kSplitR) emit_merged(beam, sStart, work, 0xffffff00u | unsigned(lc), tile, zr, R);
-            if (merge) {
-                // Lanes with this radius; every kMergeLayers-th of them (in lane
-                // order) writes the item of itself and the next ones.
-                const unsigned same = __match_any_sync(mergeLanes, R);
-                const unsigned below = (1u << lane) - 1u;
-                const int rank = __popc(same & below);
-                if (rank % kMergeLayers == 0) {
-                    unsigned layers = 0xffffffffu;
-                    unsigned rest = same & ~below;
-                    for (int n = 0; n < kMergeLayers && rest; ++n) {
-                        const int l = __ffs(rest) - 1;
-                        rest &= rest - 1u;
-                        layers = (layers & ~(0xffu << (8 * n))) | (unsigned(base + l) << (8 * n));
-                    }
-                    emit_merged(beam, sStart, work, layers, tile, zr, R);
-                }
-            }
+            // The lanes of one radius are one item; its first lane writes it.
+            const unsigned same = __match_any_sync(0xffffffffu, R);
+            if (R >= 0 && lane == __ffs(same) - 1) emit_merged(beam, sStart, work, same, base, tile, zr, R);
         }
         rMax = __reduce_max_sync(0xffffffffu, rMax);
         if (lane == 0 && rMax >= 0) {
@@ -693,20 +682,18 @@ __global__ void work_merge_kernel(BeamGeomDev g, int layer0, int nLayers, const 
 }
 
 // Halo cells start empty: IDD 0 and rSigmaEff +inf (wrapper.cu:4124-4135).
-__global__ void nuc_fill_kernel(float* __restrict__ idd, float* __restrict__ rs, size_t n) {
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        idd[i] = 0.0f;
-        rs[i] = __int_as_float(0x7f800000);
-    }
+__global__ void nuc_fill_kernel(float2* __restrict__ sources, size_t n) {
+    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
+        sources[i] = make_float2(0.0f, __int_as_float(0x7f800000));
 }
 
 // One warp per (layer, step, halo tile) over [first, calcPassive) of the layer:
 // the tile's radius bucket and liveness (tileRadCalc, complete_superposition.cu:
 // 198-255, on the halo grid), its code, and its count in the halo histogram.
-__global__ void nuc_codes_kernel(BeamGeomDev gn, int layer0, int nLayers, const float* __restrict__ idd,
-                                 const float* __restrict__ rs, const LayerStateDev* __restrict__ primaryLs,
+__global__ void nuc_codes_kernel(BeamGeomDev gn, int layer0, int nLayers, const float2* __restrict__ sources,
+                                 const LayerStateDev* __restrict__ primaryLs,
                                  const BeamStateDev* __restrict__ primaryBeam, LayerStateDev* __restrict__ nucLs,
-                                 uint8_t* __restrict__ codes) {
+                                 unsigned* __restrict__ tileRange, uint8_t* __restrict__ codes) {
     const int lane = threadIdx.x & 31;
     const int tiles = gn.tilesX * gn.tilesY;
     const int first = primaryBeam->firstInside;
@@ -719,29 +706,27 @@ __global__ void nuc_codes_kernel(BeamGeomDev gn, int layer0, int nLayers, const 
         const int rem = int(i - size_t(lc) * perLayer);
         const int zr = rem / tiles, tile = rem - zr * tiles;
         if (zr >= primaryLs[layer0 + lc].calcPassive - first) continue;
-        const int tx = tile % gn.tilesX, ty = tile / gn.tilesX;
-        const float* ti = idd + (lc * static_cast<size_t>(gn.steps) + zr) * plane + size_t(ty * kTileY) * gn.pitchX +
-                          tx * kTileX + lane;
-        const float* tr = rs + (ti - idd);
-        unsigned key = 0xffffffffu;
-        bool live = false;
+        const float2* ti = sources + (lc * static_cast<size_t>(gn.steps) + zr) * plane + size_t(tile) * kTileSources + lane;
+        unsigned key = 0xffffffffu, range = 0;
         float mx = 0.0f;
 #pragma unroll
         for (int r = 0; r < kTileY; ++r) {
-            key = min(key, float_order_key(tr[size_t(r) * gn.pitchX]));
-            const float v = ti[size_t(r) * gn.pitchX];
-            live |= v > 0.0f;
-            mx = fmaxf(mx, v);
+            const float2 v = ti[r * kTileX];
+            key = min(key, float_order_key(v.y));
+            if (v.x > 0.0f) range = merge_range(range, range_hi(v.y) << 16 | range_lo(v.y));
+            mx = fmaxf(mx, v.x);
         }
         key = __reduce_min_sync(0xffffffffu, key);
-        live = __any_sync(0xffffffffu, live);
+        const unsigned hi = __reduce_max_sync(0xffffffffu, range >> 16);
+        const unsigned lo = __reduce_min_sync(0xffffffffu, range ? range & 0xffffu : 0xffffu);
         const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
         if (lane == 0 && mb) atomicMax(&nucLs[layer0 + lc].maxIddBits, mb);
         if (lane == 0) {
             const int R = tile_radius_bucket(float_from_order_key(key));
-            codes[i] = static_cast<uint8_t>(R | (live ? 0x80 : 0));
+            codes[i] = static_cast<uint8_t>(R | (hi ? 0x80 : 0));
+            if (hi) tileRange[i] = hi << 16 | lo;
             atomicAdd(&nucLs[layer0 + lc].histAll[R], 1);
-            if (live) atomicAdd(&nucLs[layer0 + lc].liveHist[R], 1);
+            if (hi) atomicAdd(&nucLs[layer0 + lc].liveHist[R], 1);
         }
     }
 }
@@ -754,27 +739,27 @@ size_t idd_smem_bytes(const BeamGeomDev& g, const LutsDev& luts) {
            static_cast<size_t>(g.steps) * 8 * (sizeof(float) + sizeof(int));
 }
 
-cudaError_t launch_nuc_prepare(const BeamGeomDev& gn, int nLayers, float* idd, float* rsigma, cudaStream_t s) {
+cudaError_t launch_nuc_prepare(const BeamGeomDev& gn, int nLayers, float2* sources, cudaStream_t s) {
     const size_t n = static_cast<size_t>(nLayers) * gn.steps * gn.pitchX * gn.pitchY;
     const int blocks = int(std::min<size_t>((n + 255) / 256, 148 * 16));
-    nuc_fill_kernel<<<blocks, 256, 0, s>>>(idd, rsigma, n);
+    nuc_fill_kernel<<<blocks, 256, 0, s>>>(sources, n);
     return cudaGetLastError();
 }
 
-cudaError_t launch_nuc_codes(const BeamGeomDev& gn, int layer0, int nLayers, const float* idd, const float* rsigma,
+cudaError_t launch_nuc_codes(const BeamGeomDev& gn, int layer0, int nLayers, const float2* sources,
                              const LayerStateDev* primaryLs, const BeamStateDev* primaryBeam, LayerStateDev* nucLs,
-                             uint8_t* codes, cudaStream_t s) {
+                             unsigned* tileRange, uint8_t* codes, cudaStream_t s) {
     const size_t warps = static_cast<size_t>(nLayers) * gn.steps * gn.tilesX * gn.tilesY;
     const int blocks = int(std::min<size_t>((warps + 7) / 8, 148 * 16));
-    nuc_codes_kernel<<<blocks, 256, 0, s>>>(gn, layer0, nLayers, idd, rsigma, primaryLs, primaryBeam, nucLs, codes);
+    nuc_codes_kernel<<<blocks, 256, 0, s>>>(gn, layer0, nLayers, sources, primaryLs, primaryBeam, nucLs, tileRange, codes);
     return cudaGetLastError();
 }
 
 cudaError_t launch_idd(const BeamGeomDev& g, const LutsDev& luts, int layer0, int nLayers, const float* density,
                        const float* wepl, const int* firstInside, const int* firstOutside, const float* rayW,
-                       const LayerParamsDev* lp, LayerStateDev* ls, const BeamStateDev* beam, float* idd,
-                       float* rsigma, uint8_t* codes, int* firstPassive, const int* rayToNuc, const float* lattice,
-                       float* nucIdd, float* nucRsigma, cudaStream_t s) {
+                       const LayerParamsDev* lp, LayerStateDev* ls, const BeamStateDev* beam, float2* sources,
+                       unsigned* tileRange, uint8_t* codes, int* firstPassive, const int* rayToNuc, const float* lattice,
+                       float2* nucSources, cudaStream_t s) {
     dim3 grid(g.tilesX, g.tilesY, nLayers);
     dim3 block(32, 8);
     const size_t smem = idd_smem_bytes(g, luts);
@@ -782,8 +767,8 @@ cudaError_t launch_idd(const BeamGeomDev& g, const LutsDev& luts, int layer0, in
                      : (g.profileMode ? idd_kernel<false, true> : idd_kernel<false, false>);
     cudaError_t e = set_smem_limit(reinterpret_cast<const void*>(k), smem);
     if (e != cudaSuccess) return e;
-    k<<<grid, block, smem, s>>>(g, luts, layer0, density, wepl, firstInside, firstOutside, rayW, lp, ls, beam, idd,
-                                rsigma, codes, firstPassive, rayToNuc, lattice, nucIdd, nucRsigma);
+    k<<<grid, block, smem, s>>>(g, luts, layer0, density, wepl, firstInside, firstOutside, rayW, lp, ls, beam, sources,
+                                tileRange, codes, firstPassive, rayToNuc, lattice, nucSources);
     return cudaGetLastError();
 }
 

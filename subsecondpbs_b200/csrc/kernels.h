@@ -77,16 +77,17 @@ size_t idd_smem_bytes(const BeamGeomDev& g, const LutsDev& luts);
 // halo lattice cell (rayToNuc: [rays] -> cell or -1) into [layer][step][nucY][nucX].
 cudaError_t launch_idd(const BeamGeomDev& g, const LutsDev& luts, int layer0, int nLayers, const float* density,
                        const float* wepl, const int* firstInside, const int* firstOutside, const float* rayW,
-                       const LayerParamsDev* lp, LayerStateDev* ls, const BeamStateDev* beam, float* idd,
-                       float* rsigma, uint8_t* codes, int* firstPassive, const int* rayToNuc, const float* lattice,
-                       float* nucIdd, float* nucRsigma, cudaStream_t s);
+                       const LayerParamsDev* lp, LayerStateDev* ls, const BeamStateDev* beam, float2* sources,
+                       unsigned* tileRange, uint8_t* codes, int* firstPassive, const int* rayToNuc, const float* lattice,
+                       float2* nucSources, cudaStream_t s);
 // Histogram, overflow merge and batching (complete_superposition.cu:358-490) plus
 // the radius-sorted work list of live tiles. With primaryLs/primaryBeam set it
 // plans the nuclear halo grid `g` instead (no merge: a radius above 32 sets error
-// flag 4). `merged` selects the forward superposition's list (items of up to
-// kMergeLayers layers of one tile and step with one radius, x = the layers as bytes)
-// over the one-layer items {layer | 0xffffff00, tile, step, radius} the adjoint
-// gathers from, with each layer's box of live cells.
+// flag 4). A list item is {layers, tile, step, radius | group << 8}: a bit per layer of
+// the group of 32 chunk layers from `group` on. `merged` selects the forward
+// superposition's list (all layers of a group whose tile has one radius at one step)
+// over the one-layer items the adjoint gathers from, with each layer's box of live
+// cells.
 cudaError_t launch_bin_plan(const BeamGeomDev& g, int layer0, int nLayers, const uint8_t* codes, LayerStateDev* ls,
                             BeamStateDev* beam, int4* work, int workCapacity, bool merged,
                             const LayerStateDev* primaryLs, const BeamStateDev* primaryBeam, cudaStream_t s);
@@ -101,17 +102,18 @@ cudaError_t launch_column_bev_clear(const BeamGeomDev& g, float* bev, size_t bev
 // Nuclear halo: clear the chunk's halo IDD (0) and sigma (+inf) before the IDD
 // kernel, and the halo tile codes and histograms after the primary layer plan.
 // `gn` is the halo grid (pitch = nucX x nucY).
-cudaError_t launch_nuc_prepare(const BeamGeomDev& gn, int nLayers, float* idd, float* rsigma, cudaStream_t s);
-cudaError_t launch_nuc_codes(const BeamGeomDev& gn, int layer0, int nLayers, const float* idd, const float* rsigma,
+cudaError_t launch_nuc_prepare(const BeamGeomDev& gn, int nLayers, float2* sources, cudaStream_t s);
+cudaError_t launch_nuc_codes(const BeamGeomDev& gn, int layer0, int nLayers, const float2* sources,
                              const LayerStateDev* primaryLs, const BeamStateDev* primaryBeam, LayerStateDev* nucLs,
-                             uint8_t* codes, cudaStream_t s);
+                             unsigned* tileRange, uint8_t* codes, cudaStream_t s);
 // kernelSuperposition<R> (complete_superposition.cu:264-335) over the work list,
-// summing all layers into one BEV dose: three persistent launches (radii 16..32,
-// 8..15, 0..7) sized for `numSMs` multiprocessors accumulate the chunk in
+// summing all layers into one BEV dose: three persistent launches (radii 24..32,
+// 16..23, 0..15) sized for `numSMs` multiprocessors accumulate the chunk in
 // `bevFixed` (int64 fixed point at 2^(fixedShift + shiftOffset), all zero on entry),
-// and a fifth adds it to the float `bev` and clears it again. Integer adds commute,
+// and a fourth adds it to the float `bev` and clears it again. `sources` holds (idd,
+// rSigma) tile by tile, `tileRange` the range of rSigma of every live tile. Integer adds commute,
 // so the BEV does not depend on the order in which tiles land.
-cudaError_t launch_superpose(const BeamGeomDev& g, const float* idd, const float* rsigma, const int4* work,
+cudaError_t launch_superpose(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange, const int4* work,
                              BeamStateDev* beam, float* bev, unsigned long long* bevFixed, int shiftOffset,
                              int numSMs, cudaStream_t s);
 // Radius blocks and claim counters of the chunk's one-layer work list
@@ -120,8 +122,8 @@ cudaError_t launch_one_layer_list_view(BeamStateDev* beam, cudaStream_t s);
 // Batched influence columns: the chunk's whole one-layer work list (layers
 // [0, nCols) of `ls`), item layer q into BEV volume q (bev / bevFixed + q * stride
 // cells), each volume converted over its layer's live cells.
-cudaError_t launch_superpose_columns(const BeamGeomDev& g, const float* idd, const float* rsigma, const int4* work,
-                                     BeamStateDev* beam, const LayerStateDev* ls, int nCols, float* bev,
+cudaError_t launch_superpose_columns(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange,
+                                     const int4* work, BeamStateDev* beam, const LayerStateDev* ls, int nCols, float* bev,
                                      unsigned long long* bevFixed, size_t stride, int numSMs, cudaStream_t s);
 
 // ---- BEV -> dose ---------------------------------------------------------------
@@ -140,7 +142,7 @@ cudaError_t launch_transfer(const BeamGeomDev& g, const float* bev, const BeamSt
 cudaError_t launch_transfer_adjoint(const BeamGeomDev& g, const double* gradDose, const BeamStateDev* beam,
                                     float* gradBev, cudaStream_t s);
 // S^T and the IDD scaling over the chunk's work list: rbar[l][ray] += idd * (S^T gradBev).
-cudaError_t launch_superpose_adjoint(const BeamGeomDev& g, const float* idd, const float* rsigma, const int4* work,
+cudaError_t launch_superpose_adjoint(const BeamGeomDev& g, const float2* sources, const int4* work,
                                      BeamStateDev* beam, const float* gradBev, float* rbar, int numSMs,
                                      cudaStream_t s);
 // Transposed spot -> ray convolution (mode A): gradLattice[l][iy][ix] from rbar / rayW.
@@ -160,9 +162,9 @@ cudaError_t launch_dose_box(double* dose, float* out, const int dims[3], const i
                             cudaStream_t s);
 
 // Biological maps (bio.cu).
-cudaError_t launch_bio_channel(const BeamGeomDev& g, const BioDev& m, int layer0, int nLayers, const float* idd,
+cudaError_t launch_bio_channel(const BeamGeomDev& g, const BioDev& m, int layer0, int nLayers, const float2* sources,
                                const float* wepl, const LayerStateDev* ls, const BeamStateDev* beam,
-                               const float* layerRow, int channel, float* out, cudaStream_t s);
+                               const float* layerRow, int channel, float2* out, cudaStream_t s);
 cudaError_t launch_bio_map(const double* dose, const double* c0, const double* c1, const double* c2, size_t n,
                            const BioDev& m, int map, float* out, cudaStream_t s);
 // Resets the superposition work list's claim counters so that the list can be run again.

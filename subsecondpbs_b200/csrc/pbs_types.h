@@ -141,6 +141,7 @@ struct BeamGeomDev {
     int bevX, bevY;          // pitch + 64
     int doseX, doseY, doseZ;
     int compatBevZShift;
+    int fillDeadTiles;       // sources of tiles without a live ray are written too (debug readouts)
     // Transport model (idd_sigma.cu:102-121): Highland reference energy, sigma
     // offset and distal-dip suppression; the GAUSS_FIT nuclear model also narrows
     // the entry sigma of the convolution (wrapper.cu:3788-3795).

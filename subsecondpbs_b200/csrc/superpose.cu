@@ -1,565 +1,438 @@
 // Tile-based Gaussian superposition of the per-ray IDD into the padded BEV dose.
 //
 // Each work item is one 32x8 tile of source rays at one step with its batched radius
-// R (kernelSuperposition<R>, complete_superposition.cu:264-335), for one layer or,
-// for R <= kSplitR, for up to kMergeLayers layers whose tile has the same radius at
-// that step (their footprints land on the same BEV cells). Every source s spreads
-// idd_s * e_s(dy) * e_s(dx) over a (2R+1)^2 footprint, where
-// e_s(0) = erf(r/2) and e_s(k) = (erf((k+1/2) r) - erf((k-1/2) r)) / 2.
+// R (kernelSuperposition<R>, complete_superposition.cu:264-335) and a set of layers
+// whose tile has that radius at that step (their footprints land on the same BEV
+// cells). Every source s spreads idd_s * e_s(dy) * e_s(dx) over a (2R+1)^2 footprint.
 //
-// Formulation on the FP32 FMA pipe (one CTA per item, persistent grid):
-//   * table phase (per layer of the item): each thread builds its source's rows
-//     e_s(0..R) (float4 chunks, chunk-major so that the stores and the broadcast
-//     reads are conflict-free) and idd_s * e_s(0..R) (odd row stride); sources
-//     without dose get zero rows;
-//   * accumulation phase: a warp lane is one column distance |d| of one source
-//     column (radii 0..15) or one signed offset (radii 16..32); a source column's
-//     eight sources share the lane's output columns, so the lane keeps the whole
-//     footprint height (8+2R rows) in registers and adds idd_s e_s(|d|) * e_s(k) to
-//     rows sy+R+-k. Up to radius 15 the column at +d, equal to the one at -d, is
-//     accumulated once and added to both: the FMAs and shared loads are
-//     (R+1)/(2R+1) of the direct (2R+1)^2 formulation. Several source columns share
-//     one warp instruction; for radii 16..32 the tile's (column, offset) pairs are
-//     dealt out 32 at a time. A pair ends with one shared-memory add per footprint
-//     row and output column; pairs whose source column has no depositing source are
-//     skipped;
-//   * the footprint accumulates in 32-bit fixed point: a float add to shared memory
-//     has no native instruction on this part (it is a compare-and-swap loop, a
-//     third of the throughput of an integer add), while the integer add is native
-//     and order-independent. Every footprint value and every partial sum of it is at
-//     most the item's total dose (each e_s(k) <= 1 and each source adds to a row of
-//     a pair once), so the power-of-two scale 2^30 / total keeps every sum inside
-//     int32 with a resolution of 2^-30 of the item's dose;
-//   * the footprint of all the item's layers is then added to the BEV dose of its
-//     step (all layers of the beam share one BEV volume) in 64-bit fixed point: a
-//     BEV cell sums many items, and integer adds commute, so the dose does not depend
-//     on the order in which the items land. The chunk's exponent
-//     (layer_plan_kernel) bounds every cell below 2^62; a last pass adds the chunk
-//     to the float BEV and clears it.
-// Up to radius 7 a warp has at most one (column, distance) unit, so its column sums
-// stay in registers over all the item's layers and are flushed once per item.
-// Radii 16..32, 8..15 and 0..7 run as three persistent instances with 128, 48 and
-// 40 registers: 2, 5 and 6 CTAs per SM.
+// One warp takes one item at a time (persistent grid, no CTA barrier):
+//   * range: the item's smallest and largest rSigma, hence its interpolation nodes
+//     (node_spread.cuh: 4 or 6 on most items, 8 at most);
+//   * weights: lane x holds source column x and adds every layer's idd_s L_j(r_s) into
+//     the node weights w_j[sy][x];
+//   * rows: lane = one (node, source row); a transposed FIR filter walks the row once,
+//     two taps per |d|, and overwrites w_j[sy] with its spread T_j[sy][0 .. 32+2R);
+//   * columns: lane = one footprint column (or one half of it: the footprint is
+//     symmetric under y -> H-1-y, sy -> 7-sy, so the halves run the same code); the
+//     column's rows are summed over nodes and source rows in registers, with one
+//     shared-memory load per (node, source row);
+//   * write-out: the rows are added to the BEV dose of the item's step (all layers of
+//     the beam share one BEV volume) in 64-bit fixed point: a BEV cell sums many
+//     items, and integer adds commute, so the dose does not depend on the order in
+//     which the items land. The chunk's exponent (layer_plan_kernel) bounds every cell
+//     below 2^62; a last pass adds the chunk to the float BEV and clears it.
 #include <algorithm>
 
 #include "device_util.cuh"
-#include "work_blocks.cuh"
 #include "kernels.h"
 #include "launch_util.h"
+#include "node_spread.cuh"
+#include "work_blocks.cuh"
 
 namespace pbs {
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kWarps = kThreads / 32;
+constexpr int kSplitWide = 23;  // widest radius of the second instance
 
-// A footprint value q * 2^-sc as a BEV fixed-point value at 2^shift (truncated
-// below the BEV's resolution). q >= 0; the chunk's shift leaves headroom for items
-// of up to kMergeLayers tiles, so the result stays below 2^62.
-__device__ __forceinline__ unsigned long long to_bev_fixed(int q, int sc, int shift) {
-    const int e = shift - sc;
-    if (e >= 0) return static_cast<unsigned long long>(q) << min(e, 62);
-    return e > -63 ? static_cast<unsigned long long>(q) >> (-e) : 0ull;
-}
+// Nodes whose rows a warp holds at a time; 8 nodes go in two halves.
+constexpr int kRowNodes = 6;
+__device__ __forceinline__ int batch_nodes(int count) { return count > kRowNodes ? count / 2 : count; }
 
-// Fixed-point exponent of an item of total dose `total`: 2^(30 - ex) with
-// total < 2^ex, so total * 2^sc < 2^30.
-__device__ __forceinline__ int footprint_exponent(float total) {
-    int ex;
-    frexpf(total, &ex);
-    return min(30 - ex, 126);
-}
-
-// Adds the item's fixed-point footprint [H][Wo] to the BEV.
-template <int H, int Wo>
-__device__ __forceinline__ void write_footprint(const int* __restrict__ out, unsigned long long* __restrict__ dst,
-                                                int bevX, int sc, int shift) {
-    for (int i = threadIdx.x; i < H * Wo; i += kThreads) {
-        const int q = out[i];
-        const int oy = i / Wo, ox = i - oy * Wo;
-        if (q != 0) atomicAdd(dst + static_cast<size_t>(oy) * bevX + ox, to_bev_fixed(q, sc, shift));
-    }
-}
-
-struct ItemArgs {
-    const float* idd;
-    const float* rsig;
-    size_t layerStride;         // IDD elements per chunk layer
-    size_t src;                 // this thread's source ray within a layer
-    unsigned long long* dst;    // footprint origin in the fixed-point BEV dose
-    unsigned layers;            // chunk layers of the item, one per byte (0xff: none)
-    int bevX;
-    int shift;                  // BEV fixed-point exponent
-};
-
-// ============================================================================
-// Radii 0..15: lanes over (source column, |d|) pairs, layer by layer of a merged
-// item into one fixed-point footprint.
-// ============================================================================
-
+// Shared memory of one warp for radii up to RMax: the node tables, then kRowNodes x 4
+// rows of pairs (source rows y and 7 - y of one node, as the two halves of packed FP32
+// operations). Rows and tables have odd strides (in 8 and 16 bytes), so that the lanes
+// of the row pass, one row each, read distinct banks.
+constexpr int kPairs = kTileY / 2;
+template <int R>
+constexpr int kRowStride = kTileX + 2 * R + 1;  // pairs
+template <int R>
+constexpr int kTableStride = ((R + 2) / 2 | 1) * 2;  // pairs
 template <int RMax>
-struct PairShape {
-    static constexpr int kQ = (RMax + 1 + 3) / 4;            // float4 chunks of e_s(k), k <= RMax
-    static constexpr int kEWStride = (RMax + 1) | 1;          // odd: lanes of one row hit distinct banks
-    static constexpr int kOutInts = (kTileY + 2 * RMax) * (kTileX + 2 * RMax);
-    static constexpr size_t kSmemBytes =
-        (size_t(kQ) * kThreads * 4 + size_t(kThreads) * kEWStride + kOutInts) * sizeof(float);
-};
+constexpr int kWarpPairs = kRowNodes * (kTableStride<RMax> + kPairs * kRowStride<RMax>);
 
-// Column part of the slot of source (sy, sx) in the chunk-major e_s table
-// (slot = sy * 32 + e4_col(sx)): the low bits are XORed with bits 3..4 so that
-// source columns 4, 8 or 16 apart (read together by the lane groups of one
-// instruction) land in different banks.
-__device__ __forceinline__ int e4_col(int sx) { return sx ^ ((sx >> 3) & 3); }
+// Node weights of a tile: rows[((j - node0) * 4 + y) * stride + lane] for the row pair
+// (y, 7 - y) and the batch of nodes from node0 on. Per source the even and odd parts
+// E_p = sum idd B_p(t^2), S_p = sum idd t B_p(t^2) of each node pair are summed over the
+// layers; the weights are C_p (x_p E_p +- S_p). The layers' sources are copied into the
+// shared memory of the rows, which are written only after the last layer, as many
+// layers at a time as fit: all their loads are in flight at once, where loads into
+// registers would hold two row pairs of one layer.
+struct WeightPass {
+    const TileSource& s;
+    const NodeRange& n;
+    unsigned layers;
+    int node0;
+    float2* rows;
+    int room;  // layers that fit
+    int stride, lane;
 
-template <int R, int RMax>
-__device__ __forceinline__ void pair_item(float4* __restrict__ E4, float* __restrict__ EW, int* __restrict__ out,
-                                          unsigned* __restrict__ sCol, float* __restrict__ sSum,
-                                          const ItemArgs& a) {
-    constexpr int H = kTileY + 2 * R;
-    constexpr int Wo = kTileX + 2 * R;
-    constexpr int Q = (R + 1 + 3) / 4;
-    constexpr int EWS = PairShape<RMax>::kEWStride;
-    // A source column's footprint is the same column vector at offsets +d and -d (the
-    // weights depend on |d| only): one lane per (source column, |d|) pair adds it to
-    // both output columns. floor(32 / (R+1)) source columns, spaced so that their
-    // pairs fill distinct lanes, share one warp instruction.
-    constexpr int M = R + 1;
-    constexpr int G = 32 / M;                   // source columns per instruction
-    constexpr int S = (32 + G - 1) / G;         // column spacing
-    constexpr int kUnits = S;
-    const int t = threadIdx.x;
-    const int warp = t >> 5, lane = t & 31;
-
-    // Up to radius 7 a warp holds at most one (column, |d|) unit, whose column sums stay
-    // in registers over the item's layers and are flushed once.
-    constexpr bool kOneFlush = kUnits <= kWarps;
-
-    // H and Wo are even and `out` is 16-byte aligned.
-    for (int i = t; i < H * Wo / 4; i += kThreads) reinterpret_cast<int4*>(out)[i] = make_int4(0, 0, 0, 0);
-    // Fixed-point scale from the dose of every layer of the item: each thread sums its
-    // source over the layers, then the warps and the CTA add up. With one flush per
-    // item the sums run in the table phases and the scale is applied at the flush;
-    // with a flush per layer they run first and the scale is folded into the weights.
-    // Either way the total (the same additions in the same order) and the flushed
-    // values are the same.
-    float rowDose = 0.0f;
-    int sc = 0;
-    float scale = 1.0f;
-    auto item_scale = [&]() {
+    template <int J>
+    __device__ __forceinline__ void run() const {
+        const float2 shift = make_float2(n.shift, n.shift), inv = make_float2(n.invHalf, n.invHalf);
+        float2 even[kPairs][J / 2], odd[kPairs][J / 2];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) rowDose += __shfl_xor_sync(0xffffffffu, rowDose, o);
-        if (lane == 0) sSum[warp] = rowDose;
-        __syncthreads();
-        float total = 0.0f;
+        for (int y = 0; y < kPairs; ++y)
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) total += sSum[w];
-        sc = footprint_exponent(total);
-        scale = ldexpf(1.0f, sc);
-    };
-    if constexpr (!kOneFlush) {
+            for (int p = 0; p < J / 2; ++p) even[y][p] = odd[y][p] = make_float2(0.0f, 0.0f);
 #pragma unroll 1
-        for (int j = 0; j < kMergeLayers; ++j) {
-            const unsigned lc = (a.layers >> (8 * j)) & 0xffu;
-            if (lc == 0xffu) break;
-            rowDose += fmaxf(a.idd[lc * a.layerStride + a.src], 0.0f);
-        }
-        item_scale();
-    }
-
-    // Table phase of one layer (complete_superposition.cu:298-307): thread t is source
-    // (sy, sx) = (warp, lane); its rows e_s(0..R) go in float4 chunks (chunk-major)
-    // and idd_s e_s(0..R) 2^sc (the fixed-point scale is a power of two, so the column
-    // sums come out scaled exactly as if each were scaled at the flush); sources
-    // without dose get zero rows, and colMask[sx] collects the depositing sources of
-    // every column.
-    auto table = [&](unsigned lc, unsigned* colMask) {
-        const size_t src = lc * a.layerStride + a.src;
-        const float dose = a.idd[src];
-        if constexpr (kOneFlush) rowDose += fmaxf(dose, 0.0f);
-        const bool live = dose > 0.0f;
-        if (live) atomicOr(&colMask[lane], 1u << warp);
-        float e[4 * Q];
-        if (live) {
-            float row[R + 1];
-            superposition_row<R>(a.rsig[src], row);
-            const float doseScaled = kOneFlush ? dose : dose * scale;
+        for (unsigned m = layers; m;) {
+            int staged = 0;
+#pragma unroll 1
+            for (; m && staged < room; m &= m - 1u, ++staged)
+                copy_tile(s, __ffs(m) - 1, rows + staged * kTileSources, lane);
+            async_copies_wait();
+            __syncwarp();
+            const float2* f = rows + lane;
+#pragma unroll 1
+            for (; staged > 0; --staged, f += kTileSources) {
 #pragma unroll
-            for (int k = 0; k <= R; ++k) {
-                e[k] = row[k];
-                EW[t * EWS + k] = doseScaled * row[k];
-            }
-        } else {
+                for (int y = 0; y < kPairs; ++y) {
+                    const float2 u = f[y * kTileX], v = f[(kTileY - 1 - y) * kTileX];
+                    float2 dose;
+                    dose.x = u.y > n.from && u.y <= n.to ? fmaxf(u.x, 0.0f) : 0.0f;
+                    dose.y = v.y > n.from && v.y <= n.to ? fmaxf(v.x, 0.0f) : 0.0f;
+                    // Every t is finite: sources outside the range carry no dose.
+                    const float2 t = __ffma2_rn(make_float2(fminf(u.y, n.top), fminf(v.y, n.top)), inv, shift);
+                    float2 b[J / 2];
+                    pair_products<J>(__fmul2_rn(t, t), b);
 #pragma unroll
-            for (int k = 0; k <= R; ++k) {
-                e[k] = 0.0f;
-                EW[t * EWS + k] = 0.0f;
-            }
-        }
-#pragma unroll
-        for (int k = R + 1; k < 4 * Q; ++k) e[k] = 0.0f;
-        const int pt = warp * kTileX + e4_col(lane);
-#pragma unroll
-        for (int q = 0; q < Q; ++q)
-            E4[q * kThreads + pt] = make_float4(e[4 * q], e[4 * q + 1], e[4 * q + 2], e[4 * q + 3]);
-    };
-    // Adds the eight sources of source column sx at distance d to the column sums.
-    auto accumulate = [&](int sx, int d, float (&acc)[H]) {
-        const float* ewCol = EW + sx * EWS + d;
-        const float4* eCol = E4 + e4_col(sx);
-#pragma unroll
-        for (int sy = 0; sy < kTileY; ++sy) {
-            const float w = ewCol[sy * kTileX * EWS];
-#pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                const float4 v = eCol[q * kThreads + sy * kTileX];
-                const float ev[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int k = 4 * q + c;
-                    if (k <= R) {
-                        acc[sy + R + k] = fmaf(w, ev[c], acc[sy + R + k]);
-                        if (k > 0) acc[sy + R - k] = fmaf(w, ev[c], acc[sy + R - k]);
+                    for (int p = 0; p < J / 2; ++p) {
+                        const float2 q = __fmul2_rn(dose, b[p]);
+                        even[y][p] = __fadd2_rn(even[y][p], q);
+                        odd[y][p] = __ffma2_rn(q, t, odd[y][p]);
                     }
                 }
             }
-            // Lets the loads of the next source overlap this pair's FMAs but keeps
-            // later sources' loads from being hoisted (which would hold every row
-            // of the column in registers).
-            if (sy & 1) asm volatile("" ::: "memory");
+            __syncwarp();
         }
-    };
-    // Adds a pair's column sums to both of its output columns.
-    auto flush = [&](int sx, int d, const float (&acc)[H]) {
-        int qv[H];
 #pragma unroll
-        for (int i = 0; i < H; ++i) qv[i] = __float2int_rn(kOneFlush ? acc[i] * scale : acc[i]);
-        int* col = out + sx + R + d;
+        for (int p = 0; p < J / 2; ++p) {
+            const int j = 2 * p - node0;
+            if (J > kRowNodes && (j < 0 || j >= J / 2)) continue;
+            const float c = kNodeC[J / 2 - 2][p], cx = c * kNodeX[J / 2 - 2][p];
 #pragma unroll
-        for (int i = 0; i < H; ++i) atomicAdd(col + i * Wo, qv[i]);
-        if (d > 0) {
-            col = out + sx + R - d;
-#pragma unroll
-            for (int i = 0; i < H; ++i) atomicAdd(col + i * Wo, qv[i]);
+            for (int y = 0; y < kPairs; ++y) {
+                const float2 ev = __fmul2_rn(even[y][p], make_float2(cx, cx));
+                rows[(j * kPairs + y) * stride + lane] = __ffma2_rn(odd[y][p], make_float2(c, c), ev);
+                rows[((j + 1) * kPairs + y) * stride + lane] = __ffma2_rn(odd[y][p], make_float2(-c, -c), ev);
+            }
         }
-    };
+    }
+};
 
-    if constexpr (kOneFlush) {
-        // One pair unit per warp: its column sums stay in registers over all the
-        // item's layers and are flushed once. The column masks OR over the layers.
-        const int g = lane / M;
-        int d = lane - g * M;
-        int sx = warp + g * S;
-        const bool valid = warp < kUnits && g < G && sx < kTileX;
-        if (!valid) {
-            sx = 0;
-            d = 0;
-        }
-        float acc[H];
+// Rows: every row is convolved with its node's e in place. After source column x the
+// pending sums a[i] belong to columns x + 1 + i; column x is complete. Up to radius 15 a
+// lane takes one row pair in packed operations; above, where the pending sums of a pair
+// do not fit the registers, one row.
+template <int R>
+__device__ __forceinline__ void spread_rows(float2* __restrict__ rows, const float2* __restrict__ e, int nodes,
+                                            int lane) {
+    constexpr int U = 2;  // source columns per step: more would crowd the instruction cache
+    if constexpr (R <= 15) {
+        if (lane < nodes * kPairs) {
+            float2 k[kTableStride<R>];
+            const float4* e4 = reinterpret_cast<const float4*>(e + (lane / kPairs) * kTableStride<R>);
 #pragma unroll
-        for (int i = 0; i < H; ++i) acc[i] = 0.0f;
+            for (int q = 0; q < (R + 2) / 2; ++q) {
+                const float4 v = e4[q];
+                k[2 * q] = make_float2(v.x, v.y);
+                k[2 * q + 1] = make_float2(v.z, v.w);
+            }
+            float2* p = rows + lane * kRowStride<R>;
+            float2 a[2 * R + 1];
+#pragma unroll
+            for (int i = 0; i <= 2 * R; ++i) a[i] = make_float2(0.0f, 0.0f);
 #pragma unroll 1
-        for (int j = 0; j < kMergeLayers; ++j) {
-            const unsigned lc = (a.layers >> (8 * j)) & 0xffu;
-            if (lc == 0xffu) break;
-            table(lc, sCol);
-            __syncthreads();
-            // Lanes outside the footprint read source column 0 and are never flushed.
-            // Every lane takes part in the shuffle.
-            const unsigned colAll = __shfl_sync(0xffffffffu, sCol[lane], sx);
-            const unsigned colLive = valid ? colAll : 0u;
-            if (__any_sync(0xffffffffu, colLive != 0)) accumulate(sx, d, acc);
-            // The next layer's tables overwrite these.
-            __syncthreads();
+            for (int x = 0; x < kTileX; x += U) {
+                float2 v[U], out[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = p[x + u];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    out[u] = __ffma2_rn(v[u], k[R], a[0]);
+#pragma unroll
+                    for (int i = 0; i < 2 * R; ++i)
+                        a[i] = __ffma2_rn(v[u], k[i + 1 < R ? R - 1 - i : i + 1 - R], a[i + 1]);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) p[x + u] = out[u];
+            }
+#pragma unroll
+            for (int i = 0; i < 2 * R; ++i) p[kTileX + i] = a[i];
         }
-        item_scale();
-        const unsigned colAll = __shfl_sync(0xffffffffu, sCol[lane], sx);
-        const unsigned colLive = valid ? colAll : 0u;
-        if (colLive) flush(sx, d, acc);
-        __syncthreads();
-        if (t < kTileX) sCol[t] = 0;
     } else {
 #pragma unroll 1
-        for (int j = 0; j < kMergeLayers; ++j) {
-            const unsigned lc = (a.layers >> (8 * j)) & 0xffu;
-            if (lc == 0xffu) break;
-            // The layers alternate between two column-mask buffers: a buffer is
-            // cleared after the barrier that ends its layer's accumulation, and
-            // refilled two layers later.
-            unsigned* colMask = sCol + (j & 1) * kTileX;
-            table(lc, colMask);
-            __syncthreads();
-            // Lanes outside the footprint read source column 0 and are never flushed;
-            // pairs whose source column has no depositing source are skipped.
-            const unsigned colBits = colMask[lane];
+        for (int row = lane; row < nodes * kTileY; row += 32) {
+            float k[kTableStride<R>];
+            const float4* e4 = reinterpret_cast<const float4*>(e + (row / kTileY) * kTableStride<R>);
+#pragma unroll
+            for (int q = 0; q < (R + 2) / 2; ++q) {
+                const float4 v = e4[q];
+                k[2 * q] = v.x;
+                k[2 * q + 1] = v.z;
+            }
+            float* p = reinterpret_cast<float*>(rows + (row >> 1) * kRowStride<R>) + (row & 1);
+            float a[2 * R + 1];
+#pragma unroll
+            for (int i = 0; i <= 2 * R; ++i) a[i] = 0.0f;
 #pragma unroll 1
-            for (int u = warp; u < kUnits; u += kWarps) {
-                const int g = lane / M;
-                int d = lane - g * M;
-                int sx = u + g * S;
-                const bool valid = g < G && sx < kTileX;
-                if (!valid) {
-                    sx = 0;
-                    d = 0;
+            for (int x = 0; x < kTileX; x += U) {
+                float v[U], out[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = p[2 * (x + u)];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    out[u] = fmaf(v[u], k[R], a[0]);
+#pragma unroll
+                    for (int i = 0; i < 2 * R; ++i)
+                        a[i] = fmaf(v[u], k[i + 1 < R ? R - 1 - i : i + 1 - R], a[i + 1]);
                 }
-                const unsigned colAll = __shfl_sync(0xffffffffu, colBits, sx);
-                const unsigned colLive = valid ? colAll : 0u;
-                if (!__any_sync(0xffffffffu, colLive != 0)) continue;
-                float acc[H];
 #pragma unroll
-                for (int i = 0; i < H; ++i) acc[i] = 0.0f;
-                accumulate(sx, d, acc);
-                if (colLive) flush(sx, d, acc);
+                for (int u = 0; u < U; ++u) p[2 * (x + u)] = out[u];
             }
-            // The next layer's tables overwrite these.
-            __syncthreads();
-            if (t < kTileX) colMask[t] = 0;
+#pragma unroll
+            for (int i = 0; i < 2 * R; ++i) p[2 * (kTileX + i)] = a[i];
         }
     }
-    __syncthreads();
-
-    // ---- write-out -------------------------------------------------------------
-    write_footprint<H, Wo>(out, a.dst, a.bevX, sc, a.shift);
 }
 
-template <int R, int RHi, int RMax>
-__device__ __forceinline__ bool dispatch_pair(int r, float4* E4, float* EW, int* out, unsigned* sCol, float* sSum,
-                                              const ItemArgs& a) {
-    if (r == R) {
-        pair_item<R, RMax>(E4, EW, out, sCol, sSum, a);
-        return true;
-    }
-    if constexpr (R < RHi) return dispatch_pair<R + 1, RHi, RMax>(r, E4, EW, out, sCol, sSum, a);
-    return false;
+// Adds a footprint value (scaled to the BEV's fixed point) to a BEV cell. A batch of
+// nodes, or the rounding of the interpolation, can make it negative: the cells are
+// two's complement and their sum is taken as zero where it ends below it.
+__device__ __forceinline__ void add_to_bev(unsigned long long* cell, float v) {
+    if (fabsf(v) >= 0.5f) atomicAdd(cell, static_cast<unsigned long long>(__float2ll_rn(v)));
 }
 
-// ============================================================================
-// Radii 16..32: one layer per item, lanes over (source column, signed offset).
-// ============================================================================
+// A BEV cell as a float.
+__device__ __forceinline__ float from_bev(unsigned long long cell, double unit) {
+    return fmaxf(float(double(static_cast<long long>(cell)) * unit), 0.0f);
+}
 
-template <int RMax>
-struct WideShape {
-    static constexpr int kQ = (RMax + 1 + 3) / 4;            // float4 chunks of e_s(k), k <= RMax
-    static constexpr int kEWStride = (RMax + 1) | 1;          // odd: lanes of one row hit distinct banks
-    static constexpr int kOutFloats = (kTileY + 2 * RMax) * (kTileX + 2 * RMax);
-    static constexpr size_t kSmemBytes =
-        (size_t(kQ) * kThreads * 4 + size_t(kThreads) * kEWStride + kOutFloats) * sizeof(float);
-};
-
-template <int R, int RMax>
-__device__ __forceinline__ void wide_item(float4* __restrict__ E4, float* __restrict__ EW, int* __restrict__ out,
-                                          unsigned* __restrict__ sCol, float* __restrict__ sSum,
-                                          const ItemArgs& a) {
-    constexpr int H = kTileY + 2 * R;
-    constexpr int Wo = kTileX + 2 * R;
-    constexpr int Q = (R + 1 + 3) / 4;
-    constexpr int EWS = WideShape<RMax>::kEWStride;
-    constexpr int M = 2 * R + 1;                 // signed offsets per source column
-    constexpr int kPairs = kTileX * M;
-    constexpr int kUnits = (kPairs + 31) / 32;
-    const int t = threadIdx.x;
-    const int warp = t >> 5, lane = t & 31;
-    const size_t src = (a.layers & 0xffu) * a.layerStride + a.src;
-
-    // ---- table phase ----------------------------------------------------------
-    {
-        const float dose = a.idd[src];
-        const bool live = dose > 0.0f;
-        if (live) atomicOr(&sCol[lane], 1u << warp);
-        float rowDose = live ? dose : 0.0f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) rowDose += __shfl_xor_sync(0xffffffffu, rowDose, o);
-        if (lane == 0) sSum[warp] = rowDose;
-        float e[4 * Q];
-        if (live) {
-            float row[R + 1];
-            superposition_row<R>(a.rsig[src], row);
-#pragma unroll
-            for (int k = 0; k <= R; ++k) {
-                e[k] = row[k];
-                EW[t * EWS + k] = dose * row[k];
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k <= R; ++k) {
-                e[k] = 0.0f;
-                EW[t * EWS + k] = 0.0f;
-            }
-        }
-#pragma unroll
-        for (int k = R + 1; k < 4 * Q; ++k) e[k] = 0.0f;
-        const int pt = warp * kTileX + e4_col(lane);
-#pragma unroll
-        for (int q = 0; q < Q; ++q) E4[q * kThreads + pt] = make_float4(e[4 * q], e[4 * q + 1], e[4 * q + 2], e[4 * q + 3]);
-        for (int i = t; i < H * Wo / 4; i += kThreads) reinterpret_cast<int4*>(out)[i] = make_int4(0, 0, 0, 0);
-    }
-    __syncthreads();
-
-    float total = 0.0f;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) total += sSum[w];
-    const int sc = footprint_exponent(total);
-    const float scale = ldexpf(1.0f, sc);
-
-    // ---- accumulation phase -----------------------------------------------------
-    const unsigned colBits = sCol[lane];
+// Columns: a lane takes one footprint column, rows y and H-1-y as a pair (under
+// y -> H-1-y, sy -> 7-sy the footprint's form does not change), 32 columns at a time.
+// The last W % 32 columns go to several groups of lanes, each with every G-th node, whose
+// sums are added up. A finished strip of columns is laid over the rows it came from
+// (each column is read by its own pass only) and added to the BEV by a loop: the same
+// straight-line code for every footprint row would not fit the instruction cache.
+template <int R>
+__device__ __forceinline__ void spread_columns(float2* __restrict__ rows, const float2* __restrict__ e, int nodes,
+                                               int lane, unsigned long long* __restrict__ dst, int bevX,
+                                               float scale) {
+    constexpr int W = kTileX + 2 * R, H = kTileY + 2 * R, N = H / 2;
+    constexpr int kLast = W % 32;
+    constexpr int kLastShift = kLast == 0 ? 0 : (kLast <= 4 ? 3 : (kLast <= 8 ? 2 : (kLast <= 16 ? 1 : 0)));
+    constexpr int kSlots = kRowNodes * kPairs;  // rows of the strip
 #pragma unroll 1
-    for (int u = warp; u < kUnits; u += kWarps) {
-        const int pr = u * 32 + lane;
-        const bool valid = pr < kPairs;
-        int sx = pr / M;
-        int d = pr - sx * M - R;
-        if (!valid) {
-            sx = 0;
-            d = 0;
-        }
-        const int ad = d < 0 ? -d : d;
-        const unsigned colAll = __shfl_sync(0xffffffffu, colBits, sx);
-        const unsigned colLive = valid ? colAll : 0u;
-        if (!__any_sync(0xffffffffu, colLive != 0)) continue;
-        // Lanes outside the footprint read source column 0 and are never flushed.
-        const float* ewCol = EW + sx * EWS + ad;
-        const float4* eCol = E4 + e4_col(sx);
-        float acc[H];
+    for (int base = 0; base < W; base += 32) {
+        const bool last = kLast > 0 && base + 32 > W;
+        const int shift = last ? kLastShift : 0;
+        const int groups = 1 << shift, width = 32 >> shift;
+        const int group = lane >> (5 - shift), xi = lane & (width - 1);
+        const int n = last ? kLast : 32;
+        const int x = base + min(xi, n - 1);
+        float2 acc[N];
 #pragma unroll
-        for (int i = 0; i < H; ++i) acc[i] = 0.0f;
+        for (int i = 0; i < N; ++i) acc[i] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+        for (int j = group; j < nodes; j += groups) {
+            const float2* p = rows + j * kPairs * kRowStride<R> + x;
+            float2 t[kTileY];
 #pragma unroll
-        for (int sy = 0; sy < kTileY; ++sy) {
-            const float w = ewCol[sy * kTileX * EWS];
+            for (int y = 0; y < kPairs; ++y) {
+                const float2 v = p[y * kRowStride<R>];
+                t[y] = v;
+                t[kTileY - 1 - y] = make_float2(v.y, v.x);
+            }
+            const float4* e4 = reinterpret_cast<const float4*>(e + j * kTableStride<R>);
 #pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                const float4 v = eCol[q * kThreads + sy * kTileX];
-                const float ev[4] = {v.x, v.y, v.z, v.w};
+            for (int q = 0; q < (R + 2) / 2; ++q) {
+                // Keeps later table entries out of the registers until they are needed.
+                if (q > 0 && q % 2 == 0) asm volatile("" ::: "memory");
+                const float4 w = e4[q];
+                const float2 wk[2] = {make_float2(w.x, w.y), make_float2(w.z, w.w)};
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int k = 4 * q + c;
+                for (int c = 0; c < 2; ++c) {
+                    const int k = 2 * q + c;
                     if (k <= R) {
-                        acc[sy + R + k] = fmaf(w, ev[c], acc[sy + R + k]);
-                        if (k > 0) acc[sy + R - k] = fmaf(w, ev[c], acc[sy + R - k]);
+#pragma unroll
+                        for (int y = 0; y < kTileY; ++y) {
+                            if (y + R + k < N) acc[y + R + k] = __ffma2_rn(t[y], wk[c], acc[y + R + k]);
+                            if (k > 0 && y + R - k < N) acc[y + R - k] = __ffma2_rn(t[y], wk[c], acc[y + R - k]);
+                        }
                     }
                 }
             }
-            if (sy & 1) asm volatile("" ::: "memory");
         }
-        if (colLive) {
-            int* col = out + sx + R + d;
+        __syncwarp();
+#pragma unroll 1
+        for (int o = 16; o >= width; o >>= 1)
 #pragma unroll
-            for (int i = 0; i < H; ++i) atomicAdd(col + i * Wo, __float2int_rn(acc[i] * scale));
+            for (int i = 0; i < N; ++i) {
+                acc[i].x += __shfl_down_sync(0xffffffffu, acc[i].x, o);
+                acc[i].y += __shfl_down_sync(0xffffffffu, acc[i].y, o);
+            }
+#pragma unroll
+        for (int i0 = 0; i0 < N; i0 += kSlots) {
+            __syncwarp();
+            if (lane < n)
+#pragma unroll
+                for (int i = i0; i < N && i < i0 + kSlots; ++i) rows[(i - i0) * kRowStride<R> + x] = acc[i];
+            __syncwarp();
+            const int end = min(N, i0 + kSlots);
+            unsigned lo = (i0 + group) * bevX + x, hi = (H - 1 - i0 - group) * bevX + x;
+            const float2* f = rows + group * kRowStride<R> + x;
+#pragma unroll 1
+            for (int i = i0 + group; i < end; i += groups) {
+                const float2 v = *f;
+                if (xi < n) {
+                    add_to_bev(dst + lo, v.x * scale);
+                    add_to_bev(dst + hi, v.y * scale);
+                }
+                f += groups * kRowStride<R>;
+                lo += groups * bevX;
+                hi -= groups * bevX;
+            }
         }
     }
-    __syncthreads();
-
-    // ---- write-out ---------------------------------------------------------------
-    if (t < kTileX) sCol[t] = 0;
-    write_footprint<H, Wo>(out, a.dst, a.bevX, sc, a.shift);
 }
 
-template <int R, int RHi, int RMax>
-__device__ __forceinline__ bool dispatch_wide(int r, float4* E4, float* EW, int* out, unsigned* sCol, float* sSum,
-                                              const ItemArgs& a) {
+// The convolutions of an item at its radius.
+template <int R, int RHi>
+__device__ __forceinline__ void spread_item(int r, float2* rows, float2* e, int nodes, int lane,
+                                            unsigned long long* dst, int bevX, float scale) {
     if (r == R) {
-        wide_item<R, RMax>(E4, EW, out, sCol, sSum, a);
-        return true;
+        spread_rows<R>(rows, e, nodes, lane);
+        __syncwarp();
+        spread_columns<R>(rows, e, nodes, lane, dst, bevX, scale);
+        return;
     }
-    if constexpr (R < RHi) return dispatch_wide<R + 1, RHi, RMax>(r, E4, EW, out, sCol, sSum, a);
-    return false;
+    if constexpr (R < RHi) spread_item<R + 1, RHi>(r, rows, e, nodes, lane, dst, bevX, scale);
 }
 
-// ============================================================================
-// The persistent kernel.
-// ============================================================================
+// An item as a warp takes it from the work list, with the tile ranges of its layers
+// (lane = layer).
+struct Item {
+    unsigned layers;
+    int tile, zRel, R, base;
+    unsigned range;
+};
 
-// Persistent CTA loop over the merged items of radii RLo..RHi, claimed one at a
-// time through the range's counter (the next claim is issued before the current
-// item runs so that its latency is hidden). Items are taken radius block by radius
-// block, so the CTAs of the SM mostly run the code of one radius at a time.
+// Persistent warps over the items of radii RLo..RHi, claimed one at a time through the
+// range's counter. A claim is made two items ahead, and the next item is read and its
+// layers fetched into L2 while the current one runs, so that their latencies are hidden.
+// Items are taken radius block by radius block, so the warps of an SM mostly run the
+// code of one radius at a time.
 //
-// The three instances of a beam are launched back to back with programmatic
-// dependent launch: every CTA lets the next instance start at once (its items are
-// independent of this instance's: both only add to the fixed-point BEV), so the next
-// instance's CTAs take the SMs this instance's CTAs leave at its tail. Before it
-// exits a CTA waits for the previous instance to complete, so an instance is complete
-// only once all earlier ones are, and the kernel after the last one (launched
-// normally) sees every item's adds.
-template <bool kWide, int RLo, int RHi, int MinBlocks>
-__global__ void __launch_bounds__(kThreads, MinBlocks)
-superpose_kernel(BeamGeomDev g, const float* __restrict__ idd, const float* __restrict__ rsig,
+// The three instances of a beam (radii 24..32, 16..23 and 0..15, by the registers and
+// shared memory they need) are launched back to back with programmatic dependent launch: every CTA lets
+// the next instance start at once (its items are independent of this instance's: both
+// only add to the fixed-point BEV), so the next instance's CTAs take the SMs this
+// instance's CTAs leave at its tail. Before it exits a CTA waits for the previous
+// instance to complete, so an instance is complete only once the earlier one is, and the
+// kernel after the last one sees every item's adds. An instance of its own for radii up
+// to 7 (20 warps per SM instead of 16) was 2 to 9 % slower: its launch and tail cost more.
+template <int RLo, int RHi, int Warps, int MinBlocks>
+__global__ void __launch_bounds__(Warps * 32, MinBlocks)
+superpose_kernel(BeamGeomDev g, const float2* __restrict__ sources, const unsigned* __restrict__ tileRange,
                  const int4* __restrict__ work, BeamStateDev* __restrict__ beam, unsigned long long* __restrict__ bev,
-                 int shiftOffset, int range, size_t layerBevStride) {
-    extern __shared__ __align__(16) float sm[];
-    __shared__ int sItem[2];
-    // Per source column, its depositing sources over sy (radii 0..15: two buffers).
-    __shared__ unsigned sCol[2 * kTileX];
-    __shared__ float sSum[kTileY];
+                 int shiftOffset, size_t layerBevStride) {
+    extern __shared__ __align__(16) float2 sm[];
     __shared__ RadiusBlocks<RLo, RHi> sBlocks;
 
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int t = threadIdx.x;
-    // Range 0: R > kSplitR, 1: kSplitR2 < R <= kSplitR, 2: R <= kSplitR2.
-    int* counter = range == 0 ? &beam->workNext : (range == 1 ? &beam->workNextSmall : &beam->workNextTiny);
-    const size_t padPlane = static_cast<size_t>(g.pitchX) * g.pitchY;
+    pdl_trigger();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int* counter = RLo > kSplitWide ? &beam->workNext : (RLo > kSplitR ? &beam->workNextSmall : &beam->workNextTiny);
+    const int tiles = g.tilesX * g.tilesY;
+    const size_t padPlane = static_cast<size_t>(tiles) * kTileSources;
     const size_t bevPlane = static_cast<size_t>(g.bevX) * g.bevY;
+    float2* e = sm + warp * kWarpPairs<RHi>;
+    float2* rows = e + kRowNodes * kTableStride<RHi>;
+    constexpr int kRoom = kRowNodes * kPairs * kRowStride<RHi> / kTileSources;  // layers, 256 pairs each
 
     load_blocks<RLo, RHi>(beam, sBlocks);
-    if (t == 0) sItem[0] = atomicAdd(counter, 1);
-    if (t < 2 * kTileX) sCol[t] = 0;
-    if (t < kTileY) sSum[t] = 0.0f;
     __syncthreads();
-    ItemArgs a;
-    a.idd = idd;
-    a.rsig = rsig;
-    a.layerStride = static_cast<size_t>(g.steps) * padPlane;
-    a.bevX = g.bevX;
-    a.shift = beam->fixedShift + shiftOffset;
-    int buf = 0;
-    for (;;) {
-        const int c = sItem[buf];
-        if (c >= sBlocks.total) break;
-        if (t == 0) sItem[buf ^ 1] = atomicAdd(counter, 1);
-        const int4 it = work[block_slot<RLo, RHi>(sBlocks, c)];
-        const int tile = it.y, zRel = it.z, R = it.w;
-        const int tx = tile % g.tilesX, ty = tile / g.tilesX;
-        a.layers = static_cast<unsigned>(it.x);
-        a.src = zRel * padPlane + static_cast<size_t>(ty * kTileY + (t >> 5)) * g.pitchX + tx * kTileX + (t & 31);
+    const float scale = ldexpf(1.0f, beam->fixedShift + shiftOffset);
+    const int total = sBlocks.total;
+
+    TileSource s;
+    s.layerStride = static_cast<size_t>(g.steps) * padPlane;
+    auto source = [&](const Item& it) {
+        s.first = sources + it.base * s.layerStride + it.zRel * padPlane + it.tile * kTileSources;
+    };
+    auto fetch = [&](int c) {
+        Item it = {};
+        if (c < total) {
+            const int4 w = work[block_slot<RLo, RHi>(sBlocks, c)];
+            it.layers = static_cast<unsigned>(w.x);
+            it.tile = w.y;
+            it.zRel = w.z;
+            it.R = w.w & 0xff;
+            it.base = w.w >> 8;
+            if (it.layers >> lane & 1u)
+                it.range = tileRange[(static_cast<size_t>(it.base + lane) * g.steps + it.zRel) * tiles + it.tile];
+        }
+        return it;
+    };
+    // The first item of every warp is fixed; the counter deals out the others.
+    const int warps = gridDim.x * Warps;
+    int claim = 0;
+    if (lane == 0) claim = warps + atomicAdd(counter, 1);
+    Item next = fetch(blockIdx.x + warp * gridDim.x);
+    while (next.layers) {
+        const Item it = next;
+        next = fetch(__shfl_sync(0xffffffffu, claim, 0));
+        if (lane == 0) claim = warps + atomicAdd(counter, 1);
+        if (next.layers) {
+            source(next);
+            prefetch_tile(s, next.layers, lane);
+        }
+        const int R = it.R;
+        if (R < RLo || R > RHi) {
+            if (lane == 0) atomicOr(&beam->errorFlags, 2);
+            continue;
+        }
+        float lo, hi;
+        if (!item_range(it.range, lo, hi)) continue;
+        source(it);
+        const int tx = it.tile % g.tilesX, ty = it.tile / g.tilesX;
         // One BEV volume per layer when layerBevStride is set (one-layer items: batched
         // influence columns), else one volume for all layers.
-        a.dst = bev + (it.x & 0xff) * layerBevStride + static_cast<size_t>(zRel) * bevPlane +
-                static_cast<size_t>(ty * kTileY - R + kMaxR) * g.bevX + (tx * kTileX - R + kMaxR);
-        bool ok;
-        if constexpr (kWide) {
-            float4* E4 = reinterpret_cast<float4*>(sm);                                       // [Q][256] e_s(4q..4q+3)
-            float* EW = sm + WideShape<RHi>::kQ * kThreads * 4;                               // [256][EWS] idd_s e_s(k)
-            int* out = reinterpret_cast<int*>(EW + kThreads * WideShape<RHi>::kEWStride);   // [8+2R][32+2R]
-            ok = dispatch_wide<RLo, RHi, RHi>(R, E4, EW, out, sCol, sSum, a);
-        } else {
-            float4* E4 = reinterpret_cast<float4*>(sm);                                       // [Q][256] e_s(4q..4q+3)
-            float* EW = sm + PairShape<RHi>::kQ * kThreads * 4;                               // [256][EWS] idd_s e_s(k)
-            int* out = reinterpret_cast<int*>(EW + kThreads * PairShape<RHi>::kEWStride);   // [8+2R][32+2R]
-            ok = dispatch_pair<RLo, RHi, RHi>(R, E4, EW, out, sCol, sSum, a);
+        unsigned long long* dst = bev + (it.base + __ffs(it.layers) - 1) * layerBevStride +
+                                  static_cast<size_t>(it.zRel) * bevPlane +
+                                  static_cast<size_t>(ty * kTileY - R + kMaxR) * g.bevX + (tx * kTileX - R + kMaxR);
+        const int stride = kTileX + 2 * R + 1, eStride = ((R + 2) / 2 | 1) * 2;
+        for (float from = 0.0f;;) {
+            const NodeRange n = node_range(from, lo, hi);
+            const int batch = batch_nodes(n.count);
+            for (int node0 = 0; node0 < n.count; node0 += batch) {
+                node_tables(n, node0, batch, R, e, eStride, lane);
+                with_nodes(n.count, WeightPass{s, n, it.layers, node0, rows, kRoom, stride, lane});
+                __syncwarp();
+                spread_item<RLo, RHi>(R, rows, e, batch, lane, dst, g.bevX, scale);
+                __syncwarp();
+            }
+            if (n.top >= hi) break;
+            from = lo = n.top;
         }
-        if (!ok && t == 0) atomicOr(&beam->errorFlags, 2);
-        // Every thread is past the item (and has read sItem[buf]) before the next
-        // claim lands in that slot.
-        __syncthreads();
-        buf ^= 1;
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();
 }
 
 // `overlap`: launch as a programmatic dependent of the previous kernel on `s` (the
 // previous superposition instance).
-template <bool kWide, int RLo, int RHi, int MinBlocks>
-cudaError_t launch_range(const BeamGeomDev& g, const float* idd, const float* rsigma, const int4* work,
-                         BeamStateDev* beam, unsigned long long* bev, int shiftOffset, int gridBlocks, int range,
-                         bool overlap, size_t layerBevStride, cudaStream_t s) {
-    auto k = superpose_kernel<kWide, RLo, RHi, MinBlocks>;
-    const size_t smem = kWide ? WideShape<RHi>::kSmemBytes : PairShape<RHi>::kSmemBytes;
+template <int RLo, int RHi, int Warps, int MinBlocks>
+cudaError_t launch_range(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange, const int4* work,
+                        
+                         BeamStateDev* beam, unsigned long long* bev, int shiftOffset, int numSMs, bool overlap,
+                         size_t layerBevStride, cudaStream_t s) {
+    auto k = superpose_kernel<RLo, RHi, Warps, MinBlocks>;
+    const size_t smem = size_t(Warps) * kWarpPairs<RHi> * sizeof(float2);
     cudaError_t e = set_smem_limit(reinterpret_cast<const void*>(k), smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(gridBlocks);
-    cfg.blockDim = dim3(kThreads);
+    cfg.gridDim = dim3(numSMs * MinBlocks);
+    cfg.blockDim = dim3(Warps * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -567,7 +440,7 @@ cudaError_t launch_range(const BeamGeomDev& g, const float* idd, const float* rs
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = overlap ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k, g, idd, rsigma, work, beam, bev, shiftOffset, range, layerBevStride);
+    return cudaLaunchKernelEx(&cfg, k, g, sources, tileRange, work, beam, bev, shiftOffset, layerBevStride);
 }
 
 // Adds the fixed-point BEV of the chunk to the float BEV and clears it for the next
@@ -600,35 +473,36 @@ __global__ void __launch_bounds__(256) bev_fixed_to_float_kernel(BeamGeomDev g, 
         const ulonglong2 v = f2[pr];
         if (v.x | v.y) {
             float2 o = b2[pr];
-            o.x += float(double(v.x) * unit);
-            o.y += float(double(v.y) * unit);
+            o.x += from_bev(v.x, unit);
+            o.y += from_bev(v.y, unit);
             b2[pr] = o;
             f2[pr] = make_ulonglong2(0ull, 0ull);
         }
     }
 }
 
-// Resident CTAs per SM of the instances.
-constexpr int kWideBlocks = 2;
-constexpr int kMidBlocks = 5;
-constexpr int kNarrowBlocks = 6;
+// Warps per CTA and resident CTAs per SM of the instances.
+constexpr int kWidestWarps = 5, kWidestBlocks = 2;
+constexpr int kWideWarps = 4, kWideBlocks = 3;
+constexpr int kNarrowWarps = 4, kNarrowBlocks = 4;
 
 }  // namespace
 
 namespace {
 
 // The three instances over `work` (items sorted by range: the wide radii first).
-cudaError_t launch_instances(const BeamGeomDev& g, const float* idd, const float* rsigma, const int4* work,
+cudaError_t launch_instances(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange, const int4* work,
+                            
                              BeamStateDev* beam, unsigned long long* bevFixed, int shiftOffset, int numSMs,
                              size_t layerBevStride, cudaStream_t s) {
-    cudaError_t e = launch_range<true, kSplitR + 1, kMaxR, kWideBlocks>(
-        g, idd, rsigma, work, beam, bevFixed, shiftOffset, numSMs * kWideBlocks, 0, false, layerBevStride, s);
+    cudaError_t e = launch_range<kSplitWide + 1, kMaxR, kWidestWarps, kWidestBlocks>(
+        g, sources, tileRange, work, beam, bevFixed, shiftOffset, numSMs, false, layerBevStride, s);
     if (e != cudaSuccess) return e;
-    e = launch_range<false, kSplitR2 + 1, kSplitR, kMidBlocks>(g, idd, rsigma, work, beam, bevFixed, shiftOffset,
-                                                               numSMs * kMidBlocks, 1, true, layerBevStride, s);
+    e = launch_range<kSplitR + 1, kSplitWide, kWideWarps, kWideBlocks>(g, sources, tileRange, work, beam, bevFixed,
+                                                                       shiftOffset, numSMs, true, layerBevStride, s);
     if (e != cudaSuccess) return e;
-    return launch_range<false, 0, kSplitR2, kNarrowBlocks>(g, idd, rsigma, work, beam, bevFixed, shiftOffset,
-                                                           numSMs * kNarrowBlocks, 2, true, layerBevStride, s);
+    return launch_range<0, kSplitR, kNarrowWarps, kNarrowBlocks>(g, sources, tileRange, work, beam, bevFixed, shiftOffset,
+                                                                 numSMs, true, layerBevStride, s);
 }
 
 // A superposition over the chunk's whole one-layer work list (work_scatter_kernel):
@@ -675,8 +549,8 @@ __global__ void __launch_bounds__(256) column_fixed_to_float_kernel(BeamGeomDev 
         const ulonglong2 v = f2[pr];
         if (v.x | v.y) {
             float2 o = b2[pr];
-            o.x += float(double(v.x) * unit);
-            o.y += float(double(v.y) * unit);
+            o.x += from_bev(v.x, unit);
+            o.y += from_bev(v.y, unit);
             b2[pr] = o;
             f2[pr] = make_ulonglong2(0ull, 0ull);
         }
@@ -685,10 +559,11 @@ __global__ void __launch_bounds__(256) column_fixed_to_float_kernel(BeamGeomDev 
 
 }  // namespace
 
-cudaError_t launch_superpose(const BeamGeomDev& g, const float* idd, const float* rsigma, const int4* work,
+cudaError_t launch_superpose(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange, const int4* work,
+                            
                              BeamStateDev* beam, float* bev, unsigned long long* bevFixed, int shiftOffset, int numSMs,
                              cudaStream_t s) {
-    cudaError_t e = launch_instances(g, idd, rsigma, work, beam, bevFixed, shiftOffset, numSMs, 0, s);
+    cudaError_t e = launch_instances(g, sources, tileRange, work, beam, bevFixed, shiftOffset, numSMs, 0, s);
     if (e != cudaSuccess) return e;
     e = launch_pdl(bev_fixed_to_float_kernel, dim3(numSMs * 8), dim3(256), 0, s, g,
                    static_cast<const BeamStateDev*>(beam), bevFixed, bev, shiftOffset);
@@ -701,13 +576,14 @@ cudaError_t launch_one_layer_list_view(BeamStateDev* beam, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_superpose_columns(const BeamGeomDev& g, const float* idd, const float* rsigma, const int4* work,
+cudaError_t launch_superpose_columns(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange,
+                                     const int4* work,
                                      BeamStateDev* beam, const LayerStateDev* ls, int nCols, float* bev,
                                      unsigned long long* bevFixed, size_t stride, int numSMs, cudaStream_t s) {
     if (nCols <= 0) return cudaSuccess;
     if (stride % 2) return cudaErrorInvalidValue;
     one_layer_list_view_kernel<<<1, 64, 0, s>>>(beam);
-    cudaError_t e = launch_instances(g, idd, rsigma, work, beam, bevFixed, 0, numSMs, stride, s);
+    cudaError_t e = launch_instances(g, sources, tileRange, work, beam, bevFixed, 0, numSMs, stride, s);
     if (e != cudaSuccess) return e;
     const int per = std::max(1, (numSMs * 8) / nCols);
     column_fixed_to_float_kernel<<<dim3(per, nCols), 256, 0, s>>>(g, beam, ls, bevFixed, bev, stride);
