@@ -88,7 +88,7 @@ void PinnedBuf::release() {
 Context::~Context() {
     cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
-    for (DevBuf* b : {&cidd, &density, &sp, &rrl, &ct, &ctQuad, &dose64, &dens, &wepl, &weplMin, &rayW, &interm, &lattice,
+    for (DevBuf* b : {&cidd, &density, &sp, &rrl, &huTissue, &ct, &ctQuad, &dose64, &material, &wepl, &weplMin, &rayW, &interm, &lattice,
                       &sources, &bev, &cpb, &subspots, &floatOut, &firstIn, &firstOut, &firstPassive, &codes, &tileRange,
                       &work, &lp, &ls, &bs, &stats, &nucWeight, &nucSqSigma, &rayToNuc, &nucSources,
                       &nucCodes, &nucRange, &nucWork, &nucBev, &bevFixed, &nucLs, &nucBs, &errWord, &gradDoseBuf, &bevGrad, &rbarBuf,
@@ -265,6 +265,22 @@ int Context::set_energy(const PbsEnergyDesc& e) {
     PBS_CUDA(cudaMemcpyAsync(rrl.ptr, rrlHost.data(), rrlHost.size() * 4, cudaMemcpyHostToDevice, stream), "LUT");
     copiedH2D += (ciddHost.size() + densityHost.size() + spHost.size() + rrlHost.size()) * 4 +
                  (hasNuc ? 2 * nTab * 4 : 0);
+    // Density and stopping power on one axis, packed for the tracer.
+    luts.hu = nullptr;
+    if (e.n_density_samples == e.n_sp_samples && e.density_scale_fact == e.sp_scale_fact) {
+        const int n = e.n_density_samples;
+        std::vector<float4> packed(n);
+        for (int i = 0; i < n; ++i) {
+            const int j = std::min(i + 1, n - 1);
+            packed[i] = make_float4(densityHost[i], densityHost[j] - densityHost[i], spHost[i], spHost[j] - spHost[i]);
+        }
+        if ((rc = huTissue.ensure(packed.size() * sizeof(float4)))) return rc;
+        PBS_CUDA(cudaMemcpyAsync(huTissue.ptr, packed.data(), packed.size() * sizeof(float4), cudaMemcpyHostToDevice,
+                                 stream),
+                 "LUT");
+        copiedH2D += packed.size() * sizeof(float4);
+        luts.hu = static_cast<const float4*>(huTissue.ptr);
+    }
     luts.cidd = static_cast<const float*>(cidd.ptr);
     luts.nS = e.n_energy_samples;
     luts.nE = e.n_energies;
@@ -737,7 +753,8 @@ BeamBuffers beam_buffers(const BeamPlan& P, size_t nSubspotData, int nuclear, lo
     z.chunk = int(std::max<size_t>(1, std::min<size_t>(budget / std::max<size_t>(perLayer, 1), L)));
     z.chunk = std::min(z.chunk, 64);
     const size_t chunk = size_t(z.chunk);
-    z.dens = z.wepl = S * rays * 4;
+    z.material = S * rays * sizeof(float2);
+    z.wepl = S * rays * 4;
     z.weplMin = S * 4;
     z.firstIn = z.firstOut = rays * 4;
     z.rayW = L * rays * 4;
@@ -775,19 +792,19 @@ BeamBuffers beam_buffers(const BeamPlan& P, size_t nSubspotData, int nuclear, lo
 }
 
 size_t BeamBuffers::total(bool withTrace) const {
-    return (withTrace ? dens + wepl + weplMin + firstIn + firstOut : 0) + rayW + bev + codes + range + work + sources +
+    return (withTrace ? material + wepl + weplMin + firstIn + firstOut : 0) + rayW + bev + codes + range + work + sources +
            firstPassive + lp + ls + bs + lattice + interm + subspots + cpb + rayToNuc + nucSources + nucCodes +
            nucRange + nucWork + nucBev + nucLs + nucBs + bevFixed;
 }
 
 size_t trace_bytes(size_t steps, size_t rays) {
-    // dens, wepl | firstIn, firstOut | weplMin | inOut, each part 256-byte aligned
+    // material | wepl | firstIn, firstOut | weplMin | inOut, each part 256-byte aligned
     auto up = [](size_t n) { return (n + 255) / 256 * 256; };
-    return 2 * up(steps * rays * 4) + 2 * up(rays * 4) + up(steps * 4) + 256;
+    return up(steps * rays * sizeof(float2)) + up(steps * rays * 4) + 2 * up(rays * 4) + up(steps * 4) + 256;
 }
 
 void Context::use_stream_ordered_allocation() {
-    for (DevBuf* b : {&cidd, &density, &sp, &rrl, &ct, &ctQuad, &dose64, &dens, &wepl, &weplMin, &rayW, &interm, &lattice,
+    for (DevBuf* b : {&cidd, &density, &sp, &rrl, &huTissue, &ct, &ctQuad, &dose64, &material, &wepl, &weplMin, &rayW, &interm, &lattice,
                       &sources, &bev, &cpb, &subspots, &floatOut, &firstIn, &firstOut, &firstPassive, &codes, &tileRange,
                       &work, &lp, &ls, &bs, &stats, &nucWeight, &nucSqSigma, &rayToNuc, &nucSources,
                       &nucCodes, &nucRange, &nucWork, &nucBev, &bevFixed, &nucLs, &nucBs, &gradDoseBuf, &bevGrad, &rbarBuf, &gradInterm,
@@ -797,7 +814,7 @@ void Context::use_stream_ordered_allocation() {
 
 size_t Context::device_bytes() const {
     size_t n = 0;
-    for (const DevBuf* b : {&cidd, &density, &sp, &rrl, &ct, &ctQuad, &dose64, &dens, &wepl, &weplMin, &rayW, &interm, &lattice,
+    for (const DevBuf* b : {&cidd, &density, &sp, &rrl, &huTissue, &ct, &ctQuad, &dose64, &material, &wepl, &weplMin, &rayW, &interm, &lattice,
                             &sources, &bev, &cpb, &subspots, &floatOut, &firstIn, &firstOut, &firstPassive,
                             &codes, &tileRange, &work, &lp, &ls, &bs, &stats, &nucWeight, &nucSqSigma, &rayToNuc, &nucSources,
                             &nucCodes, &nucRange, &nucWork, &nucBev, &bevFixed, &nucLs, &nucBs, &errWord, &gradDoseBuf, &bevGrad,
@@ -809,7 +826,7 @@ size_t Context::device_bytes() const {
 
 void Context::release_beam_buffers() {
     join_side_work();
-    for (DevBuf* b : {&dens, &wepl, &weplMin, &rayW, &interm, &lattice, &sources, &bev, &cpb, &subspots,
+    for (DevBuf* b : {&material, &wepl, &weplMin, &rayW, &interm, &lattice, &sources, &bev, &cpb, &subspots,
                       &floatOut, &firstIn, &firstOut, &firstPassive, &codes, &tileRange, &work, &rayToNuc, &nucSources,
                       &nucCodes, &nucRange, &nucWork, &nucBev, &bevFixed, &gradDoseBuf, &bevGrad, &rbarBuf, &gradInterm, &gradLattice, &dose64,
                       &weqBody, &opColPtr, &opBlockOff, &opRows, &opVals, &opNorm, &opVoxels, &colBev, &colFixed,
@@ -1048,11 +1065,11 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
     trace = TraceSlot{};
     // A WEQ beam's trace is its own input, not a function of the geometry: never shared.
     if (traceStore && !P.hasWeqVolume && (rc = traceStore->acquire(*this, g, trace))) return rc;
-    if (!trace.dens) {
-        if ((rc = dens.ensure(z.dens)) || (rc = wepl.ensure(z.wepl)) || (rc = weplMin.ensure(z.weplMin)) ||
+    if (!trace.material) {
+        if ((rc = material.ensure(z.material)) || (rc = wepl.ensure(z.wepl)) || (rc = weplMin.ensure(z.weplMin)) ||
             (rc = firstIn.ensure(z.firstIn)) || (rc = firstOut.ensure(z.firstOut)))
             return rc;
-        trace.dens = static_cast<float*>(dens.ptr);
+        trace.material = static_cast<float2*>(material.ptr);
         trace.wepl = static_cast<float*>(wepl.ptr);
         trace.firstIn = static_cast<int*>(firstIn.ptr);
         trace.firstOut = static_cast<int*>(firstOut.ptr);
@@ -1224,7 +1241,7 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
     LayerParamsDev* dlp = static_cast<LayerParamsDev*>(lp.ptr);
     LayerStateDev* dls = static_cast<LayerStateDev*>(ls.ptr);
     BeamStateDev* dbs = static_cast<BeamStateDev*>(bs.ptr);
-    float* dDens = trace.dens;
+    float2* dMaterial = trace.material;
     float* dWepl = trace.wepl;
     int* dFi = trace.firstIn;
     int* dFo = trace.firstOut;
@@ -1257,15 +1274,15 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
         PBS_CUDA(cudaMemcpyAsync(weqBody.ptr, b.water_equivalence + 9, weqN * 4, cudaMemcpyHostToDevice, stream),
                  "WEQ H2D");
         copiedH2D += weqN * 4;
-        PBS_CUDA(launch_weq_trace(g, static_cast<const float*>(weqBody.ptr), P.weqNx, P.weqNy, P.weqSteps,
+        PBS_CUDA(launch_weq_trace(g, luts, static_cast<const float*>(weqBody.ptr), P.weqNx, P.weqNy, P.weqSteps,
                                   P.weqActiveSteps, P.weqStepMm, P.cpbCorner.x, P.cpbCorner.y, P.cpbRes.x, P.cpbRes.y,
-                                  P.weqX0, P.weqY0, P.weqDx, P.weqDy, dDens, dWepl, dFi, dFo, trace.weplMin, dbs,
+                                  P.weqX0, P.weqY0, P.weqDx, P.weqDy, dMaterial, dWepl, dFi, dFo, trace.weplMin, dbs,
                                   stream),
                  "weq_trace");
     } else {
         const float4* quad = !ctView && ctQuadValid ? static_cast<const float4*>(ctQuad.ptr) : nullptr;
         PBS_CUDA(launch_trace(g, luts, ctView ? ctView : static_cast<const float*>(ct.ptr), quad, ctGrid.dims[0],
-                              ctGrid.dims[1], ctGrid.dims[2], dDens, dWepl, dFi, dFo, trace.weplMin, dbs, stream),
+                              ctGrid.dims[1], ctGrid.dims[2], dMaterial, dWepl, dFi, dFo, trace.weplMin, dbs, stream),
                  "trace");
         if (trace.inOut) {
             PBS_CUDA(cudaMemcpyAsync(trace.inOut, &dbs->firstInside, 2 * sizeof(int), cudaMemcpyDeviceToDevice,
@@ -1351,7 +1368,7 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
     for (int l0 = 0; l0 < L; l0 += chunk) {
         const int nl = std::min(chunk, L - l0);
         if (nuclear) PBS_CUDA(launch_nuc_prepare(nucGeom, nl, dNucSources, stream), "nuc_prepare");
-        PBS_CUDA(launch_idd(g, luts, l0, nl, dDens, dWepl, dFi, dFo, dRayW, dlp, dls, dbs,
+        PBS_CUDA(launch_idd(g, luts, l0, nl, dMaterial, dWepl, dFi, dFo, dRayW, dlp, dls, dbs,
                             dSources, dRange, static_cast<uint8_t*>(codes.ptr), static_cast<int*>(firstPassive.ptr),
                             static_cast<const int*>(rayToNuc.ptr), static_cast<const float*>(lattice.ptr), dNucSources,
                             stream),
@@ -1677,7 +1694,17 @@ int Context::debug_copy(int which, int layer, void* out, size_t bytes) {
     PBS_CUDA(cudaMemcpy(&h, bs.ptr, sizeof(h), cudaMemcpyDeviceToHost), "debug D2H");
     const int first = h.firstInside;
     switch (which) {
-        case PBS_DBG_DENSITY: return copy(trace.dens, S * rays * 4);
+        case PBS_DBG_DENSITY: {
+            if (bytes != S * rays * 4) {
+                set_error("debug_copy: density size mismatch");
+                return PBS_ERR_INVALID_ARGUMENT;
+            }
+            std::vector<float2> m(S * rays);
+            PBS_CUDA(cudaMemcpy(m.data(), trace.material, m.size() * sizeof(float2), cudaMemcpyDeviceToHost), "debug D2H");
+            float* o = static_cast<float*>(out);
+            for (size_t i = 0; i < m.size(); ++i) o[i] = m[i].x;
+            return PBS_OK;
+        }
         case PBS_DBG_WEPL: return copy(trace.wepl, S * rays * 4);
         case PBS_DBG_FIRST_INSIDE: return copy(trace.firstIn, rays * 4);
         case PBS_DBG_FIRST_OUTSIDE: return copy(trace.firstOut, rays * 4);

@@ -37,7 +37,7 @@ struct PinnedBuf {
 // context's buffers grow to the largest beam they have run).
 struct BeamBuffers {
     int chunk = 1;
-    size_t dens = 0, wepl = 0, weplMin = 0, firstIn = 0, firstOut = 0, rayW = 0, bev = 0, codes = 0, range = 0, work = 0,
+    size_t material = 0, wepl = 0, weplMin = 0, firstIn = 0, firstOut = 0, rayW = 0, bev = 0, codes = 0, range = 0, work = 0,
            sources = 0, firstPassive = 0, lp = 0, ls = 0, bs = 0, lattice = 0, interm = 0, subspots = 0, cpb = 0;
     size_t rayToNuc = 0, nucSources = 0, nucCodes = 0, nucRange = 0, nucWork = 0, nucBev = 0, nucLs = 0, nucBs = 0;
     size_t bevFixed = 0;  // int64 accumulator of the larger of the two BEV volumes
@@ -47,13 +47,13 @@ BeamBuffers beam_buffers(const BeamPlan& P, size_t nSubspotData, int nuclear, lo
 
 struct Context;
 
-// Where a beam's trace lives: density and WEPL [S][rays], per-ray entry and exit
+// Where a beam's trace lives: material and WEPL [S][rays], per-ray entry and exit
 // steps, the per-step WEPL minimum and the beam's first-inside / first-outside
 // steps (two ints, in BeamStateDev order). A TraceStore keeps traces resident
 // across beams of the same geometry; without one the context's own buffers hold
 // the trace of its last beam.
 struct TraceSlot {
-    float* dens = nullptr;
+    float2* material = nullptr;  // density, density x radiation length
     float* wepl = nullptr;
     int* firstIn = nullptr;
     int* firstOut = nullptr;
@@ -65,7 +65,7 @@ struct TraceSlot {
 
 struct TraceStore {
     virtual ~TraceStore() = default;
-    // Fills `slot` for a beam of geometry `g` (dens == nullptr: not cached, use the
+    // Fills `slot` for a beam of geometry `g` (material == nullptr: not cached, use the
     // context's own buffers).
     virtual int acquire(Context& c, const BeamGeomDev& g, TraceSlot& slot) = 0;
     // The tracer into `slot` has been enqueued on the context stream.
@@ -123,7 +123,7 @@ struct Context {
     std::vector<float> energiesPerU, peakDepths, scaleFacts, ciddHost, densityHost, spHost, rrlHost;
     std::vector<float> nucWeightHost, nucSqSigmaHost;
     bool nucTablesAligned = false;
-    DevBuf cidd, density, sp, rrl, nucWeight, nucSqSigma;
+    DevBuf cidd, density, sp, rrl, huTissue, nucWeight, nucSqSigma;
     DevBuf profileBuf;     // the beam's CarbonPBS profile table
 
     // Biological model (pbs_context_set_bio_model): tables on the device, the
@@ -158,7 +158,7 @@ struct Context {
     DevBuf dose64;
 
     // Per-beam working set (grow-only).
-    DevBuf dens, wepl, weplMin, rayW, interm, lattice, sources, bev, cpb, subspots, floatOut;
+    DevBuf material, wepl, weplMin, rayW, interm, lattice, sources, bev, cpb, subspots, floatOut;
     DevBuf firstIn, firstOut, firstPassive, codes, tileRange, work, lp, ls, bs, stats;
     // Nuclear halo working set and the device word collecting error flags.
     DevBuf rayToNuc, nucSources, nucCodes, nucRange, nucWork, nucBev, nucLs, nucBs, errWord;

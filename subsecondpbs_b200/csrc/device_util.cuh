@@ -37,10 +37,11 @@ __device__ __forceinline__ float float_from_order_key(unsigned k) {
 
 // A tile's range of rSigma as one word: the upper bound in the high half, the lower one
 // in the low half, each the top 16 bits of the positive float below its sign (2^-8
-// relative, rounded outwards); 0 is no depositing source. A depositing source without a
-// valid rSigma > 0 has the smallest upper and the largest lower bound.
-__device__ __forceinline__ unsigned range_hi(float r) { return r > 0.0f ? max((__float_as_uint(r) + 0x7fffu) >> 15, 1u) : 1u; }
-__device__ __forceinline__ unsigned range_lo(float r) { return r > 0.0f ? __float_as_uint(r) >> 15 : 0xffffu; }
+// relative, rounded outwards); 0 is no depositing source.
+__device__ __forceinline__ unsigned range_word(int loBits, int hiBits) {
+    const unsigned hi = max((static_cast<unsigned>(hiBits) + 0x7fffu) >> 15, 1u);
+    return min(hi, 0xffffu) << 16 | static_cast<unsigned>(max(loBits, 0)) >> 15;
+}
 __device__ __forceinline__ unsigned merge_range(unsigned a, unsigned b) {
     if (!a || !b) return a | b;
     return max(a >> 16, b >> 16) << 16 | min(a & 0xffffu, b & 0xffffu);
@@ -54,6 +55,16 @@ __device__ __forceinline__ float lut_linear_clamp_smem(const float* t, int n, fl
     const int i1 = min(i0 + 1, n - 1);
     const float a = xb - fl;
     const float v0 = t[i0], v1 = t[i1];
+    return v0 + (v1 - v0) * a;
+}
+
+// The same on a table in shared memory whose last entry is stored twice.
+__device__ __forceinline__ float lut_linear_clamp_padded(const float* t, int n, float x) {
+    const float xb = fminf(fmaxf(x - 0.5f, 0.0f), float(n - 1));
+    const float fl = floorf(xb);
+    const int i = int(fl);
+    const float a = xb - fl;
+    const float v0 = t[i], v1 = t[i + 1];
     return v0 + (v1 - v0) * a;
 }
 

@@ -50,18 +50,17 @@ __device__ __forceinline__ float profile_sample(const float* __restrict__ t, int
 
 template <bool kNuclear, bool kProfile>
 __global__ void __launch_bounds__(256)
-idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ density,
+idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ material,
            const float* __restrict__ wepl, const int* __restrict__ firstInside, const int* __restrict__ firstOutside,
            const float* __restrict__ rayW, const LayerParamsDev* __restrict__ lp, LayerStateDev* __restrict__ ls,
            const BeamStateDev* __restrict__ beam, float2* __restrict__ sources, unsigned* __restrict__ tileRange,
            uint8_t* __restrict__ codes, int* __restrict__ firstPassiveOut, const int* __restrict__ rayToNuc,
            const float* __restrict__ lattice, float2* __restrict__ nucSources) {
     extern __shared__ float smem[];
-    float* ciddRow = smem;                                    // [nS]
-    float* nucWRow = ciddRow + luts.nS;                       // [nS] with the nuclear halo
+    float* ciddRow = smem;                                    // [nS + 1], the last entry twice
+    float* nucWRow = ciddRow + luts.nS + 1;                   // [nS] with the nuclear halo
     float* nucSRow = nucWRow + (kNuclear ? luts.nS : 0);      // [nS] with the nuclear halo
-    float* rrlTab = nucSRow + (kNuclear ? luts.nS : 0);       // [nRrl]
-    float* stepNum = rrlTab + luts.nRrl;                      // [steps] 0.5 (voxel width x + y)
+    float* stepNum = nucSRow + (kNuclear ? luts.nS : 0);      // [steps] 0.5 (voxel width x + y)
     float* stepVolT = stepNum + g.steps;                      // [steps] step volume
     float* partMin = stepVolT + g.steps;                      // [steps][8]
     unsigned* partRange = reinterpret_cast<unsigned*>(partMin + g.steps * 8);  // [steps][8]
@@ -92,8 +91,9 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ de
         const int e1 = min(max(int(fl) + 1, 0), luts.nE - 1);
         const float* r0 = luts.cidd + static_cast<size_t>(e0) * luts.nS;
         const float* r1 = luts.cidd + static_cast<size_t>(e1) * luts.nS;
-        for (int d = tid; d < luts.nS; d += 256) {
-            const float a0 = __ldg(r0 + d), a1 = __ldg(r1 + d);
+        for (int d = tid; d <= luts.nS; d += 256) {
+            const int i = min(d, luts.nS - 1);
+            const float a0 = __ldg(r0 + i), a1 = __ldg(r1 + i);
             ciddRow[d] = a0 + (a1 - a0) * b;
         }
         if (kNuclear) {
@@ -109,7 +109,6 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ de
                 nucSRow[d] = c0 + (c1 - c0) * b;
             }
         }
-        for (int d = tid; d < luts.nRrl; d += 256) rrlTab[d] = __ldg(luts.rrl + d);
         // Per-step voxel widths and volumes are the same for every ray of the step
         // (fill_idd_and_sigma_params.cuh:56-80).
         for (int k = tid; k < g.steps; k += 256) {
@@ -181,12 +180,14 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ de
     float incDiv = p.sigmaSqAirLin + (2.0f * float(first) - 1.0f) * quad;
     float sigmaSq = -incDiv;
 
-    // The next step's WEPL and density are loaded one step ahead.
-    float nextSp = 0.0f, nextDens = 0.0f;
+    // The next step's WEPL and material are loaded one step ahead.
+    const float* nextW = wepl + static_cast<size_t>(first) * rayPlane + ridx;
+    const float2* nextM = material + static_cast<size_t>(first) * rayPlane + ridx;
+    float nextSp = 0.0f;
+    float2 nextMat = make_float2(0.0f, 0.0f);
     if (live && first < afterLastL) {
-        const size_t idx = static_cast<size_t>(first) * rayPlane + ridx;
-        nextSp = wepl[idx];
-        nextDens = density[idx];
+        nextSp = *nextW;
+        nextMat = *nextM;
     }
     float runMax = 0.0f;  // largest IDD of this ray (fixed-point range of the superposition)
     int stepNo = first;
@@ -203,17 +204,17 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ de
         const float nextProfileSp = kProfile && real ? wepl[static_cast<size_t>(stepNo) * rayPlane + ridx] : 0.0f;
         if (live) {
             const float cumulSp = nextSp;
-            const float dens = nextDens;
+            const float dens = nextMat.x, rRl = nextMat.y;
             if (stepNo + 1 < afterLastL) {
-                const size_t idx = static_cast<size_t>(stepNo + 1) * rayPlane + ridx;
-                nextSp = wepl[idx];
-                nextDens = density[idx];
+                nextW += rayPlane;
+                nextM += rayPlane;
+                nextSp = *nextW;
+                nextMat = *nextM;
             }
-            const float cumulDose = lut_linear_clamp_smem(ciddRow, luts.nS, cumulSp * p.energyScaleFact + 0.5f);
+            const float cumulDose = lut_linear_clamp_padded(ciddRow, luts.nS, cumulSp * p.energyScaleFact + 0.5f);
             if (cumulSp < p.peakDepth) {
                 const float resE = kECoef * __powf(p.peakDepth - 0.5f * (cumulSp + cumulSpOld), kPInv);
                 const float betaP = resE + 938.3f - __fdividef(938.3f * 938.3f, resE + 938.3f);
-                const float rRl = dens * lut_linear_clamp_smem(rrlTab, luts.nRrl, dens * luts.rrlScale + 0.5f);
                 const float thetaSq = __fdividef(eRefSq, betaP * betaP) * stepLength * rRl;
                 sigmaSq += incScat + incDiv;
                 incincScat += 2.0f * thetaSq * stepLength * stepLength;
@@ -305,19 +306,21 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float* __restrict__ de
         srcL[static_cast<size_t>(zr) * padPlane] = make_float2(res, rSigmaEff);
         if (nucIdx >= 0) nucL[static_cast<size_t>(zr) * nucPlane + nucIdx] = make_float2(nucRes, nucRSigmaEff);
 
-        // Warp minimum on order-preserving unsigned keys of the floats; the device's
-        // canonical NaN maps above +inf and drops out, as it does under fminf.
-        const unsigned mk = __reduce_min_sync(0xffffffffu, float_order_key(rSigmaEff));
-        // Range of rSigmaEff over the depositing sources. The smallest is the minimum above
-        // unless a ray without dose has a finite value too.
+        // Warp minimum over all rays and range over the depositing ones, on the bits of the
+        // floats, which order like them as long as they are positive (rSigmaEff is; the
+        // device's canonical NaN lies above +inf and drops out of the minimum, as it does
+        // under fminf). The smallest depositing value is the minimum unless a ray without
+        // dose has a finite value too.
         const bool deposits = res > 0.0f;
-        const unsigned hi = __reduce_max_sync(0xffffffffu, deposits ? range_hi(rSigmaEff) : 0u);
-        unsigned lo = range_lo(float_from_order_key(mk));
-        if (__any_sync(0xffffffffu, !deposits && rSigmaEff < __int_as_float(0x7f800000)))
-            lo = __reduce_min_sync(0xffffffffu, deposits ? range_lo(rSigmaEff) : 0xffffu);
+        const int bits = __float_as_int(rSigmaEff);
+        const int mk = __reduce_min_sync(0xffffffffu, bits);
+        const int hi = __reduce_max_sync(0xffffffffu, deposits ? bits : 0);
+        int lo = mk;
+        if (__any_sync(0xffffffffu, !deposits && bits < 0x7f800000))
+            lo = __reduce_min_sync(0xffffffffu, deposits ? bits : 0x7fffffff);
         if (lane == 0) {
-            partMin[zr * 8 + warp] = float_from_order_key(mk);
-            partRange[zr * 8 + warp] = hi ? hi << 16 | lo : 0u;
+            partMin[zr * 8 + warp] = __int_as_float(mk);
+            partRange[zr * 8 + warp] = hi > 0 ? range_word(lo, hi) : 0u;
         }
     }
     // The row's remaining steps: no dose, rSigmaEff = +inf, nothing live. Past the tile's
@@ -708,35 +711,44 @@ __global__ void nuc_codes_kernel(BeamGeomDev gn, int layer0, int nLayers, const 
         if (zr >= primaryLs[layer0 + lc].calcPassive - first) continue;
         const float2* ti = sources + (lc * static_cast<size_t>(gn.steps) + zr) * plane + size_t(tile) * kTileSources + lane;
         unsigned key = 0xffffffffu, range = 0;
+        bool live = false;
         float mx = 0.0f;
 #pragma unroll
         for (int r = 0; r < kTileY; ++r) {
             const float2 v = ti[r * kTileX];
             key = min(key, float_order_key(v.y));
-            if (v.x > 0.0f) range = merge_range(range, range_hi(v.y) << 16 | range_lo(v.y));
+            if (v.x > 0.0f && v.y > 0.0f) range = merge_range(range, range_word(__float_as_int(v.y), __float_as_int(v.y)));
+            live |= v.x > 0.0f;
             mx = fmaxf(mx, v.x);
         }
         key = __reduce_min_sync(0xffffffffu, key);
         const unsigned hi = __reduce_max_sync(0xffffffffu, range >> 16);
         const unsigned lo = __reduce_min_sync(0xffffffffu, range ? range & 0xffffu : 0xffffu);
+        live = __any_sync(0xffffffffu, live);
         const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
         if (lane == 0 && mb) atomicMax(&nucLs[layer0 + lc].maxIddBits, mb);
         if (lane == 0) {
             const int R = tile_radius_bucket(float_from_order_key(key));
-            codes[i] = static_cast<uint8_t>(R | (hi ? 0x80 : 0));
-            if (hi) tileRange[i] = hi << 16 | lo;
+            codes[i] = static_cast<uint8_t>(R | (live ? 0x80 : 0));
+            if (live) tileRange[i] = hi ? hi << 16 | lo : 0u;
             atomicAdd(&nucLs[layer0 + lc].histAll[R], 1);
-            if (hi) atomicAdd(&nucLs[layer0 + lc].liveHist[R], 1);
+            if (live) atomicAdd(&nucLs[layer0 + lc].liveHist[R], 1);
         }
     }
 }
 
 }  // namespace
 
+namespace {
+// Table rows, per-step widths and volumes, and the warps' partials of every step.
+size_t idd_smem(const BeamGeomDev& g, size_t tableFloats) {
+    return (tableFloats + 2 * static_cast<size_t>(g.steps)) * sizeof(float) +
+           static_cast<size_t>(g.steps) * 8 * (sizeof(float) + sizeof(unsigned));
+}
+}  // namespace
+
 size_t idd_smem_bytes(const BeamGeomDev& g, const LutsDev& luts) {
-    const size_t rows = static_cast<size_t>(luts.nS) * (g.nucOn ? 3 : 1);
-    return (rows + luts.nRrl + 2 * static_cast<size_t>(g.steps)) * sizeof(float) +
-           static_cast<size_t>(g.steps) * 8 * (sizeof(float) + sizeof(int));
+    return idd_smem(g, static_cast<size_t>(luts.nS) * (g.nucOn ? 3 : 1) + luts.nRrl);
 }
 
 cudaError_t launch_nuc_prepare(const BeamGeomDev& gn, int nLayers, float2* sources, cudaStream_t s) {
@@ -755,19 +767,19 @@ cudaError_t launch_nuc_codes(const BeamGeomDev& gn, int layer0, int nLayers, con
     return cudaGetLastError();
 }
 
-cudaError_t launch_idd(const BeamGeomDev& g, const LutsDev& luts, int layer0, int nLayers, const float* density,
+cudaError_t launch_idd(const BeamGeomDev& g, const LutsDev& luts, int layer0, int nLayers, const float2* material,
                        const float* wepl, const int* firstInside, const int* firstOutside, const float* rayW,
                        const LayerParamsDev* lp, LayerStateDev* ls, const BeamStateDev* beam, float2* sources,
                        unsigned* tileRange, uint8_t* codes, int* firstPassive, const int* rayToNuc, const float* lattice,
                        float2* nucSources, cudaStream_t s) {
     dim3 grid(g.tilesX, g.tilesY, nLayers);
     dim3 block(32, 8);
-    const size_t smem = idd_smem_bytes(g, luts);
+    const size_t smem = idd_smem(g, static_cast<size_t>(luts.nS) * (g.nucOn ? 3 : 1) + 1);
     auto k = g.nucOn ? (g.profileMode ? idd_kernel<true, true> : idd_kernel<true, false>)
                      : (g.profileMode ? idd_kernel<false, true> : idd_kernel<false, false>);
     cudaError_t e = set_smem_limit(reinterpret_cast<const void*>(k), smem);
     if (e != cudaSuccess) return e;
-    k<<<grid, block, smem, s>>>(g, luts, layer0, density, wepl, firstInside, firstOutside, rayW, lp, ls, beam, sources,
+    k<<<grid, block, smem, s>>>(g, luts, layer0, material, wepl, firstInside, firstOutside, rayW, lp, ls, beam, sources,
                                 tileRange, codes, firstPassive, rayToNuc, lattice, nucSources);
     return cudaGetLastError();
 }

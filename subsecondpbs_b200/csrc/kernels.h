@@ -37,11 +37,11 @@ cudaError_t launch_ct_convert_detect(float* ct, size_t n, const float* hostCtMap
 // `ctQuad` (or null) is the packed copy of the CT from launch_ct_quad: the same
 // samples from two 16-byte loads instead of eight scattered ones.
 cudaError_t launch_trace(const BeamGeomDev& g, const LutsDev& luts, const float* ctHu1000, const float4* ctQuad,
-                         int ctX, int ctY, int ctZ, float* density, float* wepl, int* firstInside, int* firstOutside,
+                         int ctX, int ctY, int ctZ, float2* material, float* wepl, int* firstInside, int* firstOutside,
                          float* weplMin, BeamStateDev* beam, cudaStream_t s);
 // Packed CT for the trace: entry (x, y, z) = the HU+1000 values at (x, y), (x+1, y),
 // (x, y+1), (x+1, y+1) of slice z, zero outside the CT, over a grid padded by two
-// voxels below and two or three above in every axis.
+// voxels below and two or three above in every axis, laid out in bricks (QuadLayout).
 size_t ct_quad_bytes(const int dims[3]);
 cudaError_t launch_ct_quad(const float* ctHu1000, const int dims[3], float4* quad, cudaStream_t s);
 // The packed entries of the voxels in the inclusive box [lo, hi] only (a CT uploaded
@@ -53,9 +53,9 @@ cudaError_t launch_ct_quad_box(const float* ctHu1000, const int dims[3], const i
 // fillBevFromWeqVolumeKernel + sliceMinVarIgnoreNeverEnter (wrapper.cu:1923-2023):
 // the exporter's water-equivalent depths [nx][ny][storedSteps] in place of the CT
 // trace, with the per-step minimum over entering rays.
-cudaError_t launch_weq_trace(const BeamGeomDev& g, const float* body, int nx, int ny, int storedSteps,
+cudaError_t launch_weq_trace(const BeamGeomDev& g, const LutsDev& luts, const float* body, int nx, int ny, int storedSteps,
                              int activeSteps, float stepMm, float rayOriginX, float rayOriginY, float rayStepX,
-                             float rayStepY, float x0, float y0, float dx, float dy, float* density, float* wepl,
+                             float rayStepY, float x0, float y0, float dx, float dy, float2* material, float* wepl,
                              int* firstInside, int* firstOutside, float* weplMin, BeamStateDev* beam, cudaStream_t s);
 cudaError_t launch_beam_planner(const BeamGeomDev& g, float* weplMin, const LayerParamsDev* lp,
                                 LayerStateDev* ls, BeamStateDev* beam, cudaStream_t s);
@@ -75,7 +75,7 @@ size_t idd_smem_bytes(const BeamGeomDev& g, const LutsDev& luts);
 // per-tile radius reduction of tileRadCalc (complete_superposition.cu:198-255).
 // With g.nucOn it also writes the nuclear halo IDD and sigma of the rays under a
 // halo lattice cell (rayToNuc: [rays] -> cell or -1) into [layer][step][nucY][nucX].
-cudaError_t launch_idd(const BeamGeomDev& g, const LutsDev& luts, int layer0, int nLayers, const float* density,
+cudaError_t launch_idd(const BeamGeomDev& g, const LutsDev& luts, int layer0, int nLayers, const float2* material,
                        const float* wepl, const int* firstInside, const int* firstOutside, const float* rayW,
                        const LayerParamsDev* lp, LayerStateDev* ls, const BeamStateDev* beam, float2* sources,
                        unsigned* tileRange, uint8_t* codes, int* firstPassive, const int* rayToNuc, const float* lattice,

@@ -106,13 +106,13 @@ __device__ __forceinline__ void copy_tile(const TileSource& s, int layer, float2
 __device__ __forceinline__ void async_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Range [lo, hi] of r over the layers of an item from the tile ranges the IDD kernel
-// left (lane = layer, range_hi / range_lo); false if no source has a valid r > 0.
+// left (lane = layer, range_word); false if no source has a valid r > 0.
 __device__ __forceinline__ bool item_range(unsigned laneRange, float& lo, float& hi) {
     const unsigned h = __reduce_max_sync(0xffffffffu, laneRange >> 16);
     const unsigned l = __reduce_min_sync(0xffffffffu, laneRange ? laneRange & 0xffffu : 0xffffu);
-    hi = fminf(__uint_as_float(h << 15), kMaxRSigma);
+    hi = fminf(__uint_as_float(h << 15), kMaxRSigma);  // (NaN too)
     lo = fminf(fmaxf(__uint_as_float(l << 15), 1.0e-12f), kMaxRSigma);
-    return h > 1u && l < 0xffffu && hi >= lo;
+    return h != 0u && hi >= lo;
 }
 
 // One range of r and its nodes: r = mid + half t, t in [-1, 1].

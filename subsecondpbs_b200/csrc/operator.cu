@@ -51,8 +51,8 @@ struct ColumnTraces : TraceStore {
                 return PBS_ERR_CUDA;
             auto up = [](size_t n) { return (n + 255) / 256 * 256; };
             char* p = static_cast<char*>(mem.ptr);
-            slot.dens = reinterpret_cast<float*>(p);
-            p += up(S * rays * 4);
+            slot.material = reinterpret_cast<float2*>(p);
+            p += up(S * rays * sizeof(float2));
             slot.wepl = reinterpret_cast<float*>(p);
             p += up(S * rays * 4);
             slot.firstIn = reinterpret_cast<int*>(p);

@@ -184,6 +184,9 @@ struct BioDev {
 struct LutsDev {
     const float* cidd;       // [nE][nS]
     int nS, nE;
+    // (density, next - density, sp, next - sp) per entry where the two tables share their
+    // axis, else null.
+    const float4* hu;
     const float* density;
     int nDensity;
     float densityScale;

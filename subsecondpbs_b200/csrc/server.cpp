@@ -75,6 +75,9 @@ void OwnedEnergy::assign(const PbsEnergyDesc& e) {
     };
     mix(density.data(), density.size() * 4);
     mix(sp.data(), sp.size() * 4);
+    mix(rrl.data(), rrl.size() * 4);
+    mix(&e.n_rrl_samples, sizeof(int));
+    mix(&e.rrl_scale_fact, sizeof(float));
     mix(&e.n_density_samples, sizeof(int));
     mix(&e.n_sp_samples, sizeof(int));
     mix(&e.density_scale_fact, sizeof(float));
@@ -533,8 +536,8 @@ int Server::trace_acquire(Slot& s, const BeamGeomDev& g, TraceSlot& ts) {
         auto up = [](size_t n) { return (n + 255) / 256 * 256; };
         char* p = static_cast<char*>(mem);
         TraceSlot t;
-        t.dens = reinterpret_cast<float*>(p);
-        p += up(S * rays * 4);
+        t.material = reinterpret_cast<float2*>(p);
+        p += up(S * rays * sizeof(float2));
         t.wepl = reinterpret_cast<float*>(p);
         p += up(S * rays * 4);
         t.firstIn = reinterpret_cast<int*>(p);
@@ -566,7 +569,7 @@ int Server::trace_done(Slot& s, TraceSlot& ts) {
     Request* r = s.current;
     TraceEntry* e = nullptr;
     for (TraceEntry* q : r->traces)
-        if (q && q->slot.dens == ts.dens) e = q;
+        if (q && q->slot.material == ts.material) e = q;
     if (!e) return fail(PBS_ERR_CUDA, "trace_done: unknown trace");
     if (cudaEventRecord(e->ready, s.ctx.stream) != cudaSuccess) return fail(PBS_ERR_CUDA, "cudaEventRecord failed");
     std::lock_guard<std::mutex> lk(mu_);

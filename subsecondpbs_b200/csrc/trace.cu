@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 
 #include "device_util.cuh"
 #include "kernels.h"
@@ -22,6 +23,25 @@ constexpr size_t kTraceCacheMaxBytes = 160 * 1024;  // CT samples kept on chip u
 // of slice z, for x in [-2, dx + 1], y in [-2, dy + 1], z in [-2, dz + 2] (zero
 // outside the CT): every floor index the clamped sample point can take.
 constexpr int kQuadPad = 2;
+
+// Entry (x, y, z) counted from the padded corner lies in a brick of 8 x 8 x 8 entries
+// (8 KB), and in it in a 128-byte line of 2 x 2 x 2. Rays cross the CT in any direction:
+// with rows of entries along x a ray that runs across them took 32 bytes of every line it
+// touched, and its neighbours touched other lines (a 512 x 512 x 200 CT, which does not
+// fit L2: 229 us for the trace of a 1 mm field, 258 us oblique).
+struct QuadLayout {
+    unsigned bricksX, bricksXY;  // bricks along x, and per brick layer in z
+    __host__ __device__ QuadLayout(int dx, int dy)
+        : bricksX((dx + kQuadPad + 2 + 7) / 8), bricksXY((dx + kQuadPad + 2 + 7) / 8 * ((dy + kQuadPad + 2 + 7) / 8)) {}
+    // The index is the sum of a term of each coordinate.
+    __host__ __device__ size_t x(unsigned v) const { return (v & 1u) | (v & 6u) << 2 | (v & ~7u) << 6; }
+    __host__ __device__ size_t y(unsigned v) const {
+        return ((v & 1u) << 1 | (v & 6u) << 4) + static_cast<size_t>(v >> 3) * bricksX * 512u;
+    }
+    __host__ __device__ size_t z(unsigned v) const {
+        return ((v & 1u) << 2 | (v & 6u) << 6) + static_cast<size_t>(v >> 3) * bricksXY * 512u;
+    }
+};
 
 struct CtCorners {
     float c[8];
@@ -74,9 +94,9 @@ __device__ __forceinline__ void ct_fetch_quad(const float4* __restrict__ quad, i
     o.tx = fx - flx;
     o.ty = fy - fly;
     o.tz = fz - flz;
-    const size_t px = size_t(dx) + kQuadPad + 2, py = size_t(dy) + kQuadPad + 2;
-    const size_t i = (size_t(z0 + kQuadPad) * py + size_t(y0 + kQuadPad)) * px + size_t(x0 + kQuadPad);
-    const float4 a = __ldg(quad + i), b = __ldg(quad + i + px * py);
+    const QuadLayout q(dx, dy);
+    const float4* p = quad + q.x(x0 + kQuadPad) + q.y(y0 + kQuadPad);
+    const float4 a = __ldg(p + q.z(z0 + kQuadPad)), b = __ldg(p + q.z(z0 + kQuadPad + 1));
     o.c[0] = a.x;
     o.c[1] = a.y;
     o.c[2] = a.z;
@@ -96,6 +116,29 @@ __device__ __forceinline__ void ct_fetch_any(const float* __restrict__ ct, const
         ct_fetch(ct, dx, dy, dz, p.x, p.y, p.z, o);
 }
 
+// Density x radiation length of a step (idd_sigma.cu:170-175) beside its density. The
+// product depends on the ray and step only: taken here it is looked up once instead of
+// once per energy layer.
+__device__ __forceinline__ float2 step_material(const LutsDev& luts, float density) {
+    return make_float2(density, density * lut_linear_clamp(luts.rrl, luts.nRrl, density * luts.rrlScale + 0.5f));
+}
+
+// Density and stopping power of a CT sample. With luts.hu the two tables share their
+// axis and are packed (value and difference to the next one of each): one index and one
+// 16-byte load instead of two and four loads, with identical arithmetic.
+template <bool kPacked>
+__device__ __forceinline__ float2 sample_tissue(const LutsDev& luts, float hu) {
+    if (kPacked) {
+        const float xb = fminf(fmaxf(hu * luts.densityScale + 0.5f - 0.5f, 0.0f), float(luts.nDensity - 1));
+        const float fl = floorf(xb);
+        const float a = xb - fl;
+        const float4 t = __ldg(luts.hu + int(fl));
+        return make_float2(t.x + t.y * a, t.z + t.w * a);
+    }
+    return make_float2(lut_linear_clamp(luts.density, luts.nDensity, hu * luts.densityScale + 0.5f),
+                       lut_linear_clamp(luts.sp, luts.nSp, hu * luts.spScale + 0.5f));
+}
+
 __device__ __forceinline__ void kahan_add(float& sum, float& comp, float v) {
     const float y = v - comp;
     const float t = sum + y;
@@ -104,27 +147,35 @@ __device__ __forceinline__ void kahan_add(float& sum, float& comp, float v) {
 }
 
 // One CTA traces 32 neighbouring rays of one ray row; warp w marches depth segment w
-// (16 segments). In pass 1 the eight CT corners of the next step are loaded while
-// the current step is combined, looked up and summed.
-// Pass 1 sums each segment, the segment sums are prefix-scanned per ray, and pass 2
-// re-marches the segment writing density and compensated cumulative WEPL.
+// (16 segments). Pass 1 samples the CT and looks the samples up: the steps' density and
+// radiation length are written, their WEPL increments are kept and summed. The segment sums are
+// prefix-scanned per ray, and pass 2 sums the increments on from there into the
+// compensated cumulative WEPL.
 //
 // Pass 2 also folds each step's WEPL into the per-step minimum over rays
-// (sliceMinVarIgnoreNeverEnter, wrapper.cu:1991-2023): one warp minimum and one
-// atomic per warp and step on the bit patterns of the non-negative WEPL values. In
+// (sliceMinVarIgnoreNeverEnter, wrapper.cu:1991-2023): warp minima of the bit patterns
+// of the non-negative WEPL values, and one atomic instruction for 32 steps (an atomic
+// per step, 416 on each address of the headline beam, took a third of the kernel). In
 // this path every ray has firstStepOutside >= 1 (lastInside starts at 0,
 // bev_ray_tracing.cu:157), so the reference's never-entered filter keeps every ray.
 //
-// With kCache the first pass keeps every CT sample of the segment in shared memory
-// ([segment step][lane], 128 B per step and warp) and the second pass reads them
-// back instead of sampling the CT again.
-template <bool kCache, bool kQuad>
-// Three CTAs per SM (at most 42 registers): the headline grid of 416 row CTAs then
-// runs as one wave instead of 1.4.
-__global__ void __launch_bounds__(32 * kTraceSegments, 3)
+// The entry step (the first one whose cumulative HU+1000 reaches 150) needs the samples
+// again, in the segments where the sum can reach it only: one or two of a ray's 16.
+//
+// With kCache the first pass keeps the increments of the segment in shared memory
+// ([segment step][lane], 128 B per step and warp); else the second pass samples the CT
+// again.
+//
+// Bound by the latency and line traffic of the CT samples. Headline beam (104 x 128 rays,
+// 256 steps) 64 -> 52 us, 1 mm CT 425 -> 166 us, oblique 1 mm beam 250 -> 152 us, of which
+// the brick layout of the packed CT gave 63 and 106 us on the last two.
+template <bool kCache, bool kQuad, bool kPacked>
+// Two CTAs per SM: a third one leaves 42 registers (the sampling spills) and, with the
+// kept increments of 512 steps, no L1 cache for the CT and the tables.
+__global__ void __launch_bounds__(32 * kTraceSegments, 2)
 trace_kernel(BeamGeomDev g, LutsDev luts, const float* __restrict__ ct, const float4* __restrict__ ctQuad, int ctX,
              int ctY, int ctZ,
-             float* __restrict__ density, float* __restrict__ wepl, int* __restrict__ firstInside,
+             float2* __restrict__ material, float* __restrict__ wepl, int* __restrict__ firstInside,
              int* __restrict__ firstOutside, unsigned* __restrict__ weplMinBits, BeamStateDev* __restrict__ beam) {
     extern __shared__ float shCache[];  // [kTraceSegments][seg][32] with kCache
     const int lane = threadIdx.x, w = threadIdx.y;
@@ -152,22 +203,52 @@ trace_kernel(BeamGeomDev g, LutsDev luts, const float* __restrict__ ct, const fl
     }
 
     // Pass 1: segment sums of HU+1000 and of WEPL increments.
-    float huSum = 0.f, spSum = 0.f, spComp = 0.f;
+    const size_t plane = static_cast<size_t>(g.rayX) * g.rayY;
+    const size_t ray0 = static_cast<size_t>(s0) * plane + static_cast<size_t>(y) * g.rayX + x;
+    float huSum = 0.f, huTop = 0.f, huFirst = 0.f, spSum = 0.f, spComp = 0.f;
+    int lastK = -1;
     float* myCache = shCache + static_cast<size_t>(w) * seg * 32 + lane;
+    // Sums up a sample, writes its material and returns its WEPL increment.
+    float2* outM = material + ray0;
+    auto take = [&](int k, float hu) {
+        const float2 tissue = sample_tissue<kPacked>(luts, hu);
+        *outM = step_material(luts, tissue.x);
+        outM += plane;
+        if (k == s0) huFirst = hu;
+        huSum += hu;
+        huTop = fmaxf(huTop, huSum);
+        if (hu > 150.0f) lastK = k;
+        const float dw = stepLen * tissue.y;
+        kahan_add(spSum, spComp, dw);
+        return dw;
+    };
     if (active && s0 < s1) {
+        // The corners of several steps are loaded before the first of them is combined.
+        constexpr int kAhead = 2;
         V3 pos = pos0;
-        CtCorners cur, nxt;
-        ct_fetch_any<kQuad>(ct, ctQuad, ctX, ctY, ctZ, pos, cur);
-        for (int k = s0; k < s1; ++k) {
-            const V3 posN = add(pos, inc);
-            if (k + 1 < s1) ct_fetch_any<kQuad>(ct, ctQuad, ctX, ctY, ctZ, posN, nxt);
-            const float hu = ct_combine(cur);
-            if (kCache) myCache[(k - s0) * 32] = hu;
-            huSum += hu;
-            const float sp = lut_linear_clamp(luts.sp, luts.nSp, hu * luts.spScale + 0.5f);
-            kahan_add(spSum, spComp, stepLen * sp);
-            pos = posN;
-            cur = nxt;
+        for (int k0 = s0; k0 < s1; k0 += kAhead) {
+            CtCorners c[kAhead];
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+                // Past the segment's end the last sample point is read again.
+                ct_fetch_any<kQuad>(ct, ctQuad, ctX, ctY, ctZ, pos, c[i]);
+                if (k0 + i + 1 < s1) pos = add(pos, inc);
+            }
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+                if (k0 + i >= s1) break;
+                const float hu = ct_combine(c[i]);
+                // The samples are kept and looked up in a loop of their own: the two
+                // together hold too many registers.
+                if (kCache)
+                    myCache[(k0 + i - s0) * 32] = hu;
+                else
+                    take(k0 + i, hu);
+            }
+        }
+        if (kCache) {
+#pragma unroll 2
+            for (int k = s0; k < s1; ++k) myCache[(k - s0) * 32] = take(k, myCache[(k - s0) * 32]);
         }
     }
     shHu[w][lane] = huSum;
@@ -181,41 +262,59 @@ trace_kernel(BeamGeomDev g, LutsDev luts, const float* __restrict__ ct, const fl
         spPre += shSp[q][lane];
     }
 
-    // Pass 2: write the per-step samples (every lane runs the loop: it holds the
-    // warp reductions of the step minimum).
-    int firstK = kNone, lastK = -1;
+    // Entry step. No step of this segment has it while the running sum stays below the
+    // threshold with room for its rounding (a NaN among the samples takes the long way);
+    // the first step has it where the sum is there already.
+    int firstK = kNone;
+    if (active && s0 < s1 && !(huPre + huTop < 149.0f)) {
+        if (!(huPre + huFirst < 150.0f)) {
+            firstK = s0;
+        } else {
+            V3 pos = pos0;
+            float cumHu = huPre;
+            for (int k = s0; k < s1 && firstK == kNone; ++k) {
+                CtCorners c;
+                ct_fetch_any<kQuad>(ct, ctQuad, ctX, ctY, ctZ, pos, c);
+                cumHu += ct_combine(c);
+                if (!(cumHu < 150.0f)) firstK = k;
+                pos = add(pos, inc);
+            }
+        }
+    }
+
+    // Pass 2: the cumulative WEPL (every lane runs the loop: it holds the warp
+    // reductions of the step minimum).
     {
         V3 pos = pos0;
-        float cumHu = huPre;
         float cum = float(spPre);
         float comp = float(double(cum) - spPre);
-        const size_t plane = static_cast<size_t>(g.rayX) * g.rayY;
-        size_t idx = static_cast<size_t>(s0) * plane + static_cast<size_t>(y) * g.rayX + x;
-        for (int k = s0; k < s1; ++k) {
+        float* out = wepl + ray0;
+        unsigned stepMin = 0xffffffffu;
+        for (int k = s0; k < s1; ++k, out += plane) {
             unsigned bits = 0xffffffffu;
             if (active) {
-                float hu;
+                float dw;
                 if (kCache) {
-                    hu = myCache[(k - s0) * 32];
+                    dw = myCache[(k - s0) * 32];
                 } else {
                     CtCorners c;
                     ct_fetch_any<kQuad>(ct, ctQuad, ctX, ctY, ctZ, pos, c);
-                    hu = ct_combine(c);
+                    dw = stepLen * sample_tissue<kPacked>(luts, ct_combine(c)).y;
+                    pos = add(pos, inc);
                 }
-                cumHu += hu;
-                density[idx] = lut_linear_clamp(luts.density, luts.nDensity, hu * luts.densityScale + 0.5f);
-                const float sp = lut_linear_clamp(luts.sp, luts.nSp, hu * luts.spScale + 0.5f);
-                kahan_add(cum, comp, stepLen * sp);
-                wepl[idx] = cum;
-                if (firstK == kNone && !(cumHu < 150.0f)) firstK = k;
-                if (hu > 150.0f) lastK = k;
-                pos = add(pos, inc);
-                idx += plane;
+                kahan_add(cum, comp, dw);
+                *out = cum;
                 // NaN stays out of the minimum, as with the reference's `v < min` test.
                 bits = cum >= 0.0f ? (__float_as_uint(cum) & 0x7fffffffu) : (cum < 0.0f ? 0u : 0xffffffffu);
             }
+            // Lane i keeps the minimum of the i-th of 32 steps; they go out together.
             bits = __reduce_min_sync(0xffffffffu, bits);
-            if (lane == 0 && bits != 0xffffffffu) atomicMin(weplMinBits + k, bits);
+            const int i = (k - s0) & 31;
+            if (lane == i) stepMin = bits;
+            if (i == 31 || k + 1 == s1) {
+                const int mine = k - i + lane;
+                if (lane <= i) atomicMin(weplMinBits + mine, stepMin);
+            }
         }
     }
     shFirst[w][lane] = firstK;
@@ -248,15 +347,18 @@ trace_kernel(BeamGeomDev g, LutsDev luts, const float* __restrict__ ct, const fl
     }
 }
 
-// Packed CT (kQuadPad): one thread per entry.
-__global__ void ct_quad_kernel(const float* __restrict__ ct, int dx, int dy, int dz, float4* __restrict__ quad) {
-    const size_t px = size_t(dx) + kQuadPad + 2, py = size_t(dy) + kQuadPad + 2, pz = size_t(dz) + kQuadPad + 3;
-    const size_t n = px * py * pz;
+// Packed CT: one thread per entry, in the order of the entries in memory.
+__global__ void ct_quad_kernel(const float* __restrict__ ct, int dx, int dy, int dz, size_t n,
+                               float4* __restrict__ quad) {
+    const QuadLayout q(dx, dy);
     for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        const int x = int(i % px) - kQuadPad;
-        const size_t r = i / px;
-        const int y = int(r % py) - kQuadPad;
-        const int z = int(r / py) - kQuadPad;
+        const unsigned e = unsigned(i) & 511u;
+        const size_t brick = i >> 9;
+        const unsigned bz = unsigned(brick / q.bricksXY), r = unsigned(brick - size_t(bz) * q.bricksXY);
+        const unsigned by = r / q.bricksX, bx = r - by * q.bricksX;
+        const int x = int(bx * 8 + (e & 1) + (e >> 2 & 6)) - kQuadPad;
+        const int y = int(by * 8 + (e >> 1 & 1) + (e >> 4 & 6)) - kQuadPad;
+        const int z = int(bz * 8 + (e >> 2 & 1) + (e >> 6 & 6)) - kQuadPad;
         auto at = [&](int xi, int yi) -> float {
             if (xi < 0 || yi < 0 || z < 0 || xi >= dx || yi >= dy || z >= dz) return 0.0f;
             return ct[(size_t(z) * dy + yi) * dx + xi];
@@ -289,7 +391,7 @@ struct WeqParams {
 constexpr int kWeqRaysPerCta = 32;
 
 __global__ void __launch_bounds__(256)
-weq_fill_kernel(BeamGeomDev g, WeqParams q, float* __restrict__ density, float* __restrict__ wepl,
+weq_fill_kernel(BeamGeomDev g, LutsDev luts, WeqParams q, float2* __restrict__ material, float* __restrict__ wepl,
                 int* __restrict__ firstInside, int* __restrict__ firstOutside, BeamStateDev* __restrict__ beam) {
     __shared__ float tile[32][33];
     __shared__ float carry[32];
@@ -335,7 +437,7 @@ weq_fill_kernel(BeamGeomDev g, WeqParams q, float* __restrict__ density, float* 
                 const float prev = kk > 0 ? tile[kk - 1][lane] : carry[lane];
                 const float d = fmaxf(0.0f, v - prev) / safeStep;
                 wepl[static_cast<size_t>(k) * plane + r] = v;
-                density[static_cast<size_t>(k) * plane + r] = d;
+                material[static_cast<size_t>(k) * plane + r] = step_material(luts, d);
                 if (d > 1.0e-4f) {
                     first = min(first, k);
                     last = max(last, k);
@@ -667,15 +769,15 @@ cudaError_t launch_ct_stats(const float* ct, size_t n, float* minmax2, cudaStrea
 }
 
 size_t ct_quad_bytes(const int dims[3]) {
-    return (size_t(dims[0]) + kQuadPad + 2) * (size_t(dims[1]) + kQuadPad + 2) * (size_t(dims[2]) + kQuadPad + 3) *
-           sizeof(float4);
+    const QuadLayout q(dims[0], dims[1]);
+    return size_t(q.bricksXY) * ((size_t(dims[2]) + kQuadPad + 3 + 7) / 8) * 512 * sizeof(float4);
 }
 
 // Packed entries (x, y, z) for x, y, z in [lo, lo + ext) only; lo may reach into the
 // padding (negative, or past the CT), where the entries hold the border zeros.
 __global__ void ct_quad_box_kernel(const float* __restrict__ ct, int dx, int dy, int dz, int3 lo, int3 ext,
                                    float4* __restrict__ quad) {
-    const size_t px = size_t(dx) + kQuadPad + 2, py = size_t(dy) + kQuadPad + 2;
+    const QuadLayout q(dx, dy);
     const size_t total = size_t(ext.x) * ext.y * ext.z;
     for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
         const int x = lo.x + int(i % size_t(ext.x));
@@ -686,7 +788,7 @@ __global__ void ct_quad_box_kernel(const float* __restrict__ ct, int dx, int dy,
             if (xi < 0 || yi < 0 || z < 0 || xi >= dx || yi >= dy || z >= dz) return 0.0f;
             return ct[(size_t(z) * dy + yi) * dx + xi];
         };
-        quad[(size_t(z + kQuadPad) * py + size_t(y + kQuadPad)) * px + size_t(x + kQuadPad)] =
+        quad[q.x(x + kQuadPad) + q.y(y + kQuadPad) + q.z(z + kQuadPad)] =
             make_float4(at(x, y), at(x + 1, y), at(x, y + 1), at(x + 1, y + 1));
     }
 }
@@ -712,12 +814,12 @@ cudaError_t launch_ct_quad_box(const float* ct, const int dims[3], const int lo[
 cudaError_t launch_ct_quad(const float* ct, const int dims[3], float4* quad, cudaStream_t s) {
     const size_t n = ct_quad_bytes(dims) / sizeof(float4);
     const int blocks = int(std::min<size_t>((n + 255) / 256, 148 * 16));
-    ct_quad_kernel<<<blocks, 256, 0, s>>>(ct, dims[0], dims[1], dims[2], quad);
+    ct_quad_kernel<<<blocks, 256, 0, s>>>(ct, dims[0], dims[1], dims[2], n, quad);
     return cudaGetLastError();
 }
 
 cudaError_t launch_trace(const BeamGeomDev& g, const LutsDev& luts, const float* ct, const float4* ctQuad, int ctX,
-                         int ctY, int ctZ, float* density, float* wepl, int* firstInside, int* firstOutside,
+                         int ctY, int ctZ, float2* material, float* wepl, int* firstInside, int* firstOutside,
                          float* weplMin, BeamStateDev* beam, cudaStream_t s) {
     // 0xff bytes: the largest unsigned pattern, the identity of the atomic minimum.
     cudaError_t e = cudaMemsetAsync(weplMin, 0xff, sizeof(float) * size_t(g.steps), s);
@@ -727,26 +829,31 @@ cudaError_t launch_trace(const BeamGeomDev& g, const LutsDev& luts, const float*
     const int seg = (g.steps + kTraceSegments - 1) / kTraceSegments;
     const size_t cache = static_cast<size_t>(kTraceSegments) * seg * 32 * sizeof(float);
     unsigned* mins = reinterpret_cast<unsigned*>(weplMin);
-    auto k = cache <= kTraceCacheMaxBytes ? (ctQuad ? trace_kernel<true, true> : trace_kernel<true, false>)
-                                          : (ctQuad ? trace_kernel<false, true> : trace_kernel<false, false>);
+    auto pick = [&](auto packed) {
+        constexpr bool kPacked = decltype(packed)::value;
+        return cache <= kTraceCacheMaxBytes
+                   ? (ctQuad ? trace_kernel<true, true, kPacked> : trace_kernel<true, false, kPacked>)
+                   : (ctQuad ? trace_kernel<false, true, kPacked> : trace_kernel<false, false, kPacked>);
+    };
+    auto k = luts.hu ? pick(std::true_type{}) : pick(std::false_type{});
     const size_t smem = cache <= kTraceCacheMaxBytes ? cache : 0;
     if (smem) {
         e = set_smem_limit(reinterpret_cast<const void*>(k), smem);
         if (e != cudaSuccess) return e;
     }
-    k<<<grid, block, smem, s>>>(g, luts, ct, ctQuad, ctX, ctY, ctZ, density, wepl, firstInside, firstOutside, mins,
+    k<<<grid, block, smem, s>>>(g, luts, ct, ctQuad, ctX, ctY, ctZ, material, wepl, firstInside, firstOutside, mins,
                                 beam);
     return cudaGetLastError();
 }
 
-cudaError_t launch_weq_trace(const BeamGeomDev& g, const float* body, int nx, int ny, int storedSteps,
+cudaError_t launch_weq_trace(const BeamGeomDev& g, const LutsDev& luts, const float* body, int nx, int ny, int storedSteps,
                              int activeSteps, float stepMm, float rayOriginX, float rayOriginY, float rayStepX,
-                             float rayStepY, float x0, float y0, float dx, float dy, float* density, float* wepl,
+                             float rayStepY, float x0, float y0, float dx, float dy, float2* material, float* wepl,
                              int* firstInside, int* firstOutside, float* weplMin, BeamStateDev* beam, cudaStream_t s) {
     WeqParams q{body, nx, ny, storedSteps, activeSteps, stepMm, rayOriginX, rayOriginY, rayStepX, rayStepY,
                 x0, y0, dx, dy};
     const int rays = g.rayX * g.rayY;
-    weq_fill_kernel<<<(rays + kWeqRaysPerCta - 1) / kWeqRaysPerCta, 256, 0, s>>>(g, q, density, wepl, firstInside,
+    weq_fill_kernel<<<(rays + kWeqRaysPerCta - 1) / kWeqRaysPerCta, 256, 0, s>>>(g, luts, q, material, wepl, firstInside,
                                                                                   firstOutside, beam);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
