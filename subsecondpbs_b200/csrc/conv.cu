@@ -76,10 +76,17 @@ __global__ void conv_y_kernel(BeamGeomDev g, const float* __restrict__ interm, f
 // SubspotInfo (include/core/common.cuh:163-217) read with the legacy gantry frame of
 // wrapper.cu:3486-3493: the subspot sits at (dx, -dy) on the reference plane.
 // subspotToCPBConvolutionOptimizedKernel (src/algorithms/convolution.cu:95-152)
-// with the ranges of calculateSubspotRangeKernel (convolution.cu:45-92).
-__global__ void subspot_to_cpb_kernel(BeamGeomDev g, const float* __restrict__ subspots, int maxSubspots,
-                                      float* __restrict__ cpb) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+// with the ranges of calculateSubspotRangeKernel (convolution.cu:45-92). One warp per
+// subspot: the erf differences of its columns (one per lane) and rows are taken once, and
+// every row is one atomic instruction per 32 columns. Bound by the atomics; a thread per
+// subspot, with two erf differences per cell, took 253 us for 6 layers of 85 spots on a
+// 190 x 126 grid in place of 8.5 us.
+constexpr int kSubspotWarps = 4;
+
+__global__ void __launch_bounds__(32 * kSubspotWarps)
+subspot_to_cpb_kernel(BeamGeomDev g, const float* __restrict__ subspots, int maxSubspots, float* __restrict__ cpb) {
+    const int lane = threadIdx.x & 31;
+    const int m = blockIdx.x * kSubspotWarps + (threadIdx.x >> 5);
     const int l = blockIdx.y;
     if (m >= maxSubspots) return;
     const float* d = subspots + (static_cast<size_t>(l) * maxSubspots + m) * 5;
@@ -92,13 +99,19 @@ __global__ void subspot_to_cpb_kernel(BeamGeomDev g, const float* __restrict__ s
     const int minY = max(0, int(floorf((posY - 3.0f * sy - cy0) / ry)));
     const int maxY = min(ny - 1, int(ceilf((posY + 3.0f * sy - cy0) / ry)));
     const float dsx = 1.41421356f * sx, dsy = 1.41421356f * sy;
-    for (int cy = minY; cy <= maxY; ++cy) {
-        const float dy = (cy0 + (float(cy) + 0.5f) * ry) - posY;
-        const float ey = erff((dy + 0.5f * ry) / dsy) - erff((dy - 0.5f * ry) / dsy);
-        for (int cx = minX; cx <= maxX; ++cx) {
+    for (int y0 = minY; y0 <= maxY; y0 += 32) {
+        const float dy = (cy0 + (float(y0 + lane) + 0.5f) * ry) - posY;
+        const float eyLane = erff((dy + 0.5f * ry) / dsy) - erff((dy - 0.5f * ry) / dsy);
+        const int rows = min(32, maxY - y0 + 1);
+        for (int x0 = minX; x0 <= maxX; x0 += 32) {
+            const int cx = x0 + lane;
             const float dx = (cx0 + (float(cx) + 0.5f) * rx) - posX;
             const float ex = erff((dx + 0.5f * rx) / dsx) - erff((dx - 0.5f * rx) / dsx);
-            atomicAdd(cpb + (static_cast<size_t>(l) * ny + cy) * nx + cx, 0.25f * ex * ey * w);
+            float* cell = cpb + (static_cast<size_t>(l) * ny + y0) * nx + cx;
+            for (int i = 0; i < rows; ++i, cell += nx) {
+                const float ey = __shfl_sync(0xffffffffu, eyLane, i);
+                if (cx <= maxX) atomicAdd(cell, 0.25f * ex * ey * w);
+            }
         }
     }
 }
@@ -237,8 +250,8 @@ cudaError_t launch_conv_cpb(const BeamGeomDev& g, const float* subspots, int max
     const size_t n = static_cast<size_t>(g.rayX) * g.rayY * g.numLayers;
     cudaError_t e = cudaMemsetAsync(cpb, 0, n * sizeof(float), s);
     if (e != cudaSuccess) return e;
-    dim3 gs((maxSubspots + 127) / 128, g.numLayers);
-    subspot_to_cpb_kernel<<<gs, 128, 0, s>>>(g, subspots, maxSubspots, cpb);
+    dim3 gs((maxSubspots + kSubspotWarps - 1) / kSubspotWarps, g.numLayers);
+    subspot_to_cpb_kernel<<<gs, 32 * kSubspotWarps, 0, s>>>(g, subspots, maxSubspots, cpb);
     dim3 block(32, 8);
     dim3 gr((g.rayX + 31) / 32, (g.rayY + 7) / 8, g.numLayers);
     cpb_to_ray_kernel<<<gr, block, 0, s>>>(g, cpb, rayW);
