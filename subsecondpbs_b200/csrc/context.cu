@@ -1421,7 +1421,8 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
             int slot = 0;
             for (int c : channels) {
                 if (c == 1 && bioModel != PBS_BIO_LQ) continue;
-                PBS_CUDA(launch_bio_channel(g, bioDev, l0, nl, dSources, dWepl, dls, dbs,
+                PBS_CUDA(launch_bio_channel(g, bioDev, l0, nl, dSources,
+                                            static_cast<const uint8_t*>(codes.ptr), dWepl, dls, dbs,
                                             static_cast<const float*>(bioLayerRow.ptr), c,
                                             static_cast<float2*>(bioSources.ptr), stream),
                          "bio_channel");

@@ -163,8 +163,9 @@ cudaError_t launch_dose_box(double* dose, float* out, const int dims[3], const i
 
 // Biological maps (bio.cu).
 cudaError_t launch_bio_channel(const BeamGeomDev& g, const BioDev& m, int layer0, int nLayers, const float2* sources,
-                               const float* wepl, const LayerStateDev* ls, const BeamStateDev* beam,
-                               const float* layerRow, int channel, float2* out, cudaStream_t s);
+                               const uint8_t* codes, const float* wepl, const LayerStateDev* ls,
+                               const BeamStateDev* beam, const float* layerRow, int channel, float2* out,
+                               cudaStream_t s);
 cudaError_t launch_bio_map(const double* dose, const double* c0, const double* c1, const double* c2, size_t n,
                            const BioDev& m, int map, float* out, cudaStream_t s);
 // Resets the superposition work list's claim counters so that the list can be run again.
