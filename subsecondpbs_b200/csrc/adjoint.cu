@@ -15,6 +15,7 @@
 #include "work_blocks.cuh"
 #include "kernels.h"
 #include "launch_util.h"
+#include "transfer_walk.cuh"
 
 namespace pbs {
 
@@ -25,8 +26,8 @@ namespace {
 // same weights. The forward adds a sample only where it is positive; a BEV sample
 // is a sum of non-negative terms, so it is zero only where every texel's
 // coefficient is zero and the linear transpose is exact.
-// Items of one dose column and 8 consecutive z, x fastest, strided over by a
-// persistent grid (the box is known only on the device; see transfer_kernel).
+// A lane takes one dose column and 8 consecutive z (walk_box; the box is known only on
+// the device).
 __global__ void __launch_bounds__(256)
 transfer_adjoint_kernel(BeamGeomDev g, const double* __restrict__ gradDose, const BeamStateDev* __restrict__ beam,
                         float* __restrict__ gradBev) {
@@ -37,17 +38,12 @@ transfer_adjoint_kernel(BeamGeomDev g, const double* __restrict__ gradDose, cons
     const int nyCols = min(((my - sy + 1 + 7) / 8) * 8, g.doseY - sy);
     const int nzc = (mz - sz + 8) / 8;
     if (nxCols <= 0 || nyCols <= 0 || nzc <= 0) return;
-    const long long items = static_cast<long long>(nxCols) * nyCols * nzc;
     const TransferParams T = beam->transfer;
     const float zShift = g.compatBevZShift ? float(beam->firstInside) : 0.0f;
     const size_t slice = static_cast<size_t>(g.doseX) * g.doseY;
     const int nx = g.bevX, ny = g.bevY, nz = g.steps;
-    for (long long it = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; it < items;
-         it += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int x = sx + static_cast<int>(it % nxCols);
-        const long long r = it / nxCols;
-        const int y = sy + static_cast<int>(r % nyCols);
-        const int z0 = sz + static_cast<int>(r / nyCols) * 8;
+    walk_box(T, sx, sy, nxCols, nyCols, nzc, [&](int x, int y, int chunk) {
+        const int z0 = sz + chunk * 8;
         const int z1 = min(mz, z0 + 7);
         const V3 start = transfer_start(T, x, y);
         for (int z = z0; z <= z1; ++z) {
@@ -70,7 +66,7 @@ transfer_adjoint_kernel(BeamGeomDev g, const double* __restrict__ gradDose, cons
                 atomicAdd(gradBev + (static_cast<size_t>(zi) * ny + yi) * nx + xi, w * gd);
             }
         }
-    }
+    });
 }
 
 constexpr int kAdjThreads = 256;

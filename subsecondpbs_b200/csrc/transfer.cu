@@ -10,6 +10,7 @@
 #include "device_util.cuh"
 #include "kernels.h"
 #include "launch_util.h"
+#include "transfer_walk.cuh"
 
 namespace pbs {
 
@@ -147,17 +148,31 @@ __global__ void column_transfer_planner_kernel(BeamGeomDev g, BeamStateDev* beam
     }
 }
 
-// primTransfDiv (src/algorithms/prim_transf_kernel.cu:11-44). The reference launches
-// ceil(width/32) x ceil(height/8) blocks from the box start, so columns up to the
-// next block boundary inside the dose grid are transferred too. Every voxel is
-// independent: the box (known only on the device) is cut into items of one dose
-// column (x, y) and kTransferZChunk consecutive z, x fastest so that a warp's FP64
-// read-modify-writes are coalesced, and a persistent grid strides over the items.
-// The chunk's voxels are sampled with independent loads (unrolled loop), so the
-// latency of the BEV samples and of the dose reads overlaps.
+// A column's BEV samples at kTransferZChunk consecutive z from z0 on (0 past `mz` and
+// outside the fan): independent loads, so that their latencies overlap.
 constexpr int kTransferZChunk = 4;
 constexpr int kTransferBlocksPerSM = 8;
 
+__device__ __forceinline__ void sample_chunk(const BeamGeomDev& g, const float* __restrict__ bev,
+                                             const TransferParams& T, float zShift, int x, int y, int z0, int mz,
+                                             float (&v)[kTransferZChunk]) {
+    const V3 start = transfer_start(T, x, y);
+#pragma unroll
+    for (int k = 0; k < kTransferZChunk; ++k) {
+        const int z = z0 + k;
+        v[k] = 0.0f;
+        if (z <= mz) {
+            const V3 f = transfer_fan_idx(T, start, z);
+            if (!(f.x + 0.5f < 0.0f || f.y + 0.5f < 0.0f || f.z + 0.5f < 0.0f))
+                v[k] = bev_sample(bev, g.bevX, g.bevY, g.steps, f.x, f.y, f.z - zShift);
+        }
+    }
+}
+
+// primTransfDiv (src/algorithms/prim_transf_kernel.cu:11-44). The reference launches
+// ceil(width/32) x ceil(height/8) blocks from the box start, so columns up to the
+// next block boundary inside the dose grid are transferred too. Every voxel is
+// independent: a persistent grid walks the box, which is known only on the device.
 __global__ void __launch_bounds__(256)
 transfer_kernel(BeamGeomDev g, const float* __restrict__ bev, const BeamStateDev* __restrict__ beam,
                 double* __restrict__ dose) {
@@ -170,33 +185,18 @@ transfer_kernel(BeamGeomDev g, const float* __restrict__ bev, const BeamStateDev
     const int ny = min(((my - sy + 1 + 7) / 8) * 8, g.doseY - sy);
     const int nzc = (mz - sz + kTransferZChunk) / kTransferZChunk;
     if (nx <= 0 || ny <= 0 || nzc <= 0) return;
-    const long long items = static_cast<long long>(nx) * ny * nzc;
     const TransferParams T = beam->transfer;
     const float zShift = g.compatBevZShift ? float(beam->firstInside) : 0.0f;
     const size_t slice = static_cast<size_t>(g.doseX) * g.doseY;
-    for (long long it = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; it < items;
-         it += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int x = sx + static_cast<int>(it % nx);
-        const long long r = it / nx;
-        const int y = sy + static_cast<int>(r % ny);
-        const int z0 = sz + static_cast<int>(r / ny) * kTransferZChunk;
-        const V3 start = transfer_start(T, x, y);
-        double* col = dose + static_cast<size_t>(y) * g.doseX + x;
+    walk_box(T, sx, sy, nx, ny, nzc, [&](int x, int y, int chunk) {
+        const int z0 = sz + chunk * kTransferZChunk;
         float v[kTransferZChunk];
-#pragma unroll
-        for (int k = 0; k < kTransferZChunk; ++k) {
-            const int z = z0 + k;
-            v[k] = 0.0f;
-            if (z <= mz) {
-                const V3 f = transfer_fan_idx(T, start, z);
-                if (!(f.x + 0.5f < 0.0f || f.y + 0.5f < 0.0f || f.z + 0.5f < 0.0f))
-                    v[k] = bev_sample(bev, g.bevX, g.bevY, g.steps, f.x, f.y, f.z - zShift);
-            }
-        }
+        sample_chunk(g, bev, T, zShift, x, y, z0, mz, v);
+        double* col = dose + static_cast<size_t>(y) * g.doseX + x;
 #pragma unroll
         for (int k = 0; k < kTransferZChunk; ++k)
             if (v[k] > 0.0f) col[static_cast<size_t>(z0 + k) * slice] += double(v[k]);
-    }
+    });
 }
 
 __global__ void dose_init_kernel(double* dose, const float* init, size_t n) {
@@ -239,35 +239,20 @@ column_transfer_kernel(BeamGeomDev g, const float* __restrict__ bev, size_t bevS
     if (!column_written_box(ls[q], g.doseX, g.doseY, fb, lo, hi)) return;
     const int nx = hi[0] - lo[0] + 1, ny = hi[1] - lo[1] + 1;
     const int nzc = (hi[2] - lo[2] + kTransferZChunk) / kTransferZChunk;
-    const long long items = static_cast<long long>(nx) * ny * nzc;
     const TransferParams T = beam->transfer;
     const float* v0 = bev + static_cast<size_t>(q) * bevStride;
     const size_t fbN = static_cast<size_t>(fb.ext[0]) * fb.ext[1] * fb.ext[2];
     double* out = colDose + static_cast<size_t>(q) * fbN;
     const size_t slice = static_cast<size_t>(fb.ext[0]) * fb.ext[1];
-    for (long long it = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; it < items;
-         it += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int x = lo[0] + static_cast<int>(it % nx);
-        const long long r = it / nx;
-        const int y = lo[1] + static_cast<int>(r % ny);
-        const int z0 = lo[2] + static_cast<int>(r / ny) * kTransferZChunk;
-        const V3 start = transfer_start(T, x, y);
-        double* col = out + static_cast<size_t>(y - fb.lo[1]) * fb.ext[0] + (x - fb.lo[0]);
+    walk_box(T, lo[0], lo[1], nx, ny, nzc, [&](int x, int y, int chunk) {
+        const int z0 = lo[2] + chunk * kTransferZChunk;
         float v[kTransferZChunk];
-#pragma unroll
-        for (int k = 0; k < kTransferZChunk; ++k) {
-            const int z = z0 + k;
-            v[k] = 0.0f;
-            if (z <= hi[2]) {
-                const V3 f = transfer_fan_idx(T, start, z);
-                if (!(f.x + 0.5f < 0.0f || f.y + 0.5f < 0.0f || f.z + 0.5f < 0.0f))
-                    v[k] = bev_sample(v0, g.bevX, g.bevY, g.steps, f.x, f.y, f.z);
-            }
-        }
+        sample_chunk(g, v0, T, 0.0f, x, y, z0, hi[2], v);
+        double* col = out + static_cast<size_t>(y - fb.lo[1]) * fb.ext[0] + (x - fb.lo[0]);
 #pragma unroll
         for (int k = 0; k < kTransferZChunk; ++k)
             if (v[k] > 0.0f) col[static_cast<size_t>(z0 + k - fb.lo[2]) * slice] += double(v[k]);
-    }
+    });
 }
 
 // Batched influence columns: zeroes column q's float BEV volume over its layer's
