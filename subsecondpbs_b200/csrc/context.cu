@@ -1046,15 +1046,17 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
         column_layout(P, colBox, colCells, perColumn);
         const size_t fbN = size_t(colBox.ext[0]) * colBox.ext[1] * colBox.ext[2];
         const size_t c = size_t(chunk);
+        const size_t doses = cols->norms() ? 0 : c * fbN * 8;  // row norms need no columns
         const bool had = colBev.bytes >= c * colCells * 4 && colFixed.bytes >= c * colCells * 8 &&
-                         colDose.bytes >= c * fbN * 8;
+                         colDose.bytes >= doses;
         if ((rc = colBev.ensure(c * colCells * 4)) || (rc = colFixed.ensure(c * colCells * 8)) ||
-            (rc = colDose.ensure(c * fbN * 8)))
+            (doses > 0 && (rc = colDose.ensure(doses))))
             return rc;
         if (!had || !colClean) {
             PBS_CUDA(cudaMemsetAsync(colBev.ptr, 0, colBev.bytes, stream), "memset column BEV");
             PBS_CUDA(cudaMemsetAsync(colFixed.ptr, 0, colFixed.bytes, stream), "memset column BEV");
-            PBS_CUDA(cudaMemsetAsync(colDose.ptr, 0, colDose.bytes, stream), "memset column dose");
+            if (colDose.bytes > 0)
+                PBS_CUDA(cudaMemsetAsync(colDose.ptr, 0, colDose.bytes, stream), "memset column dose");
         }
         // Clean again once every chunk's columns are compacted and cleared.
         colClean = false;
@@ -1398,10 +1400,14 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
             PBS_CUDA(launch_superpose_columns(g, dSources, dRange, static_cast<const int4*>(work.ptr), dbs, dls + l0, nl,
                                               cBev, cFixed, colCells, smCount, stream),
                      "superpose_columns");
-            PBS_CUDA(launch_column_transfer(g, cBev, colCells, dbs, dls + l0, nl, colBox,
-                                            static_cast<double*>(colDose.ptr), stream),
-                     "column_transfer");
-            if ((rc = cols->columns(l0, nl))) return rc;
+            if (double* norm = cols->norms()) {
+                PBS_CUDA(launch_column_norms(g, cBev, colCells, dbs, dls + l0, nl, colBox, norm, stream), "column_norms");
+            } else {
+                PBS_CUDA(launch_column_transfer(g, cBev, colCells, dbs, dls + l0, nl, colBox,
+                                                static_cast<double*>(colDose.ptr), stream),
+                         "column_transfer");
+                if ((rc = cols->columns(l0, nl))) return rc;
+            }
             PBS_CUDA(launch_column_bev_clear(g, cBev, colCells, dls + l0, nl, stream), "column_bev_clear");
             continue;
         }

@@ -262,6 +262,9 @@ struct Context {
     struct ColumnSink {
         virtual ~ColumnSink() = default;
         virtual int columns(int first, int count) = 0;
+        // Grid that takes the columns' squares (row norms) in place of their transfer into
+        // colDose; `columns` is not called then.
+        virtual double* norms() { return nullptr; }
     };
     // Batched influence columns of plan P: the box every column's dose buffer is laid
     // out over, the cells of one BEV volume, and the device bytes of one column.

@@ -97,6 +97,10 @@ cudaError_t launch_bin_plan(const BeamGeomDev& g, int layer0, int nLayers, const
 // over fb). The BEV clear zeroes each volume's live cells afterwards.
 cudaError_t launch_column_transfer(const BeamGeomDev& g, const float* bev, size_t bevStride, BeamStateDev* beam,
                                    LayerStateDev* ls, int nCols, const ColBox& fb, double* colDose, cudaStream_t s);
+// The same boxes, and the sum of the columns' squares added to `norm` (dose grid) in
+// place of the transfer.
+cudaError_t launch_column_norms(const BeamGeomDev& g, const float* bev, size_t bevStride, BeamStateDev* beam,
+                                LayerStateDev* ls, int nCols, const ColBox& fb, double* norm, cudaStream_t s);
 cudaError_t launch_column_bev_clear(const BeamGeomDev& g, float* bev, size_t bevStride, const LayerStateDev* ls,
                                     int nCols, cudaStream_t s);
 // Nuclear halo: clear the chunk's halo IDD (0) and sigma (+inf) before the IDD

@@ -402,45 +402,6 @@ __global__ void __launch_bounds__(kOpThreads) col_write_kernel(double* __restric
     }
 }
 
-// Row norms of a batch of columns: every voxel of fb adds the squares of the columns
-// whose box holds it, in column order (deterministic), and zeroes them.
-constexpr int kMaxColumnsPerBatch = 64;
-__global__ void __launch_bounds__(kOpThreads) col_norm_kernel(double* __restrict__ colDose, ColBox fb,
-                                                              const LayerStateDev* __restrict__ ls, int nCols, int X,
-                                                              int Y, double* __restrict__ norm) {
-    __shared__ int sLo[kMaxColumnsPerBatch][3], sHi[kMaxColumnsPerBatch][3];
-    __shared__ int sAny[kMaxColumnsPerBatch];
-    for (int q = threadIdx.x; q < nCols; q += blockDim.x) {
-        int lo[3], hi[3];
-        sAny[q] = column_written_box(ls[q], X, Y, fb, lo, hi);
-        for (int i = 0; i < 3; ++i) {
-            sLo[q][i] = lo[i];
-            sHi[q][i] = hi[i];
-        }
-    }
-    __syncthreads();
-    const size_t fbN = static_cast<size_t>(fb.ext[0]) * fb.ext[1] * fb.ext[2];
-    for (size_t at = blockIdx.x * size_t(blockDim.x) + threadIdx.x; at < fbN; at += size_t(gridDim.x) * blockDim.x) {
-        const int x = fb.lo[0] + static_cast<int>(at % fb.ext[0]);
-        const size_t r = at / fb.ext[0];
-        const int y = fb.lo[1] + static_cast<int>(r % fb.ext[1]);
-        const int z = fb.lo[2] + static_cast<int>(r / fb.ext[1]);
-        double acc = 0.0;
-        bool any = false;
-        for (int q = 0; q < nCols; ++q) {
-            if (!sAny[q] || x < sLo[q][0] || x > sHi[q][0] || y < sLo[q][1] || y > sHi[q][1] || z < sLo[q][2] ||
-                z > sHi[q][2])
-                continue;
-            double* d = colDose + static_cast<size_t>(q) * fbN + at;
-            const double v = *d;
-            *d = 0.0;
-            acc += v * v;
-            any = true;
-        }
-        if (any) norm[(static_cast<long long>(z) * Y + y) * X + x] += acc;
-    }
-}
-
 // The voxels the column just transferred can have written: the grid's dirty box,
 // or the whole grid when the context does not track one.
 OpBox dirty_op_box(const Context& c) {
@@ -461,6 +422,8 @@ OpBox dirty_op_box(const Context& c) {
     a.n = empty ? 0 : static_cast<long long>(a.ext[0]) * a.ext[1] * a.ext[2];
     return a;
 }
+
+constexpr int kMaxColumnsPerBatch = 64;
 
 // Spots per batched pass of an influence export (one plan layer and one BEV volume
 // and dose buffer each): at most the layers of one chunk's layer plan, and as many
@@ -812,24 +775,17 @@ int Context::influence_row_norms(const PbsBeamDesc& beam, int nuclear, long long
         return op_cuda(cudaGetLastError(), "row norm kernel");
     };
     if (!nuclear && !bioModel && !carbonProfile) {
-        // Batched: each batch's columns in their own dose buffers, their squares added
-        // voxel by voxel in column order.
+        // Batched: the squares of a batch's columns, voxel by voxel in column order; in the
+        // reference's depth convention the columns come one at a time.
         struct Sink : ColumnSink {
             Context& c;
             decltype(add)& run;
             double* norm;
             Sink(Context& ctx, decltype(add)& f, double* nm) : c(ctx), run(f), norm(nm) {}
-            int columns(int first, int count) override {
-                if (c.compatBevZShift) return run(dirty_op_box(c), false);
-                const ColBox fb = c.colBox;
-                const size_t fbN = size_t(fb.ext[0]) * fb.ext[1] * fb.ext[2];
-                if (fbN == 0 || count <= 0) return PBS_OK;
-                const int blocks = static_cast<int>(std::min<size_t>((fbN + kOpThreads - 1) / kOpThreads, 148 * 8));
-                col_norm_kernel<<<blocks, kOpThreads, 0, c.stream>>>(
-                    static_cast<double*>(c.colDose.ptr), fb, static_cast<const LayerStateDev*>(c.ls.ptr) + first,
-                    count, c.doseGrid.dims[0], c.doseGrid.dims[1], norm);
-                return op_cuda(cudaGetLastError(), "column row norms");
+            int columns(int, int) override {
+                return run(dirty_op_box(c), false);
             }
+            double* norms() override { return c.compatBevZShift ? nullptr : norm; }
         } sink(*this, add, norm);
         ColBox fb;
         size_t maxChunks = 0;

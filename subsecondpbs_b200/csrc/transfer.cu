@@ -255,6 +255,53 @@ column_transfer_kernel(BeamGeomDev g, const float* __restrict__ bev, size_t bevS
     });
 }
 
+// Batched influence columns, row norms: every voxel's samples in the columns whose box
+// holds it, squared and added up in column order into the voxel's norm. The sampling
+// coordinates are the same in all columns. Against transferring the columns into dose
+// buffers of their own and adding those up, no column is written, read and cleared
+// again (64 columns on 256 x 256 x 160 voxels: 181 + 434 -> 209 us).
+__global__ void __launch_bounds__(256)
+column_norm_kernel(BeamGeomDev g, const float* __restrict__ bev, size_t bevStride,
+                   const BeamStateDev* __restrict__ beam, const LayerStateDev* __restrict__ ls, int nCols, ColBox fb,
+                   double* __restrict__ norm) {
+    extern __shared__ int sBox[];  // [nCols][6]: lo and hi of the column's box (hi < lo: none)
+    __shared__ int sAll[6];
+    if (threadIdx.x < 6) sAll[threadIdx.x] = threadIdx.x < 3 ? 0x7fffffff : -1;
+    __syncthreads();
+    for (int q = threadIdx.x; q < nCols; q += blockDim.x) {
+        int lo[3], hi[3];
+        const bool any = column_written_box(ls[q], g.doseX, g.doseY, fb, lo, hi);
+        for (int i = 0; i < 3; ++i) {
+            sBox[q * 6 + i] = any ? lo[i] : 0x7fffffff;
+            sBox[q * 6 + 3 + i] = any ? hi[i] : -1;
+            if (any) {
+                atomicMin(&sAll[i], lo[i]);
+                atomicMax(&sAll[3 + i], hi[i]);
+            }
+        }
+    }
+    __syncthreads();
+    if (sAll[3] < sAll[0]) return;
+    const TransferParams T = beam->transfer;
+    walk_box(T, sAll[0], sAll[1], sAll[3] - sAll[0] + 1, sAll[4] - sAll[1] + 1, sAll[5] - sAll[2] + 1,
+             [&](int x, int y, int chunk) {
+                 const int z = sAll[2] + chunk;
+                 const V3 f = transfer_fan_idx(T, transfer_start(T, x, y), z);
+                 if (f.x + 0.5f < 0.0f || f.y + 0.5f < 0.0f || f.z + 0.5f < 0.0f) return;
+                 double acc = 0.0;
+#pragma unroll 4
+                 for (int q = 0; q < nCols; ++q) {
+                     const int* b = sBox + q * 6;
+                     if (x < b[0] || y < b[1] || z < b[2] || x > b[3] || y > b[4] || z > b[5]) continue;
+                     const double v = fmaxf(bev_sample(bev + static_cast<size_t>(q) * bevStride, g.bevX, g.bevY,
+                                                       g.steps, f.x, f.y, f.z),
+                                            0.0f);
+                     acc += v * v;
+                 }
+                 if (acc != 0.0) norm[(static_cast<size_t>(z) * g.doseY + y) * g.doseX + x] += acc;
+             });
+}
+
 // Batched influence columns: zeroes column q's float BEV volume over its layer's
 // live cells (the only cells its superposition wrote), so every volume is zero for
 // the next batch.
@@ -317,6 +364,18 @@ cudaError_t launch_column_transfer(const BeamGeomDev& g, const float* bev, size_
     // Blocks per column: a few waves over all columns together.
     const int per = std::max(1, (sms * kTransferBlocksPerSM) / nCols);
     column_transfer_kernel<<<dim3(per, nCols), 256, 0, s>>>(g, bev, bevStride, beam, ls, fb, colDose);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_column_norms(const BeamGeomDev& g, const float* bev, size_t bevStride, BeamStateDev* beam,
+                                LayerStateDev* ls, int nCols, const ColBox& fb, double* norm, cudaStream_t s) {
+    if (nCols <= 0) return cudaSuccess;
+    if (nCols > 1024) return cudaErrorInvalidValue;
+    column_transfer_planner_kernel<<<1, ((nCols + 31) / 32) * 32, 0, s>>>(g, beam, ls, nCols);
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const size_t smem = size_t(nCols) * 6 * sizeof(int);
+    column_norm_kernel<<<sms * kTransferBlocksPerSM, 256, smem, s>>>(g, bev, bevStride, beam, ls, nCols, fb, norm);
     return cudaGetLastError();
 }
 
