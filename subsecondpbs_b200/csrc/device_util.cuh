@@ -109,4 +109,17 @@ __device__ __forceinline__ void superposition_row(float rs, float (&e)[R + 1]) {
     }
 }
 
+// Calls f(x, y, z) for the cells of a box of w x rows x planes: a warp takes a row at a
+// time, so that a cell costs no division (with one 64-bit division per axis and cell,
+// clearing 64 influence columns took 64 us in place of 34 us).
+template <typename F>
+__device__ __forceinline__ void walk_rows(int w, int rows, int planes, F f) {
+    const unsigned warps = gridDim.x * blockDim.x >> 5, n = static_cast<unsigned>(rows) * planes;
+    const int lane = threadIdx.x & 31;
+    for (unsigned r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += warps) {
+        const int z = static_cast<int>(r / rows), y = static_cast<int>(r - static_cast<unsigned>(z) * rows);
+        for (int x = lane; x < w; x += 32) f(x, y, z);
+    }
+}
+
 }  // namespace pbs

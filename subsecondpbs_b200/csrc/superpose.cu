@@ -460,16 +460,11 @@ __global__ void __launch_bounds__(256) bev_fixed_to_float_kernel(BeamGeomDev g, 
     const int z0 = max(beam->liveLo[2], 0), z1 = min(beam->liveHi[2], planes - 1);
     if (x1 < x0 || y1 < y0 || z1 < z0) return;
     const int pw = (x1 - x0 + 1) / 2, rows = y1 - y0 + 1;
-    const size_t n = static_cast<size_t>(pw) * rows * (z1 - z0 + 1);
     const double unit = ldexp(1.0, -(beam->fixedShift + shiftOffset));
     ulonglong2* f2 = reinterpret_cast<ulonglong2*>(fixed);
     float2* b2 = reinterpret_cast<float2*>(bev);
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        const int xp = static_cast<int>(i % pw);
-        const size_t r = i / pw;
-        const int y = y0 + static_cast<int>(r % rows);
-        const int z = z0 + static_cast<int>(r / rows);
-        const size_t pr = ((static_cast<size_t>(z) * g.bevY + y) * g.bevX + x0) / 2 + xp;
+    walk_rows(pw, rows, z1 - z0 + 1, [&](int xp, int y, int z) {
+        const size_t pr = ((static_cast<size_t>(z0 + z) * g.bevY + y0 + y) * g.bevX + x0) / 2 + xp;
         const ulonglong2 v = f2[pr];
         if (v.x | v.y) {
             float2 o = b2[pr];
@@ -478,7 +473,7 @@ __global__ void __launch_bounds__(256) bev_fixed_to_float_kernel(BeamGeomDev g, 
             b2[pr] = o;
             f2[pr] = make_ulonglong2(0ull, 0ull);
         }
-    }
+    });
 }
 
 // Warps per CTA and resident CTAs per SM of the instances.
@@ -535,17 +530,12 @@ __global__ void __launch_bounds__(256) column_fixed_to_float_kernel(BeamGeomDev 
     const int z0 = max(st.liveLo[2], 0), z1 = min(st.liveHi[2], g.steps - 1);
     if (x1 < x0 || y1 < y0 || z1 < z0) return;
     const int pw = (x1 - x0 + 1) / 2, rows = y1 - y0 + 1;
-    const size_t n = static_cast<size_t>(pw) * rows * (z1 - z0 + 1);
     const double unit = ldexp(1.0, -beam->fixedShift);
     // stride is even (bevX is), so every volume starts on a cell pair.
     ulonglong2* f2 = reinterpret_cast<ulonglong2*>(fixed + static_cast<size_t>(q) * stride);
     float2* b2 = reinterpret_cast<float2*>(bev + static_cast<size_t>(q) * stride);
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        const int xp = static_cast<int>(i % pw);
-        const size_t r = i / pw;
-        const int y = y0 + static_cast<int>(r % rows);
-        const int z = z0 + static_cast<int>(r / rows);
-        const size_t pr = ((static_cast<size_t>(z) * g.bevY + y) * g.bevX + x0) / 2 + xp;
+    walk_rows(pw, rows, z1 - z0 + 1, [&](int xp, int y, int z) {
+        const size_t pr = ((static_cast<size_t>(z0 + z) * g.bevY + y0 + y) * g.bevX + x0) / 2 + xp;
         const ulonglong2 v = f2[pr];
         if (v.x | v.y) {
             float2 o = b2[pr];
@@ -554,7 +544,7 @@ __global__ void __launch_bounds__(256) column_fixed_to_float_kernel(BeamGeomDev 
             b2[pr] = o;
             f2[pr] = make_ulonglong2(0ull, 0ull);
         }
-    }
+    });
 }
 
 }  // namespace

@@ -212,18 +212,13 @@ __global__ void dose_to_float_kernel(const double* dose, float* out, size_t n) {
 // Box [lo, lo + ext) of a [dims.z][dims.y][dims.x] grid: zeroes the FP64 dose there
 // (out == nullptr) or converts it to float into the same voxels of `out`.
 __global__ void dose_box_kernel(double* dose, float* out, int3 dims, int3 lo, int3 ext) {
-    const size_t total = size_t(ext.x) * ext.y * ext.z;
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
-        const int x = int(i % size_t(ext.x));
-        const size_t r = i / size_t(ext.x);
-        const int y = int(r % size_t(ext.y));
-        const int z = int(r / size_t(ext.y));
+    walk_rows(ext.x, ext.y, ext.z, [&](int x, int y, int z) {
         const size_t v = (size_t(z + lo.z) * dims.y + (y + lo.y)) * size_t(dims.x) + (x + lo.x);
         if (out)
             out[v] = float(dose[v]);
         else
             dose[v] = 0.0;
-    }
+    });
 }
 
 // Batched influence columns: column q (blockIdx.y) samples its own BEV volume
@@ -315,28 +310,18 @@ __global__ void __launch_bounds__(256) column_bev_clear_kernel(BeamGeomDev g, fl
     const int z0 = max(st.liveLo[2], 0), z1 = min(st.liveHi[2], g.steps - 1);
     if (x1 < x0 || y1 < y0 || z1 < z0) return;
     const int w = x1 - x0 + 1, rows = y1 - y0 + 1;
-    const size_t n = static_cast<size_t>(w) * rows * (z1 - z0 + 1);
     float* v0 = bev + static_cast<size_t>(q) * bevStride;
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-        const int x = x0 + static_cast<int>(i % w);
-        const size_t r = i / w;
-        const int y = y0 + static_cast<int>(r % rows);
-        const int z = z0 + static_cast<int>(r / rows);
-        v0[(static_cast<size_t>(z) * g.bevY + y) * g.bevX + x] = 0.0f;
-    }
+    walk_rows(w, rows, z1 - z0 + 1, [&](int x, int y, int z) {
+        v0[(static_cast<size_t>(z0 + z) * g.bevY + y0 + y) * g.bevX + x0 + x] = 0.0f;
+    });
 }
 
 // Box [lo, lo + ext) of the FP64 grid initialised from the same voxels of a float grid.
 __global__ void dose_box_init_kernel(double* dose, const float* init, int3 dims, int3 lo, int3 ext) {
-    const size_t total = size_t(ext.x) * ext.y * ext.z;
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
-        const int x = int(i % size_t(ext.x));
-        const size_t r = i / size_t(ext.x);
-        const int y = int(r % size_t(ext.y));
-        const int z = int(r / size_t(ext.y));
+    walk_rows(ext.x, ext.y, ext.z, [&](int x, int y, int z) {
         const size_t v = (size_t(z + lo.z) * dims.y + (y + lo.y)) * size_t(dims.x) + (x + lo.x);
         dose[v] = double(init[v]);
-    }
+    });
 }
 
 }  // namespace
