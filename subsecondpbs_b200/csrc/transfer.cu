@@ -254,8 +254,9 @@ column_transfer_kernel(BeamGeomDev g, const float* __restrict__ bev, size_t bevS
 // holds it, squared and added up in column order into the voxel's norm. The sampling
 // coordinates are the same in all columns. Against transferring the columns into dose
 // buffers of their own and adding those up, no column is written, read and cleared
-// again (64 columns on 256 x 256 x 160 voxels: 181 + 434 -> 209 us).
-__global__ void __launch_bounds__(256)
+// again (64 columns on 256 x 256 x 160 voxels: 181 + 434 -> 85 us; with the
+// registers of an unbounded kernel, one block per SM, 209).
+__global__ void __launch_bounds__(256, 4)
 column_norm_kernel(BeamGeomDev g, const float* __restrict__ bev, size_t bevStride,
                    const BeamStateDev* __restrict__ beam, const LayerStateDev* __restrict__ ls, int nCols, ColBox fb,
                    double* __restrict__ norm) {
