@@ -39,8 +39,8 @@ __device__ __forceinline__ float float_from_order_key(unsigned k) {
 // in the low half, each the top 16 bits of the positive float below its sign (2^-8
 // relative, rounded outwards); 0 is no depositing source.
 __device__ __forceinline__ unsigned range_word(int loBits, int hiBits) {
-    const unsigned hi = max((static_cast<unsigned>(hiBits) + 0x7fffu) >> 15, 1u);
-    return min(hi, 0xffffu) << 16 | static_cast<unsigned>(max(loBits, 0)) >> 15;
+    const unsigned hi = min(static_cast<unsigned>(hiBits) + 0x7fffu, 0x7fffffffu);  // (NaN: 0xffff)
+    return max(__byte_perm(static_cast<unsigned>(max(loBits, 0)) << 1, hi << 1, 0x7632), 0x10000u);
 }
 __device__ __forceinline__ unsigned merge_range(unsigned a, unsigned b) {
     if (!a || !b) return a | b;

@@ -19,11 +19,23 @@ constexpr float kECoef = 8.639415f;   // (10 alpha)^(-1/p) (raytracedicom_integr
 constexpr float kSqrt2 = 1.41421356f;
 constexpr int kMaxChunkLayers = 64;
 
-// Divisions in the per-step walk use the approximate reciprocal (__fdividef, within
-// 2 ulp): the IEEE quotient's range check and slow path cost more ALU and branch
-// issue than the rest of a step's arithmetic. The tile radius bucket keeps its
-// IEEE division (tile_radius_bucket).
-//
+// Divisions in the per-step walk use the approximate reciprocal (within 2 ulp): the IEEE
+// quotient's range check and slow path cost more ALU and branch issue than the rest of
+// a step's arithmetic. Operands that are never subnormal take the forms without the
+// scaling that those need. The tile radius bucket keeps its IEEE division
+// (tile_radius_bucket).
+__device__ __forceinline__ float div_normal(float a, float b) {
+    float q;
+    asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(q) : "f"(a), "f"(b));
+    return q;
+}
+__device__ __forceinline__ float pow_normal(float x, float y) {
+    float l, r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y * l));
+    return r;
+}
+
 // One CTA = one 32x8 tile of rays for one layer. Each thread walks its ray from the
 // beam's first-inside step to the layer's cut-off step (fillIddAndSigmaKernel,
 // idd_sigma.cu:46-259). After every step each warp reduces min(rSigmaEff) and
@@ -60,9 +72,9 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
     float* ciddRow = smem;                                    // [nS + 1], the last entry twice
     float* nucWRow = ciddRow + luts.nS + 1;                   // [nS] with the nuclear halo
     float* nucSRow = nucWRow + (kNuclear ? luts.nS : 0);      // [nS] with the nuclear halo
-    float* stepNum = nucSRow + (kNuclear ? luts.nS : 0);      // [steps] 0.5 (voxel width x + y)
-    float* stepVolT = stepNum + g.steps;                      // [steps] step volume
-    float* partMin = stepVolT + g.steps;                      // [steps][8]
+    // [steps] (0.5 (voxel width x + y), step volume)
+    float2* stepGeo = reinterpret_cast<float2*>(ciddRow + (((kNuclear ? 3 : 1) * luts.nS + 2) & ~1));
+    float* partMin = reinterpret_cast<float*>(stepGeo + g.steps);              // [steps][8]
     unsigned* partRange = reinterpret_cast<unsigned*>(partMin + g.steps * 8);  // [steps][8]
     __shared__ int shHist[kBuckets], shLive[kBuckets], shPassive[8], shEnd;
 
@@ -79,6 +91,42 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
     const LayerParamsDev p = lp[l];
     const int first = beam->firstInside;
     const int afterLastL = ls[l].afterLast;
+
+    const bool real = x < g.rayX && y < g.rayY;
+    const size_t rayPlane = static_cast<size_t>(g.rayX) * g.rayY;
+    const size_t padPlane = static_cast<size_t>(g.pitchX) * g.pitchY;
+    const size_t layerStride = static_cast<size_t>(g.steps) * padPlane;
+    // This thread's source of the tile (tile-major planes).
+    float2* srcL = sources + lc * layerStride + static_cast<size_t>(ty * g.tilesX + tx) * kTileSources + tid;
+    const size_t ridx = static_cast<size_t>(y) * g.rayX + x;
+
+    int firstIn = 0;
+    unsigned int afterLast = 0;
+    float rayWeight = 0.0f;
+    bool live = false;
+    if (real) {
+        firstIn = firstInside[ridx];
+        afterLast = static_cast<unsigned int>(min(firstOutside[ridx], afterLastL));
+        rayWeight = rayW[static_cast<size_t>(l) * rayPlane + ridx];
+        live = true;
+        if (rayWeight < 1e-6f || afterLast < static_cast<unsigned int>(first)) {
+            live = false;
+            afterLast = 0;
+        }
+    }
+    // No live ray: every step's bucket is 0 and nothing reads the tile's sources.
+    if (!__syncthreads_or(live) && !g.fillDeadTiles) {
+        const int nSteps = max(afterLastL - first, 0);
+        const size_t tiles = static_cast<size_t>(g.tilesX) * g.tilesY;
+        uint8_t* code = codes + static_cast<size_t>(lc) * g.steps * tiles + static_cast<size_t>(ty) * g.tilesX + tx;
+        for (int zr = tid; zr < nSteps; zr += 256) code[zr * tiles] = 0;
+        if (real && firstPassiveOut) firstPassiveOut[static_cast<size_t>(lc) * rayPlane + ridx] = 0;
+        if (tid == 0) {
+            if (nSteps > 0) atomicAdd(&ls[l].histAll[0], nSteps);
+            atomicMax(&ls[l].maxFirstPassive, 0);
+        }
+        return;
+    }
 
     // CIDD row of this layer's energy: the bilinear CIDD texture lookup at a fixed
     // energy coordinate is a depth lerp of the energy-interpolated row.
@@ -115,9 +163,9 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
             const float zk = g.fanCorner.z + float(k) * g.fanDelta.z;
             const float vwx = g.fanDelta.x * (1.0f - zk / g.sourceDist.x);
             const float vwy = g.fanDelta.y * (1.0f - zk / g.sourceDist.y);
-            stepNum[k] = 0.5f * (vwx + vwy);
             const unsigned int ku = static_cast<unsigned int>(k);
-            stepVolT[k] = g.volConst + float(ku) * g.volLin + float(ku * ku) * g.volSq;
+            stepGeo[k] = make_float2(0.5f * (vwx + vwy),
+                                     g.volConst + float(ku) * g.volLin + float(ku * ku) * g.volSq);
         }
         if (tid < kBuckets) {
             shHist[tid] = 0;
@@ -126,29 +174,6 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
         if (tid == 0) shEnd = first;
     }
     __syncthreads();
-
-    const bool real = x < g.rayX && y < g.rayY;
-    const size_t rayPlane = static_cast<size_t>(g.rayX) * g.rayY;
-    const size_t padPlane = static_cast<size_t>(g.pitchX) * g.pitchY;
-    const size_t layerStride = static_cast<size_t>(g.steps) * padPlane;
-    // This thread's source of the tile (tile-major planes).
-    float2* srcL = sources + lc * layerStride + static_cast<size_t>(ty * g.tilesX + tx) * kTileSources + tid;
-    const size_t ridx = static_cast<size_t>(y) * g.rayX + x;
-
-    int firstIn = 0;
-    unsigned int afterLast = 0;
-    float rayWeight = 0.0f;
-    bool live = false;
-    if (real) {
-        firstIn = firstInside[ridx];
-        afterLast = static_cast<unsigned int>(min(firstOutside[ridx], afterLastL));
-        rayWeight = rayW[static_cast<size_t>(l) * rayPlane + ridx];
-        live = true;
-        if (rayWeight < 1e-6f || afterLast < static_cast<unsigned int>(first)) {
-            live = false;
-            afterLast = 0;
-        }
-    }
 
     // Nuclear halo of this ray (idd_sigma.cu:88-98, 131-142): only rays under a
     // halo lattice cell carry a halo value; the cell's raw spot weight is its
@@ -189,12 +214,14 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
         nextSp = *nextW;
         nextMat = *nextM;
     }
+    float2* dst = srcL;
     float runMax = 0.0f;  // largest IDD of this ray (fixed-point range of the superposition)
     int stepNo = first;
+#pragma unroll 2
     for (; stepNo < afterLastL; ++stepNo) {
         // Once no ray of the row is live, every later step is (0, +inf): the fill
-        // below writes those without the per-step walk.
-        if (!__any_sync(0xffffffffu, live)) break;
+        // below writes those without the per-step walk (looked at every fourth step).
+        if (!((stepNo - first) & 3) && !__any_sync(0xffffffffu, live)) break;
         float res = 0.0f;
         float rSigmaEff = __int_as_float(0x7f800000);
         float nucRes = 0.0f;
@@ -213,9 +240,9 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
             }
             const float cumulDose = lut_linear_clamp_padded(ciddRow, luts.nS, cumulSp * p.energyScaleFact + 0.5f);
             if (cumulSp < p.peakDepth) {
-                const float resE = kECoef * __powf(p.peakDepth - 0.5f * (cumulSp + cumulSpOld), kPInv);
-                const float betaP = resE + 938.3f - __fdividef(938.3f * 938.3f, resE + 938.3f);
-                const float thetaSq = __fdividef(eRefSq, betaP * betaP) * stepLength * rRl;
+                const float resE = kECoef * pow_normal(p.peakDepth - 0.5f * (cumulSp + cumulSpOld), kPInv);
+                const float betaP = resE + 938.3f - div_normal(938.3f * 938.3f, resE + 938.3f);
+                const float thetaSq = div_normal(eRefSq, betaP * betaP) * stepLength * rRl;
                 sigmaSq += incScat + incDiv;
                 incincScat += 2.0f * thetaSq * stepLength * stepLength;
                 incScat += incincScat;
@@ -223,23 +250,24 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
             } else if (!suppressDip) {
                 sigmaSq -= 1.5f * (incScat + incDiv) * dens;
             }
-            rSigmaEff = __fdividef(stepNum[stepNo], kSqrt2 * (sqrtf(sigmaSq) + sigmaDelta));
-            const float mass = dens * stepVolT[stepNo];
+            const float2 geo = stepGeo[stepNo];
+            rSigmaEff = div_normal(geo.x, kSqrt2 * (sqrtf(sigmaSq) + sigmaDelta));
+            const float mass = dens * geo.y;
             if (nucOn) {
                 const float depthMidIdx = 0.5f * (cumulSp + cumulSpOld) * p.energyScaleFact + 0.5f;
                 if (mass > 1e-2f) {
                     const float nucWeight = lut_linear_clamp_smem(nucWRow, luts.nS, depthMidIdx);
-                    res = __fdividef((1.0f - nucWeight) * rayWeight * (cumulDose - cumulDoseOld), mass);
+                    res = div_normal((1.0f - nucWeight) * rayWeight * (cumulDose - cumulDoseOld), mass);
                     if (nucIdx >= 0)
                         nucRes = __fdividef(nucWeight * nucRayWeight * (cumulDose - cumulDoseOld), mass * spotDist * spotDist);
                 }
                 if (nucIdx >= 0) {
                     const float nucSqSigma = lut_linear_clamp_smem(nucSRow, luts.nS, depthMidIdx);
-                    nucRSigmaEff = 0.5f * spotDist * (2.0f * stepNum[stepNo]) /
+                    nucRSigmaEff = 0.5f * spotDist * (2.0f * stepGeo[stepNo].x) /
                                    (kSqrt2 * sqrtf(sigmaSq + nucSqSigma + entrySigmaSq));
                 }
             } else if (mass > 1e-2f) {
-                res = __fdividef(rayWeight * (cumulDose - cumulDoseOld), mass);
+                res = div_normal(rayWeight * (cumulDose - cumulDoseOld), mass);
             }
             cumulSpOld = cumulSp;
             cumulDoseOld = cumulDose;
@@ -291,7 +319,7 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
                         const float initR2 = p.bp0 + 2.0f * p.bp1 * phy + p.bp2 * phy * phy;
                         const float axisSq = 0.5f * fmaxf(0.0f, initR2 + sumS2 / sumW);
                         const float axis = sqrtf(fmaxf(0.0f, axisSq));
-                        rSigmaEff = 0.5f * stepNum[stepNo] / (kSqrt2 * (axis + 0.21f));
+                        rSigmaEff = 0.5f * stepGeo[stepNo].x / (kSqrt2 * (axis + 0.21f));
                     }
                 }
             }
@@ -302,8 +330,9 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
             }
         }
         runMax = fmaxf(runMax, res);
+        *dst = make_float2(res, rSigmaEff);
+        dst += padPlane;
         const int zr = stepNo - first;
-        srcL[static_cast<size_t>(zr) * padPlane] = make_float2(res, rSigmaEff);
         if (nucIdx >= 0) nucL[static_cast<size_t>(zr) * nucPlane + nucIdx] = make_float2(nucRes, nucRSigmaEff);
 
         // Warp minimum over all rays and range over the depositing ones, on the bits of the
@@ -323,16 +352,14 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
             partRange[zr * 8 + warp] = hi > 0 ? range_word(lo, hi) : 0u;
         }
     }
-    // The row's remaining steps: no dose, rSigmaEff = +inf, nothing live. Past the tile's
+    // The row's remaining steps: no dose, rSigmaEff = +inf, nothing live (the halo's planes
+    // start out like that). Past the tile's
     // last walked step no tile is live and nothing reads its sources.
     if (lane == 0) atomicMax(&shEnd, stepNo);
     __syncthreads();
     const int fillEnd = g.fillDeadTiles ? afterLastL : shEnd;
     for (int k = stepNo; k < fillEnd; ++k)
         srcL[static_cast<size_t>(k - first) * padPlane] = make_float2(0.0f, __int_as_float(0x7f800000));
-    if (nucIdx >= 0)
-        for (int k = stepNo; k < afterLastL; ++k)
-            nucL[static_cast<size_t>(k - first) * nucPlane + nucIdx] = make_float2(0.0f, __int_as_float(0x7f800000));
     for (int zr = stepNo - first + lane; zr < afterLastL - first; zr += 32) {
         partMin[zr * 8 + warp] = __int_as_float(0x7f800000);
         partRange[zr * 8 + warp] = 0;
@@ -774,7 +801,7 @@ cudaError_t launch_idd(const BeamGeomDev& g, const LutsDev& luts, int layer0, in
                        float2* nucSources, cudaStream_t s) {
     dim3 grid(g.tilesX, g.tilesY, nLayers);
     dim3 block(32, 8);
-    const size_t smem = idd_smem(g, static_cast<size_t>(luts.nS) * (g.nucOn ? 3 : 1) + 1);
+    const size_t smem = idd_smem(g, static_cast<size_t>(luts.nS) * (g.nucOn ? 3 : 1) + 2);
     auto k = g.nucOn ? (g.profileMode ? idd_kernel<true, true> : idd_kernel<true, false>)
                      : (g.profileMode ? idd_kernel<false, true> : idd_kernel<false, false>);
     cudaError_t e = set_smem_limit(reinterpret_cast<const void*>(k), smem);
