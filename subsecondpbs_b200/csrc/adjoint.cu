@@ -15,6 +15,7 @@
 #include "work_blocks.cuh"
 #include "kernels.h"
 #include "launch_util.h"
+#include "node_spread.cuh"
 #include "transfer_walk.cuh"
 
 namespace pbs {
@@ -69,225 +70,243 @@ transfer_adjoint_kernel(BeamGeomDev g, const double* __restrict__ gradDose, cons
     });
 }
 
-constexpr int kAdjThreads = 256;
-constexpr int kAdjOutFloats = (kTileY + 2 * kMaxR) * (kTileX + 2 * kMaxR);
-
-// S^T for one tile at radius R: each source gathers the BEV gradient over its
-// footprint with the forward's weights e(|dy|) e(|dx|) and adds idd * that sum to
-// its ray's accumulator.
-constexpr int kAdjEStride = kMaxR + 1;  // 33: odd, the threads' rows fall in distinct banks
-
+// S^T. A source's gradient is the BEV gradient gathered over its footprint with the
+// forward's weights, and those are interpolated between nodes of rSigma as there
+// (node_spread.cuh):
+//   sum_{dy,dx} e_r(dy) e_r(dx) G = sum_j L_j(r) Q_j,  Q_j = E_j(y) * G * E_j(x).
+// One warp takes one item of the forward's merged work list, a tile at one step with all
+// its layers of one radius. The separable convolutions Q_j do not depend on the layer and
+// are done once per item, two nodes (+-x_p) at a time:
+//   * columns: lane = one footprint column, its rows in registers; both nodes' eight
+//     output rows, as the pairs (y, 7 - y), go to shared memory;
+//   * rows: lane = one (node, row pair, eight columns); the results replace the rows;
+//   * lane = source column: A_p = C_p x_p (Q+ + Q-), D_p = C_p (Q+ - Q-);
+// then every layer's sources add idd sum_p B_p(t^2) (A_p + t D_p) to their rays. Bound by
+// FMA issue in the convolutions. Gathering (2R+1)^2 cells for every source and layer, as
+// pair sums, took 342 us in place of 99 us (36 layers on 64 x 64 x 128 voxels of 2 mm).
 template <int R>
-__device__ __forceinline__ void superpose_adjoint_tile(const float* __restrict__ tileG, float* __restrict__ eRow,
-                                                       float dose, float rs, float* __restrict__ rbarRay, int sy,
-                                                       int sx) {
-    constexpr int Wo = kTileX + 2 * R;
-    float e[R + 1];
-    superposition_row<R>(rs, e);
-#pragma unroll
-    for (int k = 0; k <= R; ++k) eRow[k] = e[k];
-    // Rows R-k and R+k share the weight e[k]; within a row the columns R-j and
-    // R+j share e[j] (kept in registers; the row weight comes from eRow).
-    auto row_sum = [&](int i) {
-        const float* row = tileG + (sy + i) * Wo + sx + R;
-        float v = e[0] * row[0];
-#pragma unroll
-        for (int j = 1; j <= R; ++j) v = fmaf(e[j], row[-j] + row[j], v);
-        return v;
-    };
-    float acc = e[0] * row_sum(R);
+__device__ __forceinline__ void gather_columns(const float* __restrict__ src, int bevX, const float2* __restrict__ e,
+                                               float2* __restrict__ rows, int lane) {
+    constexpr int W = kTileX + 2 * R, H = kTileY + 2 * R, N = H / 2;
 #pragma unroll 1
-    for (int k = 1; k <= R; ++k) acc = fmaf(eRow[k], row_sum(R - k) + row_sum(R + k), acc);
-    atomicAdd(rbarRay, dose * acc);
-}
-
-// S^T for one tile at radius R <= kSplitR, in the forward's (source column, |d|)
-// pair form. A source's gradient is
-//   sum_d e(d) P_d,  P_d = sum_k e(|k|) c_d[sy + R + k],
-// where c_d is the sum of the footprint's gradient columns sx + R + d and
-// sx + R - d (one column for d = 0), the same for the eight sources of the column.
-// A lane is one (column, |d|) pair: it sums its two gradient columns once into
-// registers, then forms P_d for the column's eight sources with their weights read
-// as broadcast float4 chunks, and stores them; each source thread then sums
-// e(d) P_d over d. The shared-memory reads per source drop from (2R+1)^2 scalars
-// to about (2H + 8 Q)/8 per pair.
-template <int R>
-__device__ __forceinline__ void superpose_adjoint_pairs(const float* __restrict__ tileG, float4* __restrict__ E4,
-                                                        float* __restrict__ P, float dose, float rs,
-                                                        float* __restrict__ rbarRay) {
-    constexpr int H = kTileY + 2 * R;
-    constexpr int Wo = kTileX + 2 * R;
-    constexpr int Q = (R + 1 + 3) / 4;
-    constexpr int PS = (R + 1) | 1;             // odd row stride of P
-    constexpr int M = R + 1;
-    constexpr int G = 32 / M;                   // source columns per warp instruction
-    constexpr int S = (32 + G - 1) / G;         // column spacing, units
-    const int t = threadIdx.x;
-    const int warp = t >> 5, lane = t & 31;
-    const bool live = rbarRay != nullptr;
-    // Weights of source t = (sy, sx) = (warp, lane), chunk-major with the column
-    // swizzle of the forward kernel.
-    float e[4 * Q];
-    if (live) {
-        float row[R + 1];
-        superposition_row<R>(rs, row);
+    for (int x = lane; x < W; x += 32) {
+        float2 t[N];
 #pragma unroll
-        for (int k = 0; k <= R; ++k) e[k] = row[k];
-    } else {
-#pragma unroll
-        for (int k = 0; k <= R; ++k) e[k] = 0.0f;
-    }
-#pragma unroll
-    for (int k = R + 1; k < 4 * Q; ++k) e[k] = 0.0f;
-    const int col = lane ^ ((lane >> 3) & 3);
-#pragma unroll
-    for (int q = 0; q < Q; ++q)
-        E4[q * kAdjThreads + warp * kTileX + col] = make_float4(e[4 * q], e[4 * q + 1], e[4 * q + 2], e[4 * q + 3]);
-    __syncthreads();
+        for (int i = 0; i < N; ++i) t[i] = make_float2(__ldg(src + i * bevX + x), __ldg(src + (H - 1 - i) * bevX + x));
 #pragma unroll 1
-    for (int u = warp; u < S; u += kAdjThreads / 32) {
-        const int g = lane / M;
-        int d = lane - g * M;
-        int sx = u + g * S;
-        const bool valid = g < G && sx < kTileX;
-        if (!valid) {
-            sx = 0;
-            d = 0;
-        }
-        float c[H];
-        const float* ca = tileG + sx + R + d;
-        const float* cb = tileG + sx + R - d;
+        for (int j = 0; j < 2; ++j) {
+            float2 acc[kPairs];
 #pragma unroll
-        for (int i = 0; i < H; ++i) c[i] = ca[i * Wo] + (d > 0 ? cb[i * Wo] : 0.0f);
-        const float4* eCol = E4 + (sx ^ ((sx >> 3) & 3));
+            for (int y = 0; y < kPairs; ++y) acc[y] = make_float2(0.0f, 0.0f);
+            const float4* e4 = reinterpret_cast<const float4*>(e + j * kTableStride<R>);
 #pragma unroll
-        for (int sy = 0; sy < kTileY; ++sy) {
-            float ev[4 * Q];
+            for (int q = 0; q < (R + 2) / 2; ++q) {
+                const float4 w = e4[q];
+                const float2 wk[2] = {make_float2(w.x, w.y), make_float2(w.z, w.w)};
 #pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                const float4 v = eCol[q * kAdjThreads + sy * kTileX];
-                ev[4 * q] = v.x;
-                ev[4 * q + 1] = v.y;
-                ev[4 * q + 2] = v.z;
-                ev[4 * q + 3] = v.w;
+                for (int c = 0; c < 2; ++c) {
+                    const int k = 2 * q + c;
+                    if (k <= R) {
+#pragma unroll
+                        for (int y = 0; y < kPairs; ++y) {
+                            const int i0 = y + R - k, i1 = y + R + k;
+                            const float2 lo = i0 < N ? t[i0 < N ? i0 : 0] : make_float2(t[H - 1 - i0].y, t[H - 1 - i0].x);
+                            const float2 hi = i1 < N ? t[i1 < N ? i1 : 0] : make_float2(t[H - 1 - i1].y, t[H - 1 - i1].x);
+                            acc[y] = __ffma2_rn(lo, wk[c], acc[y]);
+                            if (k > 0) acc[y] = __ffma2_rn(hi, wk[c], acc[y]);
+                        }
+                    }
+                }
             }
-            float pd = ev[0] * c[sy + R];
 #pragma unroll
-            for (int k = 1; k <= R; ++k) pd = fmaf(ev[k], c[sy + R - k] + c[sy + R + k], pd);
-            if (valid) P[(sy * kTileX + sx) * PS + d] = pd;
+            for (int y = 0; y < kPairs; ++y) rows[(j * kPairs + y) * kRowStride<R> + x] = acc[y];
         }
-    }
-    __syncthreads();
-    if (live) {
-        float acc = 0.0f;
-#pragma unroll
-        for (int k = 0; k <= R; ++k) acc = fmaf(e[k], P[t * PS + k], acc);
-        atomicAdd(rbarRay, dose * acc);
     }
 }
 
-// Radii above kSplitR gather per source (superpose_adjoint_tile); the others run
-// in pair form with every thread of the CTA (rbarRay null: no live source).
-template <int R, int RHi>
-__device__ __forceinline__ void adjoint_dispatch(int r, const float* tileG, float* eRow, float4* E4, float* P,
-                                                 float dose, float rs, float* rbarRay, int sy, int sx) {
-    if (r == R) {
-        if constexpr (R <= kSplitR) {
-            superpose_adjoint_pairs<R>(tileG, E4, P, dose, rs, rbarRay);
-        } else {
-            if (rbarRay) superpose_adjoint_tile<R>(tileG, eRow, dose, rs, rbarRay, sy, sx);
+// The eight rows of two nodes, each convolved along x over its 32 sources: the result of
+// source column sx lies at sx. Lanes of one half-warp read distinct banks (odd stride).
+template <int R>
+__device__ __forceinline__ void gather_rows(float2* __restrict__ rows, const float2* __restrict__ e, int lane) {
+    constexpr int kOut = kTileX / 4;
+    const int row = lane & 7;
+    float2 k[kTableStride<R>];
+    const float4* e4 = reinterpret_cast<const float4*>(e + (row / kPairs) * kTableStride<R>);
+#pragma unroll
+    for (int q = 0; q < (R + 2) / 2; ++q) {
+        const float4 v = e4[q];
+        k[2 * q] = make_float2(v.x, v.y);
+        k[2 * q + 1] = make_float2(v.z, v.w);
+    }
+    float2* p = rows + row * kRowStride<R> + (lane >> 3) * kOut;
+    float2 acc[kOut];
+#pragma unroll
+    for (int o = 0; o < kOut; ++o) acc[o] = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int i = 0; i < kOut + 2 * R; ++i) {
+        const float2 v = p[i];
+#pragma unroll
+        for (int o = 0; o < kOut; ++o) {
+            const int d = i - o - R, a = d < 0 ? -d : d;
+            if (a <= R) acc[o] = __ffma2_rn(v, k[a <= R ? a : 0], acc[o]);
         }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 0; o < kOut; ++o) p[o] = acc[o];
+}
+
+template <int R, int RHi>
+__device__ __forceinline__ void gather_item(int r, const float* src, int bevX, const float2* e, float2* rows, int lane) {
+    if (r == R) {
+        gather_columns<R>(src, bevX, e, rows, lane);
+        __syncwarp();
+        gather_rows<R>(rows, e, lane);
         return;
     }
-    if constexpr (R < RHi) adjoint_dispatch<R + 1, RHi>(r, tileG, eRow, E4, P, dose, rs, rbarRay, sy, sx);
+    if constexpr (R < RHi) gather_item<R + 1, RHi>(r, src, bevX, e, rows, lane);
 }
 
-// Shared memory of an instance for radii up to RHi: the tile's gradient footprint,
-// then either the pair form's weight chunks and pair sums (RHi <= kSplitR) or each
-// source's weight row.
-template <int RHi>
-struct AdjShape {
-    static constexpr int kTile = (kTileY + 2 * RHi) * (kTileX + 2 * RHi);  // 16(4+R)(16+R) bytes: 16-byte aligned
-    static constexpr bool kPairs = RHi <= kSplitR;
-    static constexpr int kQ = (RHi + 1 + 3) / 4;
-    static constexpr int kPS = (RHi + 1) | 1;
-    static constexpr int kRest = kPairs ? kQ * kAdjThreads * 4 + kAdjThreads * kPS : kAdjThreads * kAdjEStride;
-    static constexpr size_t kSmemBytes = size_t(kTile + kRest) * sizeof(float);
+// The sources of an item's layers: idd times the interpolated gradient into their rays.
+struct SourceGradients {
+    const TileSource& s;
+    const NodeRange& n;
+    unsigned layers;
+    const float2* ad;  // (A_p, D_p) [p][2][4][32]
+    float* rbar;       // the lane's ray of row 0 in the first layer of the item's group
+    size_t rayPlane;
+    int rayX, lane;
+
+    template <int J>
+    __device__ __forceinline__ void run() const {
+        const float2 shift = make_float2(n.shift, n.shift), inv = make_float2(n.invHalf, n.invHalf);
+        float2 a[kPairs][J / 2], d[kPairs][J / 2];
+#pragma unroll
+        for (int p = 0; p < J / 2; ++p)
+#pragma unroll
+            for (int y = 0; y < kPairs; ++y) {
+                a[y][p] = ad[((p * 2) * kPairs + y) * kTileX + lane];
+                d[y][p] = ad[((p * 2 + 1) * kPairs + y) * kTileX + lane];
+            }
+#pragma unroll 1
+        for (unsigned m = layers; m; m &= m - 1u) {
+            const int l = __ffs(m) - 1;
+            const float2* f = s.first + l * s.layerStride + lane;
+            float* out = rbar + l * rayPlane;
+            float2 src[kTileY];
+#pragma unroll
+            for (int y = 0; y < kTileY; ++y) src[y] = f[y * kTileX];
+#pragma unroll
+            for (int y = 0; y < kPairs; ++y) {
+                const float2 u = src[y], v = src[kTileY - 1 - y];
+                float2 dose;
+                dose.x = u.y > n.from && u.y <= n.to ? fmaxf(u.x, 0.0f) : 0.0f;
+                dose.y = v.y > n.from && v.y <= n.to ? fmaxf(v.x, 0.0f) : 0.0f;
+                const float2 t = __ffma2_rn(make_float2(fminf(u.y, n.top), fminf(v.y, n.top)), inv, shift);
+                float2 b[J / 2];
+                pair_products<J>(__fmul2_rn(t, t), b);
+                float2 acc = make_float2(0.0f, 0.0f);
+#pragma unroll
+                for (int p = 0; p < J / 2; ++p) acc = __ffma2_rn(b[p], __ffma2_rn(t, d[y][p], a[y][p]), acc);
+                // Rays outside the ray grid carry no dose.
+                if (dose.x > 0.0f) atomicAdd(out + y * rayX, dose.x * acc.x);
+                if (dose.y > 0.0f) atomicAdd(out + (kTileY - 1 - y) * rayX, dose.y * acc.y);
+            }
+        }
+    }
 };
 
-// Persistent CTAs over the radii RLo..RHi of the chunk's one-layer work list, taken
-// radius block by radius block through the range's counter as in the forward
-// superposition. The three instances of a beam overlap in the same way: each CTA
-// lets the next instance launch at once (their items only add into the rays'
-// accumulators) and waits for the previous instance before it exits.
-template <int RLo, int RHi, int MinBlocks>
-__global__ void __launch_bounds__(kAdjThreads, MinBlocks)
-superpose_adjoint_kernel(BeamGeomDev g, const float2* __restrict__ sources,
-                         const int4* __restrict__ work, BeamStateDev* __restrict__ beam, const float* __restrict__ gradBev,
-                         float* __restrict__ rbar, int range) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    extern __shared__ __align__(16) float adjSm[];
-    using Sh = AdjShape<RHi>;
-    float* tileG = adjSm;                        // [8+2R][32+2R] BEV gradient of the tile's footprint
-    float* eS = adjSm + Sh::kTile;               // [256][kAdjEStride] each source's weights (R > kSplitR)
-    float4* E4 = reinterpret_cast<float4*>(eS);  // pair form: weight chunks [Q][256] ...
-    float* P = eS + Sh::kQ * kAdjThreads * 4;    // ... and pair sums [256][PS]
-    __shared__ int sItem[2];
+// Shared memory of a warp (pairs): two nodes' tables, their eight rows, and A and D.
+template <int RMax>
+constexpr int kAdjWarpPairs = 2 * kTableStride<RMax> + 2 * kPairs * kRowStride<RMax> + kMaxNodes * kPairs * kTileX;
+
+// Persistent warps over the items of radii RLo..RHi, claimed through the range's counter.
+// The three instances of a beam overlap as the forward's do: each CTA lets the next
+// instance launch at once (their items only add into the rays' accumulators) and waits
+// for the previous instance before it exits.
+template <int RLo, int RHi, int Warps, int MinBlocks>
+__global__ void __launch_bounds__(Warps * 32, MinBlocks)
+superpose_adjoint_kernel(BeamGeomDev g, const float2* __restrict__ sources, const unsigned* __restrict__ tileRange,
+                         const int4* __restrict__ work, BeamStateDev* __restrict__ beam,
+                         const float* __restrict__ gradBev, float* __restrict__ rbar) {
+    pdl_trigger();
+    extern __shared__ __align__(16) float2 adjSm[];
     __shared__ RadiusBlocks<RLo, RHi> sBlocks;
-    const int t = threadIdx.x;
-    int* counter = range == 0 ? &beam->workNext : (range == 1 ? &beam->workNextSmall : &beam->workNextTiny);
-    const size_t padPlane = static_cast<size_t>(g.pitchX) * g.pitchY;
-    const size_t layerStride = static_cast<size_t>(g.steps) * padPlane;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int* counter = RLo > kSplitWide ? &beam->workNext : (RLo > kSplitR ? &beam->workNextSmall : &beam->workNextTiny);
+    const int tiles = g.tilesX * g.tilesY;
+    const size_t padPlane = static_cast<size_t>(tiles) * kTileSources;
     const size_t bevPlane = static_cast<size_t>(g.bevX) * g.bevY;
     const size_t rayPlane = static_cast<size_t>(g.rayX) * g.rayY;
+    float2* e = adjSm + warp * kAdjWarpPairs<RHi>;
+    float2* rows = e + 2 * kTableStride<RHi>;
+    float2* ad = rows + 2 * kPairs * kRowStride<RHi>;
+
     load_blocks<RLo, RHi>(beam, sBlocks);
-    if (t == 0) sItem[0] = atomicAdd(counter, 1);
     __syncthreads();
-    int buf = 0;
-    for (;;) {
-        const int c = sItem[buf];
-        if (c >= sBlocks.total) break;
-        if (t == 0) sItem[buf ^ 1] = atomicAdd(counter, 1);
+    const int total = sBlocks.total, warps = gridDim.x * Warps;
+    // The first item of every warp is fixed; the counter deals out the others.
+    for (int c = blockIdx.x + warp * gridDim.x; c < total;) {
+        int claim = 0;
+        if (lane == 0) claim = warps + atomicAdd(counter, 1);
         const int4 it = work[block_slot<RLo, RHi>(sBlocks, c)];
-        const int lc = (it.w >> 8) + __ffs(it.x) - 1, tile = it.y, zRel = it.z, R = it.w & 0xff;
+        c = __shfl_sync(0xffffffffu, claim, 0);
+        const unsigned layers = static_cast<unsigned>(it.x);
+        const int tile = it.y, zRel = it.z, R = it.w & 0xff, base = it.w >> 8;
+        if (R < RLo || R > RHi) {
+            if (lane == 0) atomicOr(&beam->errorFlags, 2);
+            continue;
+        }
+        unsigned range = 0;
+        if (layers >> lane & 1u)
+            range = tileRange[(static_cast<size_t>(base + lane) * g.steps + zRel) * tiles + tile];
+        TileSource s;
+        s.layerStride = static_cast<size_t>(g.steps) * padPlane;
+        s.first = sources + base * s.layerStride + zRel * padPlane + tile * kTileSources;
+        prefetch_tile(s, layers, lane);
+        float lo, hi;
+        if (!item_range(range, lo, hi)) continue;
         const int tx = tile % g.tilesX, ty = tile / g.tilesX;
-        const int Ho = kTileY + 2 * R, Wo = kTileX + 2 * R;
         const float* src = gradBev + static_cast<size_t>(zRel) * bevPlane +
                            static_cast<size_t>(ty * kTileY - R + kMaxR) * g.bevX + (tx * kTileX - R + kMaxR);
-        for (int i = t; i < Ho * Wo; i += kAdjThreads) {
-            const int oy = i / Wo, ox = i - oy * Wo;
-            tileG[i] = src[static_cast<size_t>(oy) * g.bevX + ox];
+        float* out = rbar + base * rayPlane + static_cast<size_t>(ty * kTileY) * g.rayX + tx * kTileX + lane;
+        const int stride = kTileX + 2 * R + 1, eStride = ((R + 2) / 2 | 1) * 2;
+        for (float from = 0.0f;;) {
+            const NodeRange n = node_range(from, lo, hi);
+#pragma unroll 1
+            for (int p = 0; p < n.count / 2; ++p) {
+                node_tables(n, 2 * p, 2, R, e, eStride, lane);
+                __syncwarp();
+                gather_item<RLo, RHi>(R, src, g.bevX, e, rows, lane);
+                __syncwarp();
+                const float cp = kNodeC[n.count / 2 - 2][p], cx = cp * kNodeX[n.count / 2 - 2][p];
+#pragma unroll
+                for (int y = 0; y < kPairs; ++y) {
+                    const float2 qp = rows[y * stride + lane], qm = rows[(kPairs + y) * stride + lane];
+                    ad[((p * 2) * kPairs + y) * kTileX + lane] = make_float2(cx * (qp.x + qm.x), cx * (qp.y + qm.y));
+                    ad[((p * 2 + 1) * kPairs + y) * kTileX + lane] = make_float2(cp * (qp.x - qm.x), cp * (qp.y - qm.y));
+                }
+                __syncwarp();
+            }
+            with_nodes(n.count, SourceGradients{s, n, layers, ad, out, rayPlane, g.rayX, lane});
+            if (n.top >= hi) break;
+            from = lo = n.top;
         }
-        __syncthreads();
-        const int sy = t >> 5, sx = t & 31;
-        const int ry = ty * kTileY + sy, rx = tx * kTileX + sx;
-        const size_t s = lc * layerStride + zRel * padPlane + static_cast<size_t>(tile) * kTileSources + t;
-        const float2 source = sources[s];
-        const float dose = source.x;
-        const bool live = dose > 0.0f && ry < g.rayY && rx < g.rayX;
-        if (R >= RLo && R <= RHi)
-            adjoint_dispatch<RLo, RHi>(R, tileG, eS + t * kAdjEStride, E4, P, dose, live ? source.y : 0.0f,
-                                       live ? rbar + lc * rayPlane + static_cast<size_t>(ry) * g.rayX + rx : nullptr,
-                                       sy, sx);
-        // Every thread is past the item (and has read sItem[buf]) before the next
-        // claim lands in that slot.
-        __syncthreads();
-        buf ^= 1;
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();
 }
 
-template <int RLo, int RHi, int MinBlocks>
-cudaError_t launch_adjoint_range(const BeamGeomDev& g, const float2* sources, const int4* work,
-                                 BeamStateDev* beam, const float* gradBev, float* rbar, int numSMs, int range,
+template <int RLo, int RHi, int Warps, int MinBlocks>
+cudaError_t launch_adjoint_range(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange,
+                                 const int4* work, BeamStateDev* beam, const float* gradBev, float* rbar, int numSMs,
                                  bool overlap, cudaStream_t s) {
-    auto k = superpose_adjoint_kernel<RLo, RHi, MinBlocks>;
-    const size_t smem = AdjShape<RHi>::kSmemBytes;
+    auto k = superpose_adjoint_kernel<RLo, RHi, Warps, MinBlocks>;
+    const size_t smem = size_t(Warps) * kAdjWarpPairs<RHi> * sizeof(float2);
     cudaError_t e = set_smem_limit(reinterpret_cast<const void*>(k), smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(numSMs * MinBlocks);
-    cfg.blockDim = dim3(kAdjThreads);
+    cfg.blockDim = dim3(Warps * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -295,13 +314,8 @@ cudaError_t launch_adjoint_range(const BeamGeomDev& g, const float2* sources, co
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = overlap ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k, g, sources, work, beam, gradBev, rbar, range);
+    return cudaLaunchKernelEx(&cfg, k, g, sources, tileRange, work, beam, gradBev, rbar);
 }
-
-// Resident CTAs per SM of the adjoint instances (radii 16..32, 8..15, 0..7).
-constexpr int kAdjWideBlocks = 3;
-constexpr int kAdjMidBlocks = 4;
-constexpr int kAdjNarrowBlocks = 6;
 
 }  // namespace
 
@@ -315,19 +329,16 @@ cudaError_t launch_transfer_adjoint(const BeamGeomDev& g, const double* gradDose
     return cudaGetLastError();
 }
 
-cudaError_t launch_superpose_adjoint(const BeamGeomDev& g, const float2* sources, const int4* work,
-                                     BeamStateDev* beam, const float* gradBev, float* rbar, int numSMs,
-                                     cudaStream_t s) {
-    cudaError_t e = launch_one_layer_list_view(beam, s);
+cudaError_t launch_superpose_adjoint(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange,
+                                     const int4* work, BeamStateDev* beam, const float* gradBev, float* rbar,
+                                     int numSMs, cudaStream_t s) {
+    cudaError_t e = launch_adjoint_range<kSplitWide + 1, kMaxR, 4, 2>(g, sources, tileRange, work, beam, gradBev, rbar,
+                                                                      numSMs, false, s);
     if (e != cudaSuccess) return e;
-    e = launch_adjoint_range<kSplitR + 1, kMaxR, kAdjWideBlocks>(g, sources, work, beam, gradBev, rbar, numSMs,
-                                                                 0, false, s);
+    e = launch_adjoint_range<kSplitR + 1, kSplitWide, 4, 3>(g, sources, tileRange, work, beam, gradBev, rbar, numSMs,
+                                                            true, s);
     if (e != cudaSuccess) return e;
-    e = launch_adjoint_range<kSplitR2 + 1, kSplitR, kAdjMidBlocks>(g, sources, work, beam, gradBev, rbar, numSMs,
-                                                                   1, true, s);
-    if (e != cudaSuccess) return e;
-    return launch_adjoint_range<0, kSplitR2, kAdjNarrowBlocks>(g, sources, work, beam, gradBev, rbar, numSMs, 2,
-                                                               true, s);
+    return launch_adjoint_range<0, kSplitR, 4, 4>(g, sources, tileRange, work, beam, gradBev, rbar, numSMs, true, s);
 }
 
 }  // namespace pbs

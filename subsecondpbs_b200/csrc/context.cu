@@ -1377,7 +1377,7 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
                  "idd");
         if (l0 == 0 && (rc = mark(4))) return rc;
         PBS_CUDA(launch_bin_plan(g, l0, nl, static_cast<const uint8_t*>(codes.ptr), dls, dbs,
-                                 static_cast<int4*>(work.ptr), workCap, adj == nullptr && !columnLists, nullptr,
+                                 static_cast<int4*>(work.ptr), workCap, !columnLists, nullptr,
                                  nullptr, stream),
                  "bin_plan");
         if (nuclear) {
@@ -1385,7 +1385,7 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
                                       static_cast<uint8_t*>(nucCodes.ptr), stream),
                      "nuc_codes");
             PBS_CUDA(launch_bin_plan(nucGeom, l0, nl, static_cast<const uint8_t*>(nucCodes.ptr), dNucLs, dNucBs,
-                                     static_cast<int4*>(nucWork.ptr), nucWorkCap, adj == nullptr, dls, dbs, stream),
+                                     static_cast<int4*>(nucWork.ptr), nucWorkCap, true, dls, dbs, stream),
                      "nuc_bin_plan");
         }
         if (l0 == 0 && (rc = mark(5))) return rc;
@@ -1502,6 +1502,7 @@ int Context::finish_adjoint(const AdjointArgs& a, const PbsBeamDesc& b) {
     PBS_CUDA(cudaMemsetAsync(rbarBuf.ptr, 0, L * rays * 4, stream), "memset");
     PBS_CUDA(launch_transfer_adjoint(g, a.gradDose, dbs, static_cast<float*>(bevGrad.ptr), stream), "transfer_adjoint");
     PBS_CUDA(launch_superpose_adjoint(g, static_cast<const float2*>(sources.ptr),
+                                      static_cast<const unsigned*>(tileRange.ptr),
                                       static_cast<const int4*>(work.ptr), dbs, static_cast<const float*>(bevGrad.ptr),
                                       static_cast<float*>(rbarBuf.ptr), smCount, stream),
              "superpose_adjoint");

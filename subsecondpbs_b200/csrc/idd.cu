@@ -425,13 +425,11 @@ layer_plan_kernel(BeamGeomDev g, int layer0, int nLayers, LayerStateDev* __restr
     __shared__ int sCalc[kMaxChunkLayers];
     __shared__ int sWarpSum[kMaxChunkLayers / 32];
     __shared__ long long sWarpFma[kMaxChunkLayers / 32];
-    __shared__ int sSplit[2];
     pdl_trigger();
     const int lc = threadIdx.x;
     const bool nuclear = primaryLs != nullptr;
     const int first = nuclear ? primaryBeam->firstInside : beam->firstInside;
     const int tiles = g.tilesX * g.tilesY;
-    if (lc < 2) sSplit[lc] = 0;
     if (lc < nLayers) {
         LayerStateDev& st = ls[layer0 + lc];
         // Every input of the layer is read before its outputs are written: the outputs
@@ -528,11 +526,8 @@ layer_plan_kernel(BeamGeomDev g, int layer0, int nLayers, LayerStateDev* __restr
     __syncthreads();
     int acc = incl - runSum;
     for (int w = 0; w < warp; ++w) acc += sWarpSum[w];
-    const int pSplit = (kMaxR - kSplitR) * nLayers, pSplit2 = (kMaxR - kSplitR2) * nLayers;
     for (int p = p0; p < p1; ++p) {
         const int r = kMaxR - p / nLayers, q = p % nLayers;
-        if (p == pSplit) sSplit[0] = acc;
-        if (p == pSplit2) sSplit[1] = acc;
         ls[layer0 + q].offR[r] = acc;
         if (q == 0) beam->rStart[r] = acc;
         acc += sLive[q][r];
@@ -550,7 +545,6 @@ layer_plan_kernel(BeamGeomDev g, int layer0, int nLayers, LayerStateDev* __restr
             acc += sWarpSum[w];
             fma += sWarpFma[w];
         }
-        const int split = sSplit[0], split2 = sSplit[1];
         int mp = beam->maxCalcPassive;
         for (int q = 0; q < nLayers; ++q) mp = max(mp, sCalc[q]);
         beam->maxCalcPassive = mp;
@@ -560,9 +554,7 @@ layer_plan_kernel(BeamGeomDev g, int layer0, int nLayers, LayerStateDev* __restr
         }
         beam->workCount = acc;
         beam->workNext = 0;
-        beam->workSplit = min(split, acc);
         beam->workNextSmall = 0;
-        beam->workSplit2 = min(split2, acc);
         beam->workNextTiny = 0;
         for (int r = 0; r <= kMaxR; ++r) beam->mergedR[r] = 0;
         // Fixed-point range of the chunk's BEV: a cell sums at most `acc` tile

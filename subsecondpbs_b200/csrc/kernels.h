@@ -120,9 +120,6 @@ cudaError_t launch_nuc_codes(const BeamGeomDev& gn, int layer0, int nLayers, con
 cudaError_t launch_superpose(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange, const int4* work,
                              BeamStateDev* beam, float* bev, unsigned long long* bevFixed, int shiftOffset,
                              int numSMs, cudaStream_t s);
-// Radius blocks and claim counters of the chunk's one-layer work list
-// (merged == false in launch_bin_plan), for the superposition kernels.
-cudaError_t launch_one_layer_list_view(BeamStateDev* beam, cudaStream_t s);
 // Batched influence columns: the chunk's whole one-layer work list (layers
 // [0, nCols) of `ls`), item layer q into BEV volume q (bev / bevFixed + q * stride
 // cells), each volume converted over its layer's live cells.
@@ -146,9 +143,9 @@ cudaError_t launch_transfer(const BeamGeomDev& g, const float* bev, const BeamSt
 cudaError_t launch_transfer_adjoint(const BeamGeomDev& g, const double* gradDose, const BeamStateDev* beam,
                                     float* gradBev, cudaStream_t s);
 // S^T and the IDD scaling over the chunk's work list: rbar[l][ray] += idd * (S^T gradBev).
-cudaError_t launch_superpose_adjoint(const BeamGeomDev& g, const float2* sources, const int4* work,
-                                     BeamStateDev* beam, const float* gradBev, float* rbar, int numSMs,
-                                     cudaStream_t s);
+cudaError_t launch_superpose_adjoint(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange,
+                                     const int4* work, BeamStateDev* beam, const float* gradBev, float* rbar,
+                                     int numSMs, cudaStream_t s);
 // Transposed spot -> ray convolution (mode A): gradLattice[l][iy][ix] from rbar / rayW.
 cudaError_t launch_conv_lattice_adjoint(const BeamGeomDev& g, const float* rbar, const float* rayW, float* gradInterm,
                                         float* gradLattice, const LayerStateDev* ls, const BeamStateDev* beam,

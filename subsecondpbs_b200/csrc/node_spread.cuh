@@ -26,6 +26,16 @@
 namespace pbs {
 
 constexpr int kMaxNodes = 8;
+constexpr int kSplitWide = 23;  // widest radius of the second of the three instances
+
+// Rows of a tile in pairs (y and 7 - y, the two halves of packed FP32 operations), and
+// strides of a pair's row and of a node's table in shared memory.
+constexpr int kPairs = kTileY / 2;
+template <int R>
+constexpr int kRowStride = kTileX + 2 * R + 1;
+template <int R>
+constexpr int kTableStride = ((R + 2) / 2 | 1) * 2;
+
 // r above which e_r is (1, 0, 0, ...) in 32 bits: larger values (a zero sigma) are
 // taken as this.
 constexpr float kMaxRSigma = 12.0f;
@@ -37,10 +47,10 @@ constexpr float kSmallRSigma = 0.02f;
 // Chebyshev nodes +-cos((2p+1) pi / 2J), p < J/2, of J = 4, 6, 8 nodes, and
 // 1 / (2 x_p prod_{q != p} (x_p^2 - x_q^2)). Node 2p is +x_p, node 2p+1
 // is -x_p. Even counts only: the two nodes of a pair share their basis product.
-__constant__ float kNodeX[kMaxNodes / 2 - 1][kMaxNodes / 2] = {{0.9238795f, 0.38268343f},
+static __constant__ float kNodeX[kMaxNodes / 2 - 1][kMaxNodes / 2] = {{0.9238795f, 0.38268343f},
                                                            {0.9659258f, 0.70710677f, 0.25881904f},
                                                            {0.98078525f, 0.8314696f, 0.55557024f, 0.19509032f}};
-__constant__ float kNodeC[kMaxNodes / 2 - 1][kMaxNodes / 2] = {{0.76536694f, -1.84775922f},
+static __constant__ float kNodeC[kMaxNodes / 2 - 1][kMaxNodes / 2] = {{0.76536694f, -1.84775922f},
                                                            {1.38036833f, -3.77123645f, 5.15160478f},
                                                            {3.12144614f, -8.88912625f, 13.3035158f, -15.6925653f}};
 
@@ -52,7 +62,7 @@ __device__ __forceinline__ int node_count(float ratio) {
 }
 
 // e_r(k) for r >= 1, out of line: few tiles have sources that narrow.
-__device__ __noinline__ float narrow_spread_weight(float r, int k) {
+static __device__ __noinline__ float narrow_spread_weight(float r, int k) {
     const float c = float(k);
     return k == 0 ? erff(0.5f * r) : 0.5f * (erfcf((c - 0.5f) * r) - erfcf((c + 0.5f) * r));
 }

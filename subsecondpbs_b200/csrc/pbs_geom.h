@@ -34,7 +34,6 @@ constexpr int kTileY = 8;                // SUPERP_TILE_Y, include/core/Macro.cu
 constexpr int kTileSources = kTileX * kTileY;
 constexpr int kMaxR = 32;                // MAX_SUPERP_RADIUS, include/core/Macro.cuh:64
 constexpr int kSplitR = 15;              // radii <= kSplitR run in the medium and narrow superposition instances
-constexpr int kSplitR2 = 7;              // radii <= kSplitR2 run in the narrow instance
 constexpr int kMinTilesInBatch = 16;     // MIN_TILES_IN_BATCH, include/core/Macro.cuh:67
 constexpr float kBpDepthCutoff = 1.05f;  // BP_DEPTH_CUTOFF, include/core/Macro.cuh:46
 

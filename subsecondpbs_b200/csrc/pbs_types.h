@@ -63,17 +63,14 @@ struct BeamStateDev {
     float pxSpMultX, pxSpMultY;
     int maxCalcPassive;
     int workCount;          // superposition work items of the current layer chunk
-    // The radius-sorted work list holds the wide (R > kSplitR), medium
-    // (kSplitR2 < R <= kSplitR) and narrow (R <= kSplitR2) items in that order;
-    // each range has its own claim counter (relative to the range start).
+    // Claim counters of the superposition's three instances (radii above kSplitWide, above
+    // kSplitR, and the others), beyond the first item of each of their warps.
     int workNext;
-    int workSplit;          // items with R > kSplitR
     int workNextSmall;
-    int workSplit2;         // items with R > kSplitR2
     int workNextTiny;
     // The work list holds each radius R in one block, the wide radii first; block R
-    // starts at rStart[R] (layer_plan_kernel). The layer-merged list of the forward
-    // superposition (work_merge_kernel) keeps mergedR[R] items at the start of R's
+    // starts at rStart[R] (layer_plan_kernel). The layer-merged list
+    // (work_merge_kernel) keeps mergedR[R] items at the start of R's
     // block, so the items of one radius stay together.
     int rStart[kMaxR + 1];
     int mergedR[kMaxR + 1];

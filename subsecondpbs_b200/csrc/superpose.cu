@@ -33,8 +33,6 @@ namespace pbs {
 
 namespace {
 
-constexpr int kSplitWide = 23;  // widest radius of the second instance
-
 // Nodes whose rows a warp holds at a time; 8 nodes go in two halves.
 constexpr int kRowNodes = 6;
 __device__ __forceinline__ int batch_nodes(int count) { return count > kRowNodes ? count / 2 : count; }
@@ -43,11 +41,6 @@ __device__ __forceinline__ int batch_nodes(int count) { return count > kRowNodes
 // rows of pairs (source rows y and 7 - y of one node, as the two halves of packed FP32
 // operations). Rows and tables have odd strides (in 8 and 16 bytes), so that the lanes
 // of the row pass, one row each, read distinct banks.
-constexpr int kPairs = kTileY / 2;
-template <int R>
-constexpr int kRowStride = kTileX + 2 * R + 1;  // pairs
-template <int R>
-constexpr int kTableStride = ((R + 2) / 2 | 1) * 2;  // pairs
 template <int RMax>
 constexpr int kWarpPairs = kRowNodes * (kTableStride<RMax> + kPairs * kRowStride<RMax>);
 
@@ -558,11 +551,6 @@ cudaError_t launch_superpose(const BeamGeomDev& g, const float2* sources, const 
     e = launch_pdl(bev_fixed_to_float_kernel, dim3(numSMs * 8), dim3(256), 0, s, g,
                    static_cast<const BeamStateDev*>(beam), bevFixed, bev, shiftOffset);
     if (e != cudaSuccess) return e;
-    return cudaGetLastError();
-}
-
-cudaError_t launch_one_layer_list_view(BeamStateDev* beam, cudaStream_t s) {
-    one_layer_list_view_kernel<<<1, 64, 0, s>>>(beam);
     return cudaGetLastError();
 }
 
