@@ -65,6 +65,19 @@ int pbs_subsecond_wrapper(const float* ct_data, const int ct_dims[3], const floa
                                   dose_corner, beams, num_beams, energy, gpu_id, nuclear_correction, verbose);
 }
 
+int pbs_subsecond_wrapper_zeroed(const float* ct_data, const int ct_dims[3], const float ct_resolution[3],
+                                 const float ct_corner[3], float* dose_data, const int dose_dims[3],
+                                 const float dose_resolution[3], const float dose_corner[3], const PbsBeamDesc* beams,
+                                 size_t num_beams, const PbsEnergyDesc* energy, int gpu_id, int nuclear_correction,
+                                 int verbose, int* finite) {
+    if (!finite) {
+        pbs::set_error("null argument");
+        return PBS_ERR_INVALID_ARGUMENT;
+    }
+    return pbs::subsecond_wrapper(ct_data, ct_dims, ct_resolution, ct_corner, dose_data, dose_dims, dose_resolution,
+                                  dose_corner, beams, num_beams, energy, gpu_id, nuclear_correction, verbose, finite);
+}
+
 int pbs_wrapper_copy_bytes(unsigned long long out[2]) {
     if (!out) {
         pbs::set_error("null argument");

@@ -15,6 +15,8 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "context.h"
@@ -97,6 +99,9 @@ Context::~Context() {
     staging.release();
     errHost.release();
     if (copyStream) cudaStreamSynchronize(copyStream);
+    ring.release();
+    for (cudaEvent_t e : ringDone)
+        if (e) cudaEventDestroy(e);
     if (stagingEvent) cudaEventDestroy(stagingEvent);
     if (copyStart) cudaEventDestroy(copyStart);
     if (doseCopied) cudaEventDestroy(doseCopied);
@@ -313,6 +318,24 @@ cudaError_t copy_box(void* dst, const void* src, const int dims[3], const int lo
     return cudaMemcpy3DAsync(&p, s);
 }
 
+// Calls f(first, last) for parts of the rows [0, n) of a copy, by up to four threads.
+template <typename F>
+void split_rows(size_t n, size_t bytes, F f) {
+    constexpr size_t kParts = 4, kBytesPerPart = size_t(256) << 10;
+    const size_t cores = std::max(1u, std::thread::hardware_concurrency());
+    const size_t parts = std::max<size_t>(1, std::min({kParts, cores, n, bytes / kBytesPerPart}));
+    std::thread helpers[kParts - 1];
+    size_t started = 1;
+    try {
+        for (; started < parts; ++started)
+            helpers[started - 1] = std::thread(f, n * started / parts, n * (started + 1) / parts);
+    } catch (const std::system_error&) {  // no thread to be had: the parts left are done here
+    }
+    f(size_t(0), n / parts);
+    if (started < parts) f(n * started / parts, n);
+    for (size_t i = 1; i < started; ++i) helpers[i - 1].join();
+}
+
 bool box_empty(const int lo[3], const int hi[3]) { return hi[0] < lo[0] || hi[1] < lo[1] || hi[2] < lo[2]; }
 
 unsigned long long box_bytes(const int lo[3], const int hi[3]) {
@@ -370,6 +393,94 @@ void Context::column_layout(const BeamPlan& P, ColBox& fb, size_t& bevCells, siz
     bytesPerColumn = bevCells * (sizeof(float) + sizeof(unsigned long long)) + voxels * sizeof(double);
 }
 
+// The driver copies a box of pageable memory row by row through its own staging, on one
+// thread. Here the rows go through two page-locked slots, filled or emptied by a few
+// threads while the other slot's transfer runs, and a fresh buffer's page faults are
+// shared between them. One wrapper call on 256 x 256 x 160 voxels (5 MB of CT up, 11.6 MB
+// of dose down): 5.2 -> 3.3 ms, the initial dose's 11.6 MB up (left out for a dose of
+// zeros) included in the former. A water-equivalence volume, contiguous and copied while
+// earlier beams still run, is faster by the driver's copy (383 against 719 us).
+int Context::copy_host_box(float* dev, float* host, const int dims[3], const int lo[3], const int hi[3], bool toDevice,
+                           cudaStream_t s) {
+    constexpr size_t kSlot = size_t(4) << 20;  // bytes
+    constexpr unsigned long long kSmall = 1ull << 20;
+    auto direct = [&]() -> int {
+        if (toDevice)
+            PBS_CUDA(copy_box(dev, host, dims, lo, hi, cudaMemcpyHostToDevice, s), "box H2D");
+        else
+            PBS_CUDA(copy_box(host, dev, dims, lo, hi, cudaMemcpyDeviceToHost, s), "box D2H");
+        return PBS_OK;
+    };
+    const size_t w = size_t(hi[0] - lo[0] + 1), h = size_t(hi[1] - lo[1] + 1), d = size_t(hi[2] - lo[2] + 1);
+    cudaPointerAttributes at{};
+    const bool pageable = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    if (!pageable || box_bytes(lo, hi) < kSmall || w * 4 > kSlot) return direct();
+    if (ring.ensure(2 * kSlot)) {
+        cudaGetLastError();
+        set_error("");
+        return direct();
+    }
+    for (cudaEvent_t& e : ringDone)
+        if (!e) PBS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+    // A slot holds whole planes of the box, or rows of one plane.
+    const size_t rows = kSlot / (w * 4), planes = rows / h;
+    const size_t stepY = planes ? h : rows, stepZ = planes ? planes : 1;
+    const size_t partsY = (h + stepY - 1) / stepY, parts = partsY * ((d + stepZ - 1) / stepZ);
+    struct Part {
+        size_t y, z, h, d;
+        float* slot;
+    };
+    auto part = [&](size_t i) {
+        Part p;
+        p.y = i % partsY * stepY;
+        p.z = i / partsY * stepZ;
+        p.h = std::min(stepY, h - p.y);
+        p.d = std::min(stepZ, d - p.z);
+        p.slot = static_cast<float*>(ring.ptr) + (i & 1) * (kSlot / 4);
+        return p;
+    };
+    auto between_host = [&](const Part& p) {
+        split_rows(p.h * p.d, p.h * p.d * w * 4, [&, p](size_t first, size_t last) {
+            for (size_t r = first; r < last; ++r) {
+                const size_t z = size_t(lo[2]) + p.z + r / p.h, y = size_t(lo[1]) + p.y + r % p.h;
+                float* row = host + (z * dims[1] + y) * dims[0] + lo[0];
+                if (toDevice)
+                    std::memcpy(p.slot + r * w, row, w * 4);
+                else
+                    std::memcpy(row, p.slot + r * w, w * 4);
+            }
+        });
+    };
+    auto transfer = [&](size_t i, const Part& p) -> int {
+        cudaMemcpy3DParms m = {};
+        const cudaPitchedPtr slot = make_cudaPitchedPtr(p.slot, w * 4, w, p.h);
+        const cudaPitchedPtr vol = make_cudaPitchedPtr(dev, size_t(dims[0]) * 4, size_t(dims[0]), size_t(dims[1]));
+        const cudaPos pos = make_cudaPos(size_t(lo[0]) * 4, size_t(lo[1]) + p.y, size_t(lo[2]) + p.z);
+        m.srcPtr = toDevice ? slot : vol;
+        m.dstPtr = toDevice ? vol : slot;
+        (toDevice ? m.dstPos : m.srcPos) = pos;
+        m.extent = make_cudaExtent(w * 4, p.h, p.d);
+        m.kind = toDevice ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+        PBS_CUDA(cudaMemcpy3DAsync(&m, s), "box copy");
+        PBS_CUDA(cudaEventRecord(ringDone[i & 1], s), "cudaEventRecord");
+        return PBS_OK;
+    };
+    for (size_t i = 0; i < parts + (toDevice ? 0 : 1); ++i) {
+        if (i < parts) {
+            const Part p = part(i);
+            PBS_CUDA(cudaEventSynchronize(ringDone[i & 1]), "cudaEventSynchronize");
+            if (toDevice) between_host(p);
+            if (int rc = transfer(i, p)) return rc;
+        }
+        if (!toDevice && i > 0) {
+            PBS_CUDA(cudaEventSynchronize(ringDone[(i - 1) & 1]), "cudaEventSynchronize");
+            between_host(part(i - 1));
+        }
+    }
+    return PBS_OK;
+}
+
 int Context::set_ct_region(const float* data, const GridDesc& g, const int lo[3], const int hi[3]) {
     PBS_CUDA(cudaSetDevice(device), "cudaSetDevice");
     if (!data || g.dims[0] <= 0 || g.dims[1] <= 0 || g.dims[2] <= 0 ||
@@ -383,7 +494,8 @@ int Context::set_ct_region(const float* data, const GridDesc& g, const int lo[3]
     ctView = nullptr;
     ctQuadValid = false;
     if (!box_empty(lo, hi)) {
-        PBS_CUDA(copy_box(ct.ptr, data, g.dims, lo, hi, cudaMemcpyHostToDevice, stream), "CT H2D");
+        if ((rc = copy_host_box(static_cast<float*>(ct.ptr), const_cast<float*>(data), g.dims, lo, hi, true, stream)))
+            return rc;
         copiedH2D += box_bytes(lo, hi);
     }
     // The CT type comes from the whole volume, as with a full upload.
@@ -467,28 +579,43 @@ int Context::issue_dose_copy() {
     if (!deferredInit) return PBS_OK;
     PBS_CUDA(cudaEventRecord(copyStart, stream), "cudaEventRecord");
     PBS_CUDA(cudaStreamWaitEvent(copyStream, copyStart, 0), "cudaStreamWaitEvent");
-    PBS_CUDA(copy_box(floatOut.ptr, deferredInit, doseGrid.dims, deferredLo, deferredHi, cudaMemcpyHostToDevice,
-                      copyStream),
-             "dose H2D");
+    if (int rc = copy_host_box(static_cast<float*>(floatOut.ptr), const_cast<float*>(deferredInit), doseGrid.dims,
+                               deferredLo, deferredHi, true, copyStream))
+        return rc;
     copiedH2D += box_bytes(deferredLo, deferredHi);
     PBS_CUDA(cudaEventRecord(doseCopied, copyStream), "cudaEventRecord");
     deferredInit = nullptr;
     return PBS_OK;
 }
 
-int Context::read_dose_region(float* out, const int lo[3], const int hi[3]) {
+int Context::read_dose_region(float* out, const int lo[3], const int hi[3], int* finite) {
     PBS_CUDA(cudaSetDevice(device), "cudaSetDevice");
     const size_t n = size_t(doseGrid.dims[0]) * doseGrid.dims[1] * doseGrid.dims[2];
     int rc = flush_dose_init();
     if (rc) return rc;
     if ((rc = floatOut.ensure(n * 4))) return rc;
+    if (finite) *finite = 1;
     if (!box_empty(lo, hi)) {
         // Only the region is copied back, so only the region is converted.
+        int* bad = nullptr;
+        if (finite) {
+            if ((rc = stats.ensure(64))) return rc;
+            bad = static_cast<int*>(stats.ptr);
+            PBS_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), stream), "memset");
+        }
         PBS_CUDA(launch_dose_box(static_cast<double*>(dose64.ptr), static_cast<float*>(floatOut.ptr), doseGrid.dims,
-                                 lo, hi, stream),
+                                 lo, hi, stream, bad),
                  "dose_to_float");
-        PBS_CUDA(copy_box(out, floatOut.ptr, doseGrid.dims, lo, hi, cudaMemcpyDeviceToHost, stream), "dose D2H");
+        if ((rc = copy_host_box(static_cast<float*>(floatOut.ptr), out, doseGrid.dims, lo, hi, false, stream)))
+            return rc;
         copiedD2H += box_bytes(lo, hi);
+        if (finite) {
+            int flag = 0;
+            PBS_CUDA(cudaMemcpyAsync(&flag, bad, sizeof(int), cudaMemcpyDeviceToHost, stream), "finite D2H");
+            PBS_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+            copiedD2H += sizeof(int);
+            *finite = flag == 0;
+        }
     }
     PBS_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     return take_device_errors();
@@ -1873,13 +2000,13 @@ namespace {
 thread_local unsigned long long g_lastWrapperCopies[2] = {0, 0};
 int wrapper_body(Context* ctx, const float* ctData, const GridDesc& cg, float* doseData, const GridDesc& dg,
                  const PbsBeamDesc* beams, size_t numBeams, const PbsEnergyDesc* energyData, int nuclear,
-                 int verbose);
+                 int verbose, int* finite);
 }  // namespace
 
 int subsecond_wrapper(const float* ctData, const int ctDims[3], const float ctRes[3], const float ctCorner[3],
                       float* doseData, const int doseDims[3], const float doseRes[3], const float doseCorner[3],
                       const PbsBeamDesc* beams, size_t numBeams, const PbsEnergyDesc* energyData, int gpuId,
-                      int nuclear, int verbose) {
+                      int nuclear, int verbose, int* finite) {
     GridDesc cg, dg;
     for (int i = 0; i < 3; ++i) {
         cg.dims[i] = ctDims ? ctDims[i] : 0;
@@ -1912,7 +2039,7 @@ int subsecond_wrapper(const float* ctData, const int ctDims[3], const float ctRe
         ctx = c;
     }
     ctx->copiedH2D = ctx->copiedD2H = 0;
-    int rc = wrapper_body(ctx, ctData, cg, doseData, dg, beams, numBeams, energyData, nuclear, verbose);
+    int rc = wrapper_body(ctx, ctData, cg, doseData, dg, beams, numBeams, energyData, nuclear, verbose, finite);
     g_lastWrapperCopies[0] = ctx->copiedH2D;
     g_lastWrapperCopies[1] = ctx->copiedD2H;
     return rc;
@@ -1928,7 +2055,7 @@ namespace {
 
 int wrapper_body(Context* ctx, const float* ctData, const GridDesc& cg, float* doseData, const GridDesc& dg,
                  const PbsBeamDesc* beams, size_t numBeams, const PbsEnergyDesc* energyData, int nuclear,
-                 int verbose) {
+                 int verbose, int* finite) {
     int rc;
     if ((rc = ctx->set_energy(*energyData))) return rc;
     // Every beam is planned up front, and the plan is handed to add_planned_beam: the CT
@@ -1961,7 +2088,8 @@ int wrapper_body(Context* ctx, const float* ctData, const GridDesc& cg, float* d
     }
     if ((rc = ctx->set_ct_region(ctData, cg, ctLo, ctHi))) return rc;
     if ((rc = ctx->set_dose_grid(dg))) return rc;
-    if ((rc = ctx->reset_dose_region(doseData, dLo, dHi))) return rc;
+    // (set_dose_grid has zeroed the dose.)
+    if (!finite && (rc = ctx->reset_dose_region(doseData, dLo, dHi))) return rc;
     for (size_t i = 0; i < numBeams; ++i) {
         // The plan made above used the same tables and grids as the context now holds.
         if ((rc = ctx->add_planned_beam(beams[i], nuclear, std::move(plans[i])))) return rc;
@@ -1974,7 +2102,7 @@ int wrapper_body(Context* ctx, const float* ctData, const GridDesc& cg, float* d
                              st.guaranteed_passive, st.live_tiles);
         }
     }
-    return ctx->read_dose_region(doseData, dLo, dHi);
+    return ctx->read_dose_region(doseData, dLo, dHi, finite);
 }
 
 }  // namespace

@@ -181,6 +181,9 @@ struct Context {
     bool colClean = false;
 
     PinnedBuf staging, errHost;
+    // Ring of two page-locked slots for copies of pageable host volumes (copy_host_box).
+    PinnedBuf ring;
+    cudaEvent_t ringDone[2] = {};
     cudaEvent_t stagingEvent = nullptr;
     cudaEvent_t ev[8] = {};
 
@@ -220,7 +223,13 @@ struct Context {
     // Packed CT entries of the uploaded box only (set_ct_region).
     int build_ct_quad_box(const int lo[3], const int hi[3]);
     int reset_dose_region(const float* init, const int lo[3], const int hi[3]);
-    int read_dose_region(float* out, const int lo[3], const int hi[3]);
+    // `finite` (may be null): whether every value read is finite.
+    int read_dose_region(float* out, const int lo[3], const int hi[3], int* finite = nullptr);
+    // Copies the box [lo, hi] between [Z][Y][X] float volumes of `dims` in device and
+    // host memory. Returns with the host side read or written (page-locked: in stream
+    // order, as cudaMemcpyAsync).
+    int copy_host_box(float* dev, float* host, const int dims[3], const int lo[3], const int hi[3], bool toDevice,
+                      cudaStream_t s);
     int convert_ct(int type, const GridDesc& g);
     // HU+1000 conversion of `n` device floats in place, on the context stream.
     // With dims, only the inclusive box [lo, hi] of the [dims.z][dims.y][dims.x] CT.
@@ -327,9 +336,10 @@ int operator_batch_plan(const PbsBeamDesc& beam, int maxSpotsPerBatch, OperatorP
 // Host->device and device->host bytes of the calling thread's last completed
 // subsecond_wrapper call.
 int wrapper_copy_bytes(unsigned long long out[2]);
+// With `finite`, doseData holds zeros on entry, and *finite is whether the dose is finite.
 int subsecond_wrapper(const float* ctData, const int ctDims[3], const float ctRes[3], const float ctCorner[3],
                       float* doseData, const int doseDims[3], const float doseRes[3], const float doseCorner[3],
                       const PbsBeamDesc* beams, size_t numBeams, const PbsEnergyDesc* energyData, int gpuId,
-                      int nuclear, int verbose);
+                      int nuclear, int verbose, int* finite = nullptr);
 
 }  // namespace pbs

@@ -160,7 +160,7 @@ cudaError_t launch_dose_to_float(const double* dose, float* out, size_t n, cudaS
 cudaError_t launch_dose_box_init(double* dose, const float* init, const int dims[3], const int lo[3], const int hi[3],
                                  cudaStream_t s);
 cudaError_t launch_dose_box(double* dose, float* out, const int dims[3], const int lo[3], const int hi[3],
-                            cudaStream_t s);
+                            cudaStream_t s, int* nonFinite = nullptr);
 
 // Biological maps (bio.cu).
 cudaError_t launch_bio_channel(const BeamGeomDev& g, const BioDev& m, int layer0, int nLayers, const float2* sources,

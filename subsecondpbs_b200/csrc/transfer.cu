@@ -210,14 +210,18 @@ __global__ void dose_to_float_kernel(const double* dose, float* out, size_t n) {
 }
 
 // Box [lo, lo + ext) of a [dims.z][dims.y][dims.x] grid: zeroes the FP64 dose there
-// (out == nullptr) or converts it to float into the same voxels of `out`.
-__global__ void dose_box_kernel(double* dose, float* out, int3 dims, int3 lo, int3 ext) {
+// (out == nullptr) or converts it to float into the same voxels of `out` and
+// sets *nonFinite (if given) where a value is not finite.
+__global__ void dose_box_kernel(double* dose, float* out, int3 dims, int3 lo, int3 ext, int* nonFinite) {
     walk_rows(ext.x, ext.y, ext.z, [&](int x, int y, int z) {
         const size_t v = (size_t(z + lo.z) * dims.y + (y + lo.y)) * size_t(dims.x) + (x + lo.x);
-        if (out)
-            out[v] = float(dose[v]);
-        else
+        if (out) {
+            const float f = float(dose[v]);
+            out[v] = f;
+            if (nonFinite && !isfinite(f)) *nonFinite = 1;
+        } else {
             dose[v] = 0.0;
+        }
     });
 }
 
@@ -407,7 +411,7 @@ cudaError_t launch_dose_to_float(const double* dose, float* out, size_t n, cudaS
 }
 
 cudaError_t launch_dose_box(double* dose, float* out, const int dims[3], const int lo[3], const int hi[3],
-                            cudaStream_t s) {
+                            cudaStream_t s, int* nonFinite) {
     for (int i = 0; i < 3; ++i)
         if (lo[i] < 0 || hi[i] >= dims[i] || hi[i] < lo[i]) return cudaErrorInvalidValue;
     const int3 d = make_int3(dims[0], dims[1], dims[2]);
@@ -415,7 +419,7 @@ cudaError_t launch_dose_box(double* dose, float* out, const int dims[3], const i
     const int3 e = make_int3(hi[0] - lo[0] + 1, hi[1] - lo[1] + 1, hi[2] - lo[2] + 1);
     const size_t total = size_t(e.x) * e.y * e.z;
     const int blocks = int(std::min<size_t>((total + 255) / 256, 148 * 32));
-    dose_box_kernel<<<blocks, 256, 0, s>>>(dose, out, d, l, e);
+    dose_box_kernel<<<blocks, 256, 0, s>>>(dose, out, d, l, e, nonFinite);
     return cudaGetLastError();
 }
 

@@ -73,14 +73,17 @@ def raytracedicom_wrapper(ct, ct_dims, ct_resolution, ct_corner, dose_dims, dose
     dose = np.zeros((int(dose_dims[2]), int(dose_dims[1]), int(dose_dims[0])), dtype=np.float32)
     bd, keep_b = _lib.beam_desc(beam)
     ed, keep_e = _lib.energy_desc(energy)
-    rc = lib.pbs_subsecond_wrapper(
+    # The dose is zero outside the voxels that the beam can reach, and those are looked at
+    # where they are read out.
+    finite = C.c_int(1)
+    rc = lib.pbs_subsecond_wrapper_zeroed(
         ct_arr.ctypes.data_as(C.POINTER(C.c_float)), _lib.int3(ct_dims), _lib.float3(ct_resolution),
         _lib.float3(ct_corner), dose.ctypes.data_as(C.POINTER(C.c_float)), _lib.int3(dose_dims),
         _lib.float3(dose_resolution), _lib.float3(dose_corner), C.byref(bd), 1, C.byref(ed), int(gpu_id),
-        int(bool(nuclear_correction)), int(verbose))
+        int(bool(nuclear_correction)), int(verbose), C.byref(finite))
     del keep_b, keep_e
     _lib.check(rc)
-    if not np.all(np.isfinite(dose)):
+    if not finite.value:
         raise RuntimeError("raytracedicom_wrapper produced non-finite dose values")
     return dose
 
