@@ -270,5 +270,18 @@ PBS_HD V3 transfer_fan_idx(const TransferParams& p, V3 start, int k) {
     r.y = fmul(r.y, fadd(1.0f, fdiv(r.z, fsub(p.normDist.y, r.z))));
     return add(r, p.globalOffset);
 }
+// The same in two parts: the divergence factors at k, and the index from them. Where
+// inc.z is 0 the factors are those of the whole column.
+PBS_HD void transfer_divergence(const TransferParams& p, V3 start, int k, float& fx, float& fy) {
+    const float z = fadd(start.z, fmul(float(k), p.inc.z));
+    fx = fadd(1.0f, fdiv(z, fsub(p.normDist.x, z)));
+    fy = fadd(1.0f, fdiv(z, fsub(p.normDist.y, z)));
+}
+PBS_HD V3 transfer_fan_idx(const TransferParams& p, V3 start, int k, float fx, float fy) {
+    V3 r = add(start, hadamard(v3s(float(k)), p.inc));
+    r.x = fmul(r.x, fx);
+    r.y = fmul(r.y, fy);
+    return add(r, p.globalOffset);
+}
 
 }  // namespace pbs

@@ -148,25 +148,51 @@ __global__ void column_transfer_planner_kernel(BeamGeomDev g, BeamStateDev* beam
     }
 }
 
-// A column's BEV samples at kTransferZChunk consecutive z from z0 on (0 past `mz` and
-// outside the fan): independent loads, so that their latencies overlap.
 constexpr int kTransferZChunk = 4;
 constexpr int kTransferBlocksPerSM = 8;
 
-__device__ __forceinline__ void sample_chunk(const BeamGeomDev& g, const float* __restrict__ bev,
+// BEV cells [lo, hi] outside of which a volume is zero. `reaches`: whether the sample at
+// BEV index (x, y, z) reads a cell of the box.
+struct BevBox {
+    float lo[3], hi[3];
+    __device__ __forceinline__ BevBox(const int l[3], const int h[3]) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            lo[i] = float(l[i] - 1);
+            hi[i] = float(h[i] + 1);
+        }
+    }
+    __device__ __forceinline__ bool reaches(float x, float y, float z) const {
+        return x >= lo[0] && x <= hi[0] && y >= lo[1] && y <= hi[1] && z >= lo[2] && z <= hi[2];
+    }
+};
+
+// A column's BEV samples at kTransferZChunk consecutive z from z0 on (0 past `mz` and
+// outside the fan): independent loads, so that their latencies overlap. A chunk that only
+// reads zero cells is left out as a whole (a test for each voxel would come between the
+// loads), and the divergence's divisions are done once where the beam runs across z.
+// 512 x 512 x 200 voxels, gantry 240: 237 -> 181 us with both, 227 with the latter alone;
+// 20,000 spots along x 187 -> 177. With 2 or 8 voxels in a chunk 206 and 248.
+__device__ __forceinline__ void sample_chunk(const BeamGeomDev& g, const float* __restrict__ bev, const BevBox& box,
                                              const TransferParams& T, float zShift, int x, int y, int z0, int mz,
                                              float (&v)[kTransferZChunk]) {
     const V3 start = transfer_start(T, x, y);
+    float fx, fy;
+    transfer_divergence(T, start, z0, fx, fy);
+    V3 f[kTransferZChunk];
+    bool any = false;
 #pragma unroll
     for (int k = 0; k < kTransferZChunk; ++k) {
-        const int z = z0 + k;
+        if (k > 0 && T.inc.z != 0.0f) transfer_divergence(T, start, z0 + k, fx, fy);
+        f[k] = transfer_fan_idx(T, start, z0 + k, fx, fy);
+        any = any || box.reaches(f[k].x, f[k].y, f[k].z - zShift);
         v[k] = 0.0f;
-        if (z <= mz) {
-            const V3 f = transfer_fan_idx(T, start, z);
-            if (!(f.x + 0.5f < 0.0f || f.y + 0.5f < 0.0f || f.z + 0.5f < 0.0f))
-                v[k] = bev_sample(bev, g.bevX, g.bevY, g.steps, f.x, f.y, f.z - zShift);
-        }
     }
+    if (!any) return;
+#pragma unroll
+    for (int k = 0; k < kTransferZChunk; ++k)
+        if (z0 + k <= mz && !(f[k].x + 0.5f < 0.0f || f[k].y + 0.5f < 0.0f || f[k].z + 0.5f < 0.0f))
+            v[k] = bev_sample(bev, g.bevX, g.bevY, g.steps, f[k].x, f[k].y, f[k].z - zShift);
 }
 
 // primTransfDiv (src/algorithms/prim_transf_kernel.cu:11-44). The reference launches
@@ -188,10 +214,11 @@ transfer_kernel(BeamGeomDev g, const float* __restrict__ bev, const BeamStateDev
     const TransferParams T = beam->transfer;
     const float zShift = g.compatBevZShift ? float(beam->firstInside) : 0.0f;
     const size_t slice = static_cast<size_t>(g.doseX) * g.doseY;
+    const BevBox box(beam->liveLo, beam->liveHi);
     walk_box(T, sx, sy, nx, ny, nzc, [&](int x, int y, int chunk) {
         const int z0 = sz + chunk * kTransferZChunk;
         float v[kTransferZChunk];
-        sample_chunk(g, bev, T, zShift, x, y, z0, mz, v);
+        sample_chunk(g, bev, box, T, zShift, x, y, z0, mz, v);
         double* col = dose + static_cast<size_t>(y) * g.doseX + x;
 #pragma unroll
         for (int k = 0; k < kTransferZChunk; ++k)
@@ -243,10 +270,11 @@ column_transfer_kernel(BeamGeomDev g, const float* __restrict__ bev, size_t bevS
     const size_t fbN = static_cast<size_t>(fb.ext[0]) * fb.ext[1] * fb.ext[2];
     double* out = colDose + static_cast<size_t>(q) * fbN;
     const size_t slice = static_cast<size_t>(fb.ext[0]) * fb.ext[1];
+    const BevBox box(ls[q].liveLo, ls[q].liveHi);
     walk_box(T, lo[0], lo[1], nx, ny, nzc, [&](int x, int y, int chunk) {
         const int z0 = lo[2] + chunk * kTransferZChunk;
         float v[kTransferZChunk];
-        sample_chunk(g, v0, T, 0.0f, x, y, z0, hi[2], v);
+        sample_chunk(g, v0, box, T, 0.0f, x, y, z0, hi[2], v);
         double* col = out + static_cast<size_t>(y - fb.lo[1]) * fb.ext[0] + (x - fb.lo[0]);
 #pragma unroll
         for (int k = 0; k < kTransferZChunk; ++k)
