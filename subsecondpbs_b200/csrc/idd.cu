@@ -406,105 +406,134 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
     }
 }
 
-// One thread per layer of the chunk: passive step (wrapper.cu:4975-4990), histogram
-// over [first, calcPassive) (tiles at steps >= calcPassive hold only dead rays and
-// fall in bucket 0), overflow merge into R=32 (complete_superposition.cu:412-460)
-// and batching of sparse buckets into the radius above them
-// (complete_superposition.cu:476-483). Thread 0 then lays out the chunk's work list
-// in descending radius.
+// Per layer of the chunk: passive step (wrapper.cu:4975-4990), histogram over [first,
+// calcPassive) (tiles at steps >= calcPassive hold only dead rays and fall in bucket 0),
+// overflow merge into R=32 (complete_superposition.cu:412-460) and batching of sparse
+// buckets into the radius above them (complete_superposition.cu:476-483). Then the chunk's
+// work list is laid out in descending radius.
 //
 // With `primaryLs` set the kernel plans the nuclear halo of the chunk instead
 // (performNuclearTileBasedSuperposition, complete_superposition.cu:558-708): the
 // halo histogram already covers [first, calcPassive) of the primary layer, and a
 // radius above 32 is an error (the reference throws) rather than a merge.
-__global__ void __launch_bounds__(kMaxChunkLayers)
+//
+// One block, latency bound. A warp reads and writes a layer's tables, lane = bucket, and a
+// thread per layer batches them in shared memory; with a thread per layer throughout, each
+// access to the tables was one sector per thread: 11.6 us in place of 9.6 (40 layers).
+constexpr int kPlanThreads = 1024;
+
+__global__ void __launch_bounds__(kPlanThreads)
 layer_plan_kernel(BeamGeomDev g, int layer0, int nLayers, LayerStateDev* __restrict__ ls,
                   BeamStateDev* __restrict__ beam, int workCapacity, const LayerStateDev* __restrict__ primaryLs,
                   const BeamStateDev* __restrict__ primaryBeam) {
-    __shared__ int sLive[kMaxChunkLayers][kMaxR + 1];   // live items per layer and batched radius
-    __shared__ int sCalc[kMaxChunkLayers];
-    __shared__ int sWarpSum[kMaxChunkLayers / 32];
-    __shared__ long long sWarpFma[kMaxChunkLayers / 32];
+    constexpr int kStride = kBuckets + 1 - kBuckets % 2;  // odd
+    __shared__ int sHist[kMaxChunkLayers][kStride];  // tiles per bucket; the list's offsets in the end
+    __shared__ int sMap[kMaxChunkLayers][kStride];   // live tiles per bucket, then its batched radius
+    __shared__ int sBatched[kMaxChunkLayers][kMaxR + 1];
+    __shared__ int sLive[kMaxChunkLayers][kMaxR + 1];  // live items per batched radius
+    __shared__ int sWarpSum[kPlanThreads / 32];
+    __shared__ unsigned long long sFma;
+    __shared__ unsigned sMaxIdd;
+    __shared__ int sMaxCalc;
     pdl_trigger();
-    const int lc = threadIdx.x;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const bool nuclear = primaryLs != nullptr;
     const int first = nuclear ? primaryBeam->firstInside : beam->firstInside;
     const int tiles = g.tilesX * g.tilesY;
-    if (lc < nLayers) {
-        LayerStateDev& st = ls[layer0 + lc];
-        // Every input of the layer is read before its outputs are written: the outputs
-        // go to the same struct through indexed stores, so a load placed after them
-        // would wait for them to complete.
-        int hist[kBuckets], liveHist[kBuckets];
-        for (int i = 0; i < kBuckets; ++i) {
-            hist[i] = st.histAll[i];
-            liveHist[i] = st.liveHist[i];
+    int calc = 0, afterLast = 0;
+    unsigned maxIdd = 0;
+    if (t < nLayers) {
+        const LayerStateDev& st = ls[layer0 + t];
+        afterLast = st.afterLast;
+        calc = nuclear ? primaryLs[layer0 + t].calcPassive : st.maxFirstPassive;
+        maxIdd = st.maxIddBits;
+    }
+    if (t == 0) {
+        sFma = 0;
+        sMaxIdd = 0;
+        sMaxCalc = INT_MIN;
+    }
+    for (int q = warp; q < nLayers; q += kPlanThreads / 32)
+        for (int i = lane; i < kBuckets; i += 32) {
+            sHist[q][i] = ls[layer0 + q].histAll[i];
+            sMap[q][i] = ls[layer0 + q].liveHist[i];
+            if (i <= kMaxR) {
+                sBatched[q][i] = 0;
+                sLive[q][i] = 0;
+            }
         }
-        const int afterLast = st.afterLast;
-        const int maxFirstPassive = st.maxFirstPassive;
-        int calc;
+    __syncthreads();
+    if (t < nLayers) {
+        LayerStateDev& st = ls[layer0 + t];
+        int* hist = sHist[t];
+        int* map = sMap[t];
         if (nuclear) {
-            calc = primaryLs[layer0 + lc].calcPassive;
             st.afterLast = calc;
-            st.calcPassive = calc;
             if (hist[kMaxR + 1] > 0) atomicOr(&beam->errorFlags, 4);
         } else {
-            calc = maxFirstPassive;
             if (calc < first + 1) calc = first + 1;
             if (calc < 0) calc = first + 1;
             if (calc > afterLast) calc = afterLast;
             if (calc > g.steps) calc = g.steps;
-            st.calcPassive = calc;
             if (afterLast > calc && afterLast > first) hist[0] -= (afterLast - max(calc, first)) * tiles;
         }
-        for (int i = 0; i < kBuckets; ++i) st.hist[i] = hist[i];
-        if (hist[kMaxR + 1] > 0) {
-            hist[kMaxR] += hist[kMaxR + 1];
-            hist[kMaxR + 1] = 0;
+        st.calcPassive = calc;
+        atomicMax(&sMaxCalc, calc);
+        if (maxIdd) atomicMax(&sMaxIdd, maxIdd);
+        // Batches from the widest radius down: a batch, named by its widest radius `top`,
+        // takes radii until it holds kMinTilesInBatch tiles. The overflow bucket counts as
+        // the widest radius.
+        int live = 0, top = 0, held = 0, heldLive = 0;
+        bool met = false;
+#pragma unroll 4
+        for (int rad = kMaxR; rad > 0; --rad) {
+            const int h = hist[rad] + (rad == kMaxR ? hist[kMaxR + 1] : 0);
+            const int l = map[rad] + (rad == kMaxR ? map[kMaxR + 1] : 0);
+            live += l;
+            if (!met && h > 0) {
+                met = true;
+                top = rad;
+            }
+            map[rad] = met ? top : rad;
+            if (rad == kMaxR) map[kMaxR + 1] = map[rad];
+            held += h;
+            heldLive += l;
+            if (met) {
+                sBatched[t][top] = held;
+                sLive[t][top] = heldLive;
+                if (held >= kMinTilesInBatch) {
+                    top = rad - 1;
+                    held = 0;
+                    heldLive = 0;
+                }
+            }
         }
-        int layerMax = 0;
-        for (int i = 0; i < kBuckets; ++i)
-            if (hist[i] > 0) layerMax = i;
-        int batched[kMaxR + 1];
-        int map[kBuckets];
-        for (int i = 0; i <= kMaxR; ++i) batched[i] = 0;
-        for (int i = 0; i < kBuckets; ++i) map[i] = i;
-        batched[0] = hist[0];
+        live += map[0];
+        sBatched[t][0] = hist[0];
+        sLive[t][0] = map[0];
         map[0] = 0;
-        int recRad = layerMax;
-        for (int rad = layerMax; rad > 0; --rad) {
-            map[rad] = recRad;
-            batched[recRad] += hist[rad];
-            if (batched[recRad] >= kMinTilesInBatch) recRad = rad - 1;
-        }
-        map[kMaxR + 1] = map[kMaxR];
-        int live = 0;
-        for (int i = 0; i <= kMaxR; ++i) {
-            st.batchedCounts[i] = batched[i];
-            st.curR[i] = 0;
-        }
-        int liveR[kMaxR + 1];
-        for (int i = 0; i <= kMaxR; ++i) liveR[i] = 0;
-        for (int b = 0; b < kBuckets; ++b) {
-            st.batchedR[b] = map[b];
-            liveR[map[b]] += liveHist[b];
-            live += liveHist[b];
-        }
-        for (int i = 0; i <= kMaxR; ++i) {
-            st.liveR[i] = liveR[i];
-            sLive[lc][i] = liveR[i];
-        }
         st.liveTiles = live;
-        sCalc[lc] = calc;
     }
     __syncthreads();
+    for (int q = warp; q < nLayers; q += kPlanThreads / 32) {
+        LayerStateDev& st = ls[layer0 + q];
+        for (int i = lane; i < kBuckets; i += 32) {
+            st.hist[i] = sHist[q][i];
+            st.batchedR[i] = sMap[q][i];
+            if (i <= kMaxR) {
+                st.batchedCounts[i] = sBatched[q][i];
+                st.liveR[i] = sLive[q][i];
+                st.curR[i] = 0;
+            }
+        }
+    }
 
     // Work-list offsets: radius groups in descending radius, each with its layers in
     // order, i.e. position p = (kMaxR - r) * nLayers + q. Each thread sums a run of
-    // positions, the block scans the runs, then each thread writes its offsets.
+    // positions, the block scans the runs, then each thread sets its offsets.
     const int total = (kMaxR + 1) * nLayers;
-    const int per = (total + kMaxChunkLayers - 1) / kMaxChunkLayers;
-    const int p0 = min(lc * per, total), p1 = min(p0 + per, total);
+    const int per = (total + kPlanThreads - 1) / kPlanThreads;
+    const int p0 = min(t * per, total), p1 = min(p0 + per, total);
     int runSum = 0;
     long long runFma = 0;
     for (int p = p0; p < p1; ++p) {
@@ -513,64 +542,56 @@ layer_plan_kernel(BeamGeomDev g, int layer0, int nLayers, LayerStateDev* __restr
         runSum += v;
         runFma += static_cast<long long>(v) * 256 * (2 * r + 1) * (2 * r + 1);
     }
-    const int lane = lc & 31, warp = lc >> 5;
     int incl = runSum;
     for (int o = 1; o < 32; o <<= 1) {
         const int n = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += n;
     }
-    long long wf = runFma;
-    for (int o = 16; o > 0; o >>= 1) wf += __shfl_xor_sync(0xffffffffu, wf, o);
+    for (int o = 16; o > 0; o >>= 1) runFma += __shfl_xor_sync(0xffffffffu, runFma, o);
     if (lane == 31) sWarpSum[warp] = incl;
-    if (lane == 0) sWarpFma[warp] = wf;
+    if (lane == 0 && runFma) atomicAdd(&sFma, static_cast<unsigned long long>(runFma));
     __syncthreads();
-    int acc = incl - runSum;
-    for (int w = 0; w < warp; ++w) acc += sWarpSum[w];
+    // Items before this warp's positions, and in all.
+    const int sum = sWarpSum[lane];
+    int acc = __reduce_add_sync(0xffffffffu, lane < warp ? sum : 0) + incl - runSum;
+    int items = __reduce_add_sync(0xffffffffu, sum);
     for (int p = p0; p < p1; ++p) {
         const int r = kMaxR - p / nLayers, q = p % nLayers;
-        ls[layer0 + q].offR[r] = acc;
+        sHist[q][r] = acc;
         if (q == 0) beam->rStart[r] = acc;
         acc += sLive[q][r];
     }
-    __syncthreads();
-    if (lc == 0) {
+    if (t <= kMaxR) beam->mergedR[t] = 0;
+    if (t == 0) {
         if (nuclear) {
             // The halo transfer spans the same steps as the primary one.
             beam->firstInside = first;
             beam->maxCalcPassive = primaryBeam->maxCalcPassive;
         }
-        acc = 0;
-        long long fma = 0;
-        for (int w = 0; w < kMaxChunkLayers / 32; ++w) {
-            acc += sWarpSum[w];
-            fma += sWarpFma[w];
-        }
-        int mp = beam->maxCalcPassive;
-        for (int q = 0; q < nLayers; ++q) mp = max(mp, sCalc[q]);
-        beam->maxCalcPassive = mp;
-        if (acc > workCapacity) {
+        beam->maxCalcPassive = max(beam->maxCalcPassive, sMaxCalc);
+        if (items > workCapacity) {
             atomicOr(&beam->errorFlags, 1);
-            acc = workCapacity;
+            items = workCapacity;
         }
-        beam->workCount = acc;
+        beam->workCount = items;
         beam->workNext = 0;
         beam->workNextSmall = 0;
         beam->workNextTiny = 0;
-        for (int r = 0; r <= kMaxR; ++r) beam->mergedR[r] = 0;
-        // Fixed-point range of the chunk's BEV: a cell sums at most `acc` tile
+        // Fixed-point range of the chunk's BEV: a cell sums at most `items` tile
         // footprints (merged items sum several of them), each at most 256 x the
         // largest IDD of the chunk, so with that IDD below 2^ex every cell stays below
-        // 2^(ex + 8 + ceil(log2 acc)); the shift puts that bound at 2^61.
-        unsigned mb = 0;
-        for (int q = 0; q < nLayers; ++q) mb = max(mb, ls[layer0 + q].maxIddBits);
+        // 2^(ex + 8 + ceil(log2 items)); the shift puts that bound at 2^61.
         int ex = 0;
-        frexpf(__uint_as_float(mb), &ex);
+        frexpf(__uint_as_float(sMaxIdd), &ex);
         int lg = 0;
-        while ((1LL << lg) < static_cast<long long>(max(acc, 1))) ++lg;
-        beam->fixedShift = mb ? min(61 - ex - 8 - lg, 120) : 0;
-        beam->liveTiles += acc;
-        beam->superposeFma += fma;
+        while ((1LL << lg) < static_cast<long long>(max(items, 1))) ++lg;
+        beam->fixedShift = sMaxIdd ? min(61 - ex - 8 - lg, 120) : 0;
+        beam->liveTiles += items;
+        beam->superposeFma += static_cast<long long>(sFma);
     }
+    __syncthreads();
+    for (int q = warp; q < nLayers; q += kPlanThreads / 32)
+        for (int i = lane; i <= kMaxR; i += 32) ls[layer0 + q].offR[i] = sHist[q][i];
 }
 
 // One thread per (layer, step, tile) code of the chunk: live tiles are written to
@@ -807,7 +828,7 @@ cudaError_t launch_bin_plan(const BeamGeomDev& g, int layer0, int nLayers, const
                             BeamStateDev* beam, int4* work, int workCapacity, bool merged,
                             const LayerStateDev* primaryLs, const BeamStateDev* primaryBeam, cudaStream_t s) {
     if (nLayers > kMaxChunkLayers) return cudaErrorInvalidValue;
-    layer_plan_kernel<<<1, kMaxChunkLayers, 0, s>>>(g, layer0, nLayers, ls, beam, workCapacity, primaryLs,
+    layer_plan_kernel<<<1, kPlanThreads, 0, s>>>(g, layer0, nLayers, ls, beam, workCapacity, primaryLs,
                                                     primaryBeam);
     if (merged) {
         const size_t warps = static_cast<size_t>(g.steps) * g.tilesX * g.tilesY;
