@@ -205,15 +205,26 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
     float incDiv = p.sigmaSqAirLin + (2.0f * float(first) - 1.0f) * quad;
     float sigmaSq = -incDiv;
 
-    // The next step's WEPL and material are loaded one step ahead.
+    // WEPL and material are loaded two steps ahead: where few tiles leave the SMs to one
+    // CTA each, a step waits for its loads (3 layers of 96 x 72 rays, 235 steps: 96 us with
+    // one step, 78 with two, three and four; full chips are as fast with one). One ahead
+    // with the halo, whose registers would cost a CTA per SM (400 against 408 us).
+    constexpr int kIddAhead = kNuclear ? 1 : 2;
     const float* nextW = wepl + static_cast<size_t>(first) * rayPlane + ridx;
     const float2* nextM = material + static_cast<size_t>(first) * rayPlane + ridx;
-    float nextSp = 0.0f;
-    float2 nextMat = make_float2(0.0f, 0.0f);
-    if (live && first < afterLastL) {
-        nextSp = *nextW;
-        nextMat = *nextM;
+    float aheadSp[kIddAhead];
+    float2 aheadMat[kIddAhead];
+#pragma unroll
+    for (int i = 0; i < kIddAhead; ++i) {
+        aheadSp[i] = 0.0f;
+        aheadMat[i] = make_float2(0.0f, 0.0f);
+        if (live && first + i < afterLastL) {
+            aheadSp[i] = nextW[static_cast<size_t>(i) * rayPlane];
+            aheadMat[i] = nextM[static_cast<size_t>(i) * rayPlane];
+        }
     }
+    nextW += static_cast<size_t>(kIddAhead - 1) * rayPlane;
+    nextM += static_cast<size_t>(kIddAhead - 1) * rayPlane;
     float2* dst = srcL;
     float runMax = 0.0f;  // largest IDD of this ray (fixed-point range of the superposition)
     int stepNo = first;
@@ -230,13 +241,18 @@ idd_kernel(BeamGeomDev g, LutsDev luts, int layer0, const float2* __restrict__ m
         // value of every step, live or not).
         const float nextProfileSp = kProfile && real ? wepl[static_cast<size_t>(stepNo) * rayPlane + ridx] : 0.0f;
         if (live) {
-            const float cumulSp = nextSp;
-            const float dens = nextMat.x, rRl = nextMat.y;
-            if (stepNo + 1 < afterLastL) {
+            const float cumulSp = aheadSp[0];
+            const float dens = aheadMat[0].x, rRl = aheadMat[0].y;
+#pragma unroll
+            for (int i = 0; i + 1 < kIddAhead; ++i) {
+                aheadSp[i] = aheadSp[i + 1];
+                aheadMat[i] = aheadMat[i + 1];
+            }
+            if (stepNo + kIddAhead < afterLastL) {
                 nextW += rayPlane;
                 nextM += rayPlane;
-                nextSp = *nextW;
-                nextMat = *nextM;
+                aheadSp[kIddAhead - 1] = *nextW;
+                aheadMat[kIddAhead - 1] = *nextM;
             }
             const float cumulDose = lut_linear_clamp_padded(ciddRow, luts.nS, cumulSp * p.energyScaleFact + 0.5f);
             if (cumulSp < p.peakDepth) {
