@@ -263,10 +263,11 @@ trace_kernel(BeamGeomDev g, LutsDev luts, const float* __restrict__ ct, const fl
     }
 
     // Entry step. No step of this segment has it while the running sum stays below the
-    // threshold with room for its rounding (a NaN among the samples takes the long way);
-    // the first step has it where the sum is there already.
+    // threshold with room for its rounding; the first step has it where the sum is there
+    // already. A NaN among the samples, which the largest sum drops but the segment's sum
+    // keeps, takes the long way: a sum that is not below the threshold is an entry.
     int firstK = kNone;
-    if (active && s0 < s1 && !(huPre + huTop < 149.0f)) {
+    if (active && s0 < s1 && !(huPre + huTop < 149.0f && huSum == huSum)) {
         if (!(huPre + huFirst < 150.0f)) {
             firstK = s0;
         } else {
