@@ -14,8 +14,9 @@
 // done once per item whatever its layers.
 //
 // Error: the largest deviation of the interpolant over all (dy, dx), relative to the
-// footprint's peak e_r(0)^2, depends on hi/lo only (for r R of any size); node_count
-// takes the fewest nodes that keep it below 2.5e-7. The erf differences of one source
+// source's own peak e_r(0)^2, is bounded by hi/lo alone, whatever r and R; node_count
+// takes the fewest nodes that keep it below 2.5e-7 (in 64 bits, R <= 32: 2.32e-7 with 4
+// nodes, at r = 3.9, 1.91e-7 with 6, 2.11e-7 with 8). The erf differences of one source
 // in 32-bit arithmetic are good to about 1e-6 of that peak.
 #pragma once
 
@@ -39,10 +40,9 @@ constexpr int kTableStride = ((R + 2) / 2 | 1) * 2;
 // r above which e_r is (1, 0, 0, ...) in 32 bits: larger values (a zero sigma) are
 // taken as this.
 constexpr float kMaxRSigma = 12.0f;
-// A range of r wider than kNodeRatio is cut into ranges of that ratio, except below
-// kSmallRSigma, where r (R + 1/2) < 0.65 and one range down to 0 interpolates well.
+// A range of r wider than kNodeRatio is cut into ranges of that ratio, small r included:
+// one range from 0.001 to 0.02 would miss the peak of a source at its lower end by 2e-4.
 constexpr float kNodeRatio = 1.6f;
-constexpr float kSmallRSigma = 0.02f;
 
 // Chebyshev nodes +-cos((2p+1) pi / 2J), p < J/2, of J = 4, 6, 8 nodes, and
 // 1 / (2 x_p prod_{q != p} (x_p^2 - x_q^2)). Node 2p is +x_p, node 2p+1
@@ -58,7 +58,7 @@ static __constant__ float kNodeC[kMaxNodes / 2 - 1][kMaxNodes / 2] = {{0.7653669
 // up to kNodeRatio, 8 nodes keep it).
 __device__ __forceinline__ int node_count(float ratio) {
     const float d = ratio - 1.0f;
-    return 4 + 2 * (d > 0.078f) + 2 * (d > 0.285f);
+    return 4 + 2 * (d > 0.075f) + 2 * (d > 0.285f);
 }
 
 // e_r(k) for r >= 1, out of line: few tiles have sources that narrow.
@@ -68,9 +68,11 @@ static __device__ __noinline__ float narrow_spread_weight(float r, int k) {
 }
 
 // e_r(k). For r < 1 the mean of the Gaussian over the unit cell by Gauss-Legendre
-// quadrature (3 points up to r = 0.3, else 5), which keeps the relative accuracy that
-// the difference of two erf values of nearly equal size loses. Its relative error is
-// below 5e-8; that of __expf, 1e-7 at the centre, reaches 1e-6 only where e^-9 is left.
+// quadrature (3 points up to r = 0.3, else 5): the difference of two erf values of nearly
+// equal size loses its leading digits. In exact arithmetic its error is below 4.4e-8 of
+// e_r(0); relative to e_r(k) itself it grows along the tail, to 2.7e-7 at r k = 2.1 and
+// 4.5e-6 at r k = 3 (r = 0.3; 4.1e-7 there with 5 points). __expf adds 1e-7 at the centre
+// and 1e-6 where e^-9 is left.
 __device__ __forceinline__ float spread_weight(float r, int k) {
     if (r >= 1.0f) return narrow_spread_weight(r, k);
     const float c = float(k), r2 = -r * r;
@@ -139,7 +141,7 @@ struct NodeRange {
 __device__ __forceinline__ NodeRange node_range(float from, float lo, float hi) {
     NodeRange n;
     n.from = from;
-    n.top = hi > kNodeRatio * lo ? fminf(hi, fmaxf(kNodeRatio * lo, kSmallRSigma)) : hi;
+    n.top = fminf(hi, kNodeRatio * lo);
     n.to = n.top >= hi ? __int_as_float(0x7f800000) : n.top;
     n.mid = 0.5f * (lo + n.top);
     n.half = 0.5f * (n.top - lo);
