@@ -15,8 +15,6 @@
 #include <map>
 #include <mutex>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "context.h"
@@ -318,24 +316,6 @@ cudaError_t copy_box(void* dst, const void* src, const int dims[3], const int lo
     return cudaMemcpy3DAsync(&p, s);
 }
 
-// Calls f(first, last) for parts of the rows [0, n) of a copy, by up to four threads.
-template <typename F>
-void split_rows(size_t n, size_t bytes, F f) {
-    constexpr size_t kParts = 4, kBytesPerPart = size_t(256) << 10;
-    const size_t cores = std::max(1u, std::thread::hardware_concurrency());
-    const size_t parts = std::max<size_t>(1, std::min({kParts, cores, n, bytes / kBytesPerPart}));
-    std::thread helpers[kParts - 1];
-    size_t started = 1;
-    try {
-        for (; started < parts; ++started)
-            helpers[started - 1] = std::thread(f, n * started / parts, n * (started + 1) / parts);
-    } catch (const std::system_error&) {  // no thread to be had: the parts left are done here
-    }
-    f(size_t(0), n / parts);
-    if (started < parts) f(n * started / parts, n);
-    for (size_t i = 1; i < started; ++i) helpers[i - 1].join();
-}
-
 bool box_empty(const int lo[3], const int hi[3]) { return hi[0] < lo[0] || hi[1] < lo[1] || hi[2] < lo[2]; }
 
 unsigned long long box_bytes(const int lo[3], const int hi[3]) {
@@ -393,38 +373,46 @@ void Context::column_layout(const BeamPlan& P, ColBox& fb, size_t& bevCells, siz
     bytesPerColumn = bevCells * (sizeof(float) + sizeof(unsigned long long)) + voxels * sizeof(double);
 }
 
-// The driver copies a box of pageable memory row by row through its own staging, on one
-// thread. Here the rows go through two page-locked slots, filled or emptied by a few
-// threads while the other slot's transfer runs, and a fresh buffer's page faults are
-// shared between them. One wrapper call on 256 x 256 x 160 voxels (5 MB of CT up, 11.6 MB
-// of dose down): 5.2 -> 3.3 ms, the initial dose's 11.6 MB up (left out for a dose of
-// zeros) included in the former. A water-equivalence volume, contiguous and copied while
-// earlier beams still run, is faster by the driver's copy (383 against 719 us).
+// The driver copies pageable memory through its own staging on one thread, and a box of it
+// row by row. Here it goes through two page-locked slots, filled (past the caches) or
+// emptied by a few threads while the other slot's transfer runs, and a fresh buffer's page
+// faults are shared between them. To the device a slot goes in pieces, so that the first
+// ones are under way while the others are filled. One wrapper call on 256 x 256 x 160 voxels
+// (5 MB of CT up, 11.6 MB of dose down): 3.25 ms with threads started for each slot and
+// ordinary stores, 2.55 ms with these.
+int Context::copy_ring(const void* host, unsigned long long bytes, bool& use) {
+    constexpr unsigned long long kSmall = 1ull << 20;
+    use = false;
+    cudaPointerAttributes at{};
+    const bool pageable = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    if (!pageable || bytes < kSmall) return PBS_OK;
+    if (ring.ensure(kRingSlots * kSlotBytes)) {  // no page-locked memory to be had: the driver's copy
+        cudaGetLastError();
+        set_error("");
+        return PBS_OK;
+    }
+    for (cudaEvent_t& e : ringDone)
+        if (!e) PBS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+    use = true;
+    return PBS_OK;
+}
+
 int Context::copy_host_box(float* dev, float* host, const int dims[3], const int lo[3], const int hi[3], bool toDevice,
                            cudaStream_t s) {
-    constexpr size_t kSlot = size_t(4) << 20;  // bytes
-    constexpr unsigned long long kSmall = 1ull << 20;
-    auto direct = [&]() -> int {
+    const size_t pieces = toDevice ? kSlotPieces : 1, piece = kSlotBytes / pieces;
+    const size_t w = size_t(hi[0] - lo[0] + 1), h = size_t(hi[1] - lo[1] + 1), d = size_t(hi[2] - lo[2] + 1);
+    bool use = false;
+    if (int rc = copy_ring(host, box_bytes(lo, hi), use)) return rc;
+    if (!use || w * 4 > piece) {
         if (toDevice)
             PBS_CUDA(copy_box(dev, host, dims, lo, hi, cudaMemcpyHostToDevice, s), "box H2D");
         else
             PBS_CUDA(copy_box(host, dev, dims, lo, hi, cudaMemcpyDeviceToHost, s), "box D2H");
         return PBS_OK;
-    };
-    const size_t w = size_t(hi[0] - lo[0] + 1), h = size_t(hi[1] - lo[1] + 1), d = size_t(hi[2] - lo[2] + 1);
-    cudaPointerAttributes at{};
-    const bool pageable = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
-    cudaGetLastError();
-    if (!pageable || box_bytes(lo, hi) < kSmall || w * 4 > kSlot) return direct();
-    if (ring.ensure(2 * kSlot)) {
-        cudaGetLastError();
-        set_error("");
-        return direct();
     }
-    for (cudaEvent_t& e : ringDone)
-        if (!e) PBS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
-    // A slot holds whole planes of the box, or rows of one plane.
-    const size_t rows = kSlot / (w * 4), planes = rows / h;
+    // A piece holds whole planes of the box, or rows of one plane.
+    const size_t rows = piece / (w * 4), planes = rows / h;
     const size_t stepY = planes ? h : rows, stepZ = planes ? planes : 1;
     const size_t partsY = (h + stepY - 1) / stepY, parts = partsY * ((d + stepZ - 1) / stepZ);
     struct Part {
@@ -437,22 +425,24 @@ int Context::copy_host_box(float* dev, float* host, const int dims[3], const int
         p.z = i / partsY * stepZ;
         p.h = std::min(stepY, h - p.y);
         p.d = std::min(stepZ, d - p.z);
-        p.slot = static_cast<float*>(ring.ptr) + (i & 1) * (kSlot / 4);
+        p.slot = static_cast<float*>(ring.ptr) + i % (kRingSlots * pieces) * (piece / 4);
         return p;
     };
     auto between_host = [&](const Part& p) {
-        split_rows(p.h * p.d, p.h * p.d * w * 4, [&, p](size_t first, size_t last) {
+        copyThreads.split(p.h * p.d, p.h * p.d * w * 4, [&](size_t first, size_t last) {
             for (size_t r = first; r < last; ++r) {
                 const size_t z = size_t(lo[2]) + p.z + r / p.h, y = size_t(lo[1]) + p.y + r % p.h;
                 float* row = host + (z * dims[1] + y) * dims[0] + lo[0];
                 if (toDevice)
-                    std::memcpy(p.slot + r * w, row, w * 4);
+                    stream_copy(p.slot + r * w, row, w * 4);
                 else
                     std::memcpy(row, p.slot + r * w, w * 4);
             }
         });
     };
-    auto transfer = [&](size_t i, const Part& p) -> int {
+    auto slot_done = [&](size_t i) { return ringDone[i / pieces % kRingSlots]; };
+    auto transfer = [&](size_t i) -> int {
+        const Part p = part(i);
         cudaMemcpy3DParms m = {};
         const cudaPitchedPtr slot = make_cudaPitchedPtr(p.slot, w * 4, w, p.h);
         const cudaPitchedPtr vol = make_cudaPitchedPtr(dev, size_t(dims[0]) * 4, size_t(dims[0]), size_t(dims[1]));
@@ -463,18 +453,17 @@ int Context::copy_host_box(float* dev, float* host, const int dims[3], const int
         m.extent = make_cudaExtent(w * 4, p.h, p.d);
         m.kind = toDevice ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
         PBS_CUDA(cudaMemcpy3DAsync(&m, s), "box copy");
-        PBS_CUDA(cudaEventRecord(ringDone[i & 1], s), "cudaEventRecord");
+        PBS_CUDA(cudaEventRecord(slot_done(i), s), "cudaEventRecord");
         return PBS_OK;
     };
     for (size_t i = 0; i < parts + (toDevice ? 0 : 1); ++i) {
         if (i < parts) {
-            const Part p = part(i);
-            PBS_CUDA(cudaEventSynchronize(ringDone[i & 1]), "cudaEventSynchronize");
-            if (toDevice) between_host(p);
-            if (int rc = transfer(i, p)) return rc;
+            if (i % pieces == 0) PBS_CUDA(cudaEventSynchronize(slot_done(i)), "cudaEventSynchronize");
+            if (toDevice) between_host(part(i));
+            if (int rc = transfer(i)) return rc;
         }
         if (!toDevice && i > 0) {
-            PBS_CUDA(cudaEventSynchronize(ringDone[(i - 1) & 1]), "cudaEventSynchronize");
+            PBS_CUDA(cudaEventSynchronize(slot_done(i - 1)), "cudaEventSynchronize");
             between_host(part(i - 1));
         }
     }
