@@ -470,6 +470,30 @@ int Context::copy_host_box(float* dev, float* host, const int dims[3], const int
     return PBS_OK;
 }
 
+// One call with a water-equivalence volume of 5.2 MB: 268 us, by the driver's copy 392
+// (beams on three contexts in turn).
+int Context::copy_host_floats(float* dev, const float* host, size_t n, cudaStream_t s) {
+    constexpr size_t kPiece = kSlotBytes / kSlotPieces / 4;  // floats
+    bool use = false;
+    if (int rc = copy_ring(host, n * 4, use)) return rc;
+    if (!use) {
+        PBS_CUDA(cudaMemcpyAsync(dev, host, n * 4, cudaMemcpyHostToDevice, s), "H2D");
+        return PBS_OK;
+    }
+    for (size_t i = 0, at = 0; at < n; ++i, at += kPiece) {
+        const size_t m = std::min(kPiece, n - at);
+        float* slot = static_cast<float*>(ring.ptr) + i % (kRingSlots * kSlotPieces) * kPiece;
+        const cudaEvent_t done = ringDone[i / kSlotPieces % kRingSlots];
+        if (i % kSlotPieces == 0) PBS_CUDA(cudaEventSynchronize(done), "cudaEventSynchronize");
+        copyThreads.split(m, m * 4, [&](size_t first, size_t last) {
+            stream_copy(slot + first, host + at + first, (last - first) * 4);
+        });
+        PBS_CUDA(cudaMemcpyAsync(dev + at, slot, m * 4, cudaMemcpyHostToDevice, s), "H2D");
+        PBS_CUDA(cudaEventRecord(done, s), "cudaEventRecord");
+    }
+    return PBS_OK;
+}
+
 int Context::set_ct_region(const float* data, const GridDesc& g, const int lo[3], const int hi[3]) {
     PBS_CUDA(cudaSetDevice(device), "cudaSetDevice");
     if (!data || g.dims[0] <= 0 || g.dims[1] <= 0 || g.dims[2] <= 0 ||
@@ -1389,8 +1413,7 @@ int Context::run_beam(const PbsBeamDesc& b, int nuclear, const AdjointArgs* adj,
         // Water-equivalence import: the exporter's depths replace the CT trace.
         const size_t weqN = size_t(P.weqNx) * P.weqNy * P.weqSteps;
         if ((rc = weqBody.ensure(weqN * 4))) return rc;
-        PBS_CUDA(cudaMemcpyAsync(weqBody.ptr, b.water_equivalence + 9, weqN * 4, cudaMemcpyHostToDevice, stream),
-                 "WEQ H2D");
+        if ((rc = copy_host_floats(static_cast<float*>(weqBody.ptr), b.water_equivalence + 9, weqN, stream))) return rc;
         copiedH2D += weqN * 4;
         PBS_CUDA(launch_weq_trace(g, luts, static_cast<const float*>(weqBody.ptr), P.weqNx, P.weqNy, P.weqSteps,
                                   P.weqActiveSteps, P.weqStepMm, P.cpbCorner.x, P.cpbCorner.y, P.cpbRes.x, P.cpbRes.y,

@@ -236,6 +236,8 @@ struct Context {
     // order, as cudaMemcpyAsync).
     int copy_host_box(float* dev, float* host, const int dims[3], const int lo[3], const int hi[3], bool toDevice,
                       cudaStream_t s);
+    // Copies n floats up, in the same way.
+    int copy_host_floats(float* dev, const float* host, size_t n, cudaStream_t s);
     int convert_ct(int type, const GridDesc& g);
     // HU+1000 conversion of `n` device floats in place, on the context stream.
     // With dims, only the inclusive box [lo, hi] of the [dims.z][dims.y][dims.x] CT.

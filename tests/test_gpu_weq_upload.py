@@ -1,0 +1,29 @@
+"""Water-equivalence volumes of 1.7, 6.6 and 10 MB: from pageable memory they go up in pieces
+through the page-locked slots (one piece, the slots' last one ragged, and more pieces than
+the slots hold), from page-locked memory in one copy. The dose is the same bits, also for a
+second volume that follows while the first beam may still run."""
+import numpy as np
+import pytest
+import torch
+
+from _parity import run_gpu
+from subsecondpbs_b200 import phantoms
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ray_mm", [1.0, 0.5, 0.4])
+def test_pageable_and_page_locked_volumes(ray_mm):
+    case = phantoms.weq_case(ray_mm=ray_mm, n_layers=2)
+    first = np.array(case["beam"]["water_equivalence"], np.float32)
+    second = first.copy()
+    second[9:] *= 0.9
+    assert first.nbytes > 1 << 20
+    doses = []
+    for locked in (False, True):
+        keep = [torch.from_numpy(v).pin_memory() if locked else torch.from_numpy(v.copy()) for v in (first, second)]
+        eng = run_gpu(case, beams=[dict(case["beam"], water_equivalence=k.numpy()) for k in keep], keep_debug=False)
+        doses.append(eng.read_dose())
+        eng.close()
+    assert doses[0].max() > 0.0
+    assert np.array_equal(doses[0], doses[1])
