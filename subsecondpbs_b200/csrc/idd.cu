@@ -795,16 +795,11 @@ __global__ void nuc_codes_kernel(BeamGeomDev gn, int layer0, int nLayers, const 
 
 }  // namespace
 
-namespace {
 // Table rows, per-step widths and volumes, and the warps' partials of every step.
-size_t idd_smem(const BeamGeomDev& g, size_t tableFloats) {
+size_t idd_smem_bytes(const BeamGeomDev& g, const LutsDev& luts) {
+    const size_t tableFloats = static_cast<size_t>(luts.nS) * (g.nucOn ? 3 : 1) + 2;
     return (tableFloats + 2 * static_cast<size_t>(g.steps)) * sizeof(float) +
            static_cast<size_t>(g.steps) * 8 * (sizeof(float) + sizeof(unsigned));
-}
-}  // namespace
-
-size_t idd_smem_bytes(const BeamGeomDev& g, const LutsDev& luts) {
-    return idd_smem(g, static_cast<size_t>(luts.nS) * (g.nucOn ? 3 : 1) + luts.nRrl);
 }
 
 cudaError_t launch_nuc_prepare(const BeamGeomDev& gn, int nLayers, float2* sources, cudaStream_t s) {
@@ -830,7 +825,7 @@ cudaError_t launch_idd(const BeamGeomDev& g, const LutsDev& luts, int layer0, in
                        float2* nucSources, cudaStream_t s) {
     dim3 grid(g.tilesX, g.tilesY, nLayers);
     dim3 block(32, 8);
-    const size_t smem = idd_smem(g, static_cast<size_t>(luts.nS) * (g.nucOn ? 3 : 1) + 2);
+    const size_t smem = idd_smem_bytes(g, luts);
     auto k = g.nucOn ? (g.profileMode ? idd_kernel<true, true> : idd_kernel<true, false>)
                      : (g.profileMode ? idd_kernel<false, true> : idd_kernel<false, false>);
     cudaError_t e = set_smem_limit(reinterpret_cast<const void*>(k), smem);
