@@ -239,7 +239,7 @@ PBS_API int pbs_subsecond_wrapper(const float* ct_data, const int ct_dims[3], co
                           int gpu_id, int nuclear_correction, int verbose);
 
 /* The same for a dose_data that holds zeros on entry: it is written, not read.
- * *finite is set to whether every dose value is finite. */
+ * *finite is set, where the call succeeds, to whether every dose value is finite. */
 PBS_API int pbs_subsecond_wrapper_zeroed(const float* ct_data, const int ct_dims[3], const float ct_resolution[3],
                           const float ct_corner[3], float* dose_data, const int dose_dims[3],
                           const float dose_resolution[3], const float dose_corner[3],
