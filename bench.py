@@ -495,6 +495,80 @@ def _reference_gpu(local: int, case: dict, our_e2e_ms: float) -> dict | None:
                                                       "same inputs (voxels above 10 % of Dmax)")}
 
 
+def _batched_radius(hist):
+    """Radius that a tile of each bucket is superposed with: from the widest radius down, a
+    batch takes radii until it holds 16 tiles (complete_superposition.cu:476-483); the
+    overflow bucket counts as radius 32."""
+    hist = [int(v) for v in hist]
+    top = max((r for r, v in enumerate(hist) if v), default=0)
+    out, batch, held = list(range(len(hist))), min(top, 32), 0
+    for r in range(min(top, 32), 0, -1):
+        out[r] = batch
+        held += hist[r] + (hist[33] if r == 32 else 0)
+        if held >= 16:
+            batch, held = r - 1, 0
+    out[33] = out[32]
+    return np.array(out)
+
+
+def _superpose_work(local, case, beam):
+    """FP32 operations (2 per FMA) that the superposition of this beam executes: its items
+    are the layers of one tile and step with one radius R; an item takes J = 4, 6 or 8 nodes
+    per range of rSigma (csrc/node_spread.cuh) and does for each range
+      weights: 256 sources per layer, their position and the products and sums of J / 2 pairs;
+      rows:    8 J rows of 32 sources, 2R + 1 taps;
+      columns: J x (32 + 2R) columns of 8 sources, 2R + 1 taps.
+    From the sources, radii and codes of a debug run of the same beam."""
+    from subsecondpbs_b200 import _lib as L
+    from subsecondpbs_b200.cudaCalDoseRTD import DoseEngine
+
+    eng = DoseEngine(local, keep_debug=True)
+    eng.set_energy(case["energy"])
+    eng.set_ct(case["ct"], case["ct_dims"], case["ct_resolution"], case["ct_corner"])
+    eng.set_dose_grid(case["dose_dims"], case["dose_resolution"], case["dose_corner"])
+    eng.add_beam(beam)
+    eng.synchronize()
+    st = eng.beam_stats()
+    S, (X, Y) = st["tracer_steps"], st["superp_dims"]
+    P = S * (Y // 8) * (X // 32)
+    keys, los, his = [], [], []
+    for layer in range(st["num_layers"]):
+        code = eng.debug(L.PBS_DBG_TILE_BINS, layer, (P,), np.uint8)
+        at = np.nonzero(((code & 0x80) != 0) & (code != 0xFF))[0]
+        radius = _batched_radius(eng.layer_stats(layer)["tile_rad_counts"])[code[at] & 0x3F]
+
+        def tiles(which):
+            v = eng.debug(which, layer, (S, Y, X)).reshape(S, Y // 8, 8, X // 32, 32).transpose(0, 1, 3, 2, 4)
+            return v.reshape(P, 256)[at]
+
+        dose, r = tiles(L.PBS_DBG_IDD) > 0.0, tiles(L.PBS_DBG_RSIGMA)
+        keys.append(((layer // 32) * P + at) * 33 + radius)
+        los.append(np.where(dose, r, np.inf).min(axis=1))
+        his.append(np.where(dose, r, 0.0).max(axis=1))
+    eng.close()
+    item, which, layers = np.unique(np.concatenate(keys), return_inverse=True, return_counts=True)
+    lo, hi = np.full(item.size, np.inf), np.zeros(item.size)
+    np.minimum.at(lo, which, np.concatenate(los))
+    np.maximum.at(hi, which, np.concatenate(his))
+    lo, hi = np.clip(lo, 1e-12, 12.0), np.clip(hi, 1e-12, 12.0)
+    R = (item % 33).astype(np.float64)
+    flops = np.zeros(item.size)
+    while True:
+        left = hi > 0.0
+        if not left.any():
+            return float(flops.sum()), int(item.size)
+        top = np.minimum(hi, 1.6 * lo)
+        d = top / lo - 1.0
+        J = 4 + 2 * (d > 0.075) + 2 * (d > 0.285)
+        # Position 2, its square 1, pair factors J/2, their products 0, 3 or 6, and four per pair.
+        source = 3 + J / 2 + np.where(J == 4, 0, np.where(J == 6, 3, 6)) + 2 * J
+        weights = np.where(J == 8, 2, 1) * layers * 256 * source  # 8 nodes go in two halves
+        taps = 2 * R + 1
+        flops += np.where(left, weights + 2 * 8 * J * taps * (32 + 32 + 2 * R), 0.0)
+        hi = np.where(top >= hi, 0.0, hi)
+        lo = top
+
+
 def run_ours(args):
     import ctypes as C
 
@@ -629,10 +703,11 @@ def run_ours(args):
         dist.destroy_process_group()
         return 0
 
-    # Roofline of the dominant kernel (superposition, FP32 pipe) and per-stage HBM figures.
+    # Roofline of the dominant kernel (superposition: the FP32 operations that it executes
+    # against the FP32 pipe's rate) and per-stage HBM figures.
     sup_ms = float(np.mean(stage_acc["superpose"]))
-    fma = float(stats["superpose_fma"])
-    achieved = 2.0 * fma / (sup_ms * 1e-3) / 1e12
+    executed, items = _superpose_work(local, case, beam)
+    achieved = executed / (sup_ms * 1e-3) / 1e12
     traffic = None
     tfile = ROOT / "profiles" / "superpose_traffic.json"
     if tfile.exists():
@@ -653,8 +728,8 @@ def run_ours(args):
     box = int(np.prod([max(tb[1][i] - tb[0][i] + 1, 0) for i in range(3)]))
     stage_ms = {k: float(np.mean(v)) for k, v in stage_acc.items()}
     stage_bytes = {
-        "trace": 8.0 * rays * S,                      # density + WEPL written
-        "idd": 16.0 * pad * idd_steps,                # density + WEPL read, IDD + sigma written
+        "trace": 12.0 * rays * S,                     # density, density x radiation length, WEPL written
+        "idd": 20.0 * pad * idd_steps,                # those read, IDD + sigma written (tiles without a live ray are not)
         "transfer": 16.0 * box,                       # FP64 dose read-modify-write over the box
     }
     roof_stages = []
@@ -691,7 +766,7 @@ def run_ours(args):
 
         precision = dict(prec.report(bench_dose, ref_dose, case["dose_resolution"]),
                          reference="FP64 oracle, same inputs", arithmetic="FP32 rays/superposition, "
-                         "int32 fixed-point tile footprints, Kahan WEPL, FP64 dose accumulation")
+                         "int64 fixed-point BEV, Kahan WEPL, FP64 dose accumulation")
     if carbon is not None and not args.no_cpu_baseline:
         carbon["precision"] = _carbon_precision(carbon_case, carbon_dose)
     del carbon_dose, carbon_case
@@ -712,10 +787,11 @@ def run_ours(args):
         "config": dict(CONFIG),
         "run": {"beams_per_step": world, "parallelism": f"beam-sharded x{world}", "accumulation": "FP64 dose grid",
                 "total_ms_incl_flush": total_ms},
-        "roofline": {"kernel": "superpose_kernel", "bound": "fp32", "achieved": round(achieved, 3),
+        "roofline": {"kernel": "superpose_kernel", "bound": "issue", "achieved": round(achieved, 3),
                      "peak": round(peak_fp32, 3), "unit": "TFLOP/s", "frac": round(achieved / peak_fp32, 4),
                      "traffic": traffic, "peak_source": "in-run FFMA microbenchmark (FP32 pipe, no tensor cores)",
-                     "algorithmic_flops": 2.0 * fma},
+                     "executed_flops": executed, "items": items,
+                     "reference_equivalent_flops": 2.0 * stats["superpose_fma"]},
         "roofline_stages": roof_stages,
         "stages_ms": stage_ms,
         "cpu_baseline": cpu,
