@@ -24,9 +24,10 @@ namespace {
 
 // T^T: every dose voxel of the transfer box spreads its gradient over the eight
 // BEV texels its forward sample interpolated (bev_sample in transfer.cu), with the
-// same weights. The forward adds a sample only where it is positive; a BEV sample
-// is a sum of non-negative terms, so it is zero only where every texel's
-// coefficient is zero and the linear transpose is exact.
+// same weights. The forward adds a sample only where it is positive, and BEV cells are
+// not negative: a sum of interpolated footprints that ends below zero is taken as zero.
+// The transpose ignores that, so the two match to within the interpolation's residue,
+// 2.5e-7 of the peaks of the sources that reach the cell (node_spread.cuh).
 // A lane takes one dose column and 8 consecutive z (walk_box; the box is known only on
 // the device).
 __global__ void __launch_bounds__(256)
