@@ -74,7 +74,7 @@ size_t idd_smem_bytes(const BeamGeomDev& g, const LutsDev& luts);
 // fillIddAndSigmaKernel (src/algorithms/idd_sigma.cu:46-259) fused with the
 // per-tile radius reduction of tileRadCalc (complete_superposition.cu:198-255).
 // With g.nucOn it also writes the nuclear halo IDD and sigma of the rays under a
-// halo lattice cell (rayToNuc: [rays] -> cell or -1) into [layer][step][nucY][nucX].
+// halo lattice cell (rayToNuc: [rays] -> cell or -1), by layer and step, tile by tile.
 cudaError_t launch_idd(const BeamGeomDev& g, const LutsDev& luts, int layer0, int nLayers, const float2* material,
                        const float* wepl, const int* firstInside, const int* firstOutside, const float* rayW,
                        const LayerParamsDev* lp, LayerStateDev* ls, const BeamStateDev* beam, float2* sources,
@@ -84,10 +84,9 @@ cudaError_t launch_idd(const BeamGeomDev& g, const LutsDev& luts, int layer0, in
 // the radius-sorted work list of live tiles. With primaryLs/primaryBeam set it
 // plans the nuclear halo grid `g` instead (no merge: a radius above 32 sets error
 // flag 4). A list item is {layers, tile, step, radius | group << 8}: a bit per layer of
-// the group of 32 chunk layers from `group` on. `merged` selects the forward
-// superposition's list (all layers of a group whose tile has one radius at one step)
-// over the one-layer items the adjoint gathers from, with each layer's box of live
-// cells.
+// the group of 32 chunk layers from `group` on. `merged` selects the list of the
+// superposition and its adjoint (all layers of a group whose tile has one radius at one
+// step) over the influence columns' one-layer items, with each layer's box of live cells.
 cudaError_t launch_bin_plan(const BeamGeomDev& g, int layer0, int nLayers, const uint8_t* codes, LayerStateDev* ls,
                             BeamStateDev* beam, int4* work, int workCapacity, bool merged,
                             const LayerStateDev* primaryLs, const BeamStateDev* primaryBeam, cudaStream_t s);

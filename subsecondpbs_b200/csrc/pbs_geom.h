@@ -29,11 +29,11 @@ namespace pbs {
 
 constexpr int kTileX = 32;               // SUPERP_TILE_X, include/core/Macro.cuh:65
 constexpr int kTileY = 8;                // SUPERP_TILE_Y, include/core/Macro.cuh:66
-// The IDD and rSigma of a layer are stored step by step and tile by tile, the 256 sources
-// of a tile in rows: a tile's sources are one contiguous KB.
+// The (IDD, rSigma) pairs of a layer are stored step by step and tile by tile, the 256
+// sources of a tile in rows: a tile's sources are 2 KB without a gap.
 constexpr int kTileSources = kTileX * kTileY;
 constexpr int kMaxR = 32;                // MAX_SUPERP_RADIUS, include/core/Macro.cuh:64
-constexpr int kSplitR = 15;              // radii <= kSplitR run in the medium and narrow superposition instances
+constexpr int kSplitR = 15;              // radii <= kSplitR run in the narrow superposition instance
 constexpr int kMinTilesInBatch = 16;     // MIN_TILES_IN_BATCH, include/core/Macro.cuh:67
 constexpr float kBpDepthCutoff = 1.05f;  // BP_DEPTH_CUTOFF, include/core/Macro.cuh:46
 

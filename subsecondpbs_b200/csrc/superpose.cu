@@ -423,7 +423,6 @@ superpose_kernel(BeamGeomDev g, const float2* __restrict__ sources, const unsign
 // previous superposition instance).
 template <int RLo, int RHi, int Warps, int MinBlocks>
 cudaError_t launch_range(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange, const int4* work,
-                        
                          BeamStateDev* beam, unsigned long long* bev, int shiftOffset, int numSMs, bool overlap,
                          size_t layerBevStride, cudaStream_t s) {
     auto k = superpose_kernel<RLo, RHi, Warps, MinBlocks>;
@@ -487,7 +486,6 @@ namespace {
 
 // The three instances over `work` (items sorted by range: the wide radii first).
 cudaError_t launch_instances(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange, const int4* work,
-                            
                              BeamStateDev* beam, unsigned long long* bevFixed, int shiftOffset, int numSMs,
                              size_t layerBevStride, cudaStream_t s) {
     cudaError_t e = launch_range<kSplitWide + 1, kMaxR, kWidestWarps, kWidestBlocks>(
@@ -550,7 +548,6 @@ __global__ void __launch_bounds__(256) column_fixed_to_float_kernel(BeamGeomDev 
 }  // namespace
 
 cudaError_t launch_superpose(const BeamGeomDev& g, const float2* sources, const unsigned* tileRange, const int4* work,
-                            
                              BeamStateDev* beam, float* bev, unsigned long long* bevFixed, int shiftOffset, int numSMs,
                              cudaStream_t s) {
     cudaError_t e = launch_instances(g, sources, tileRange, work, beam, bevFixed, shiftOffset, numSMs, 0, s);
