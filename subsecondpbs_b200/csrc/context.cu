@@ -97,9 +97,7 @@ Context::~Context() {
     staging.release();
     errHost.release();
     if (copyStream) cudaStreamSynchronize(copyStream);
-    ring.release();
-    for (cudaEvent_t e : ringDone)
-        if (e) cudaEventDestroy(e);
+    ringUser.end();
     if (stagingEvent) cudaEventDestroy(stagingEvent);
     if (copyStart) cudaEventDestroy(copyStart);
     if (doseCopied) cudaEventDestroy(doseCopied);
@@ -380,37 +378,28 @@ void Context::column_layout(const BeamPlan& P, ColBox& fb, size_t& bevCells, siz
 // ones are under way while the others are filled. One wrapper call on 256 x 256 x 160 voxels
 // (5 MB of CT up, 11.6 MB of dose down): 3.25 ms with threads started for each slot and
 // ordinary stores, 2.55 ms with these.
-int Context::copy_ring(const void* host, unsigned long long bytes, bool& use) {
-    constexpr unsigned long long kSmall = 1ull << 20;
-    use = false;
+static bool through_ring(const void* host, unsigned long long bytes) {
     cudaPointerAttributes at{};
     const bool pageable = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    if (!pageable || bytes < kSmall) return PBS_OK;
-    if (ring.ensure(kRingSlots * kSlotBytes)) {  // no page-locked memory to be had: the driver's copy
-        cudaGetLastError();
-        set_error("");
-        return PBS_OK;
-    }
-    for (cudaEvent_t& e : ringDone)
-        if (!e) PBS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
-    use = true;
-    return PBS_OK;
+    return pageable && bytes >= 1ull << 20;
 }
 
 int Context::copy_host_box(float* dev, float* host, const int dims[3], const int lo[3], const int hi[3], bool toDevice,
                            cudaStream_t s) {
-    const size_t pieces = toDevice ? kSlotPieces : 1, piece = kSlotBytes / pieces;
-    const size_t w = size_t(hi[0] - lo[0] + 1), h = size_t(hi[1] - lo[1] + 1), d = size_t(hi[2] - lo[2] + 1);
-    bool use = false;
-    if (int rc = copy_ring(host, box_bytes(lo, hi), use)) return rc;
-    if (!use || w * 4 > piece) {
+    auto direct = [&]() -> int {
         if (toDevice)
             PBS_CUDA(copy_box(dev, host, dims, lo, hi, cudaMemcpyHostToDevice, s), "box H2D");
         else
             PBS_CUDA(copy_box(host, dev, dims, lo, hi, cudaMemcpyDeviceToHost, s), "box D2H");
         return PBS_OK;
-    }
+    };
+    const size_t pieces = toDevice ? CopyRing::kPieces : 1, piece = CopyRing::kSlotBytes / pieces;
+    const size_t w = size_t(hi[0] - lo[0] + 1), h = size_t(hi[1] - lo[1] + 1), d = size_t(hi[2] - lo[2] + 1);
+    if (!through_ring(host, box_bytes(lo, hi)) || w * 4 > piece) return direct();
+    ringUser.begin(device);
+    CopyRingLoan ring(device, s, false);
+    if (!ring) return direct();
     // A piece holds whole planes of the box, or rows of one plane.
     const size_t rows = piece / (w * 4), planes = rows / h;
     const size_t stepY = planes ? h : rows, stepZ = planes ? planes : 1;
@@ -425,11 +414,11 @@ int Context::copy_host_box(float* dev, float* host, const int dims[3], const int
         p.z = i / partsY * stepZ;
         p.h = std::min(stepY, h - p.y);
         p.d = std::min(stepZ, d - p.z);
-        p.slot = static_cast<float*>(ring.ptr) + i % (kRingSlots * pieces) * (piece / 4);
+        p.slot = ring->mem + i % (CopyRing::kSlots * pieces) * (piece / 4);
         return p;
     };
     auto between_host = [&](const Part& p) {
-        copyThreads.split(p.h * p.d, p.h * p.d * w * 4, [&](size_t first, size_t last) {
+        ring->threads.split(p.h * p.d, p.h * p.d * w * 4, [&](size_t first, size_t last) {
             for (size_t r = first; r < last; ++r) {
                 const size_t z = size_t(lo[2]) + p.z + r / p.h, y = size_t(lo[1]) + p.y + r % p.h;
                 float* row = host + (z * dims[1] + y) * dims[0] + lo[0];
@@ -440,7 +429,7 @@ int Context::copy_host_box(float* dev, float* host, const int dims[3], const int
             }
         });
     };
-    auto slot_done = [&](size_t i) { return ringDone[i / pieces % kRingSlots]; };
+    auto slot_done = [&](size_t i) { return ring->done[i / pieces % CopyRing::kSlots]; };
     auto transfer = [&](size_t i) -> int {
         const Part p = part(i);
         cudaMemcpy3DParms m = {};
@@ -473,19 +462,21 @@ int Context::copy_host_box(float* dev, float* host, const int dims[3], const int
 // One call with a water-equivalence volume of 5.2 MB: 268 us, by the driver's copy 392
 // (beams on three contexts in turn).
 int Context::copy_host_floats(float* dev, const float* host, size_t n, cudaStream_t s) {
-    constexpr size_t kPiece = kSlotBytes / kSlotPieces / 4;  // floats
-    bool use = false;
-    if (int rc = copy_ring(host, n * 4, use)) return rc;
-    if (!use) {
+    constexpr size_t kPiece = CopyRing::kSlotBytes / CopyRing::kPieces / 4;  // floats
+    auto direct = [&]() -> int {
         PBS_CUDA(cudaMemcpyAsync(dev, host, n * 4, cudaMemcpyHostToDevice, s), "H2D");
         return PBS_OK;
-    }
+    };
+    if (!through_ring(host, n * 4)) return direct();
+    ringUser.begin(device);
+    CopyRingLoan ring(device, s, true);
+    if (!ring) return direct();
     for (size_t i = 0, at = 0; at < n; ++i, at += kPiece) {
         const size_t m = std::min(kPiece, n - at);
-        float* slot = static_cast<float*>(ring.ptr) + i % (kRingSlots * kSlotPieces) * kPiece;
-        const cudaEvent_t done = ringDone[i / kSlotPieces % kRingSlots];
-        if (i % kSlotPieces == 0) PBS_CUDA(cudaEventSynchronize(done), "cudaEventSynchronize");
-        copyThreads.split(m, m * 4, [&](size_t first, size_t last) {
+        float* slot = ring->mem + i % (CopyRing::kSlots * CopyRing::kPieces) * kPiece;
+        const cudaEvent_t done = ring->done[i / CopyRing::kPieces % CopyRing::kSlots];
+        if (i % CopyRing::kPieces == 0) PBS_CUDA(cudaEventSynchronize(done), "cudaEventSynchronize");
+        ring->threads.split(m, m * 4, [&](size_t first, size_t last) {
             stream_copy(slot + first, host + at + first, (last - first) * 4);
         });
         PBS_CUDA(cudaMemcpyAsync(dev + at, slot, m * 4, cudaMemcpyHostToDevice, s), "H2D");

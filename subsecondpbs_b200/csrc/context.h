@@ -6,7 +6,7 @@
 #include <string>
 #include <vector>
 
-#include "copy_threads.h"
+#include "copy_ring.h"
 #include "pbs_types.h"
 #include "plan.h"
 
@@ -182,12 +182,7 @@ struct Context {
     bool colClean = false;
 
     PinnedBuf staging, errHost;
-    // Ring of two page-locked slots for copies of pageable host volumes, and the threads
-    // that fill and empty them (copy_ring).
-    static constexpr size_t kRingSlots = 2, kSlotBytes = size_t(4) << 20, kSlotPieces = 2;
-    PinnedBuf ring;
-    cudaEvent_t ringDone[kRingSlots] = {};
-    CopyThreads copyThreads;
+    CopyRingUser ringUser;  // copies of pageable host volumes
     cudaEvent_t stagingEvent = nullptr;
     cudaEvent_t ev[8] = {};
 
@@ -229,8 +224,6 @@ struct Context {
     int reset_dose_region(const float* init, const int lo[3], const int hi[3]);
     // `finite` (may be null): whether every value read is finite.
     int read_dose_region(float* out, const int lo[3], const int hi[3], int* finite = nullptr);
-    // Whether a copy of `bytes` from or to `host` goes through the ring, which is made ready.
-    int copy_ring(const void* host, unsigned long long bytes, bool& use);
     // Copies the box [lo, hi] between [Z][Y][X] float volumes of `dims` in device and
     // host memory. Returns with the host side read or written (page-locked: in stream
     // order, as cudaMemcpyAsync).
