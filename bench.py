@@ -518,7 +518,9 @@ def _superpose_work(local, case, beam):
       weights: 256 sources per layer, their position and the products and sums of J / 2 pairs;
       rows:    8 J rows of 32 sources, 2R + 1 taps;
       columns: J x (32 + 2R) columns of 8 sources, 2R + 1 taps.
-    From the sources, radii and codes of a debug run of the same beam."""
+    From the sources, radii and codes of a debug run of the same beam. Returns them, the
+    items, and the (ray, step, layer) triples that the IDD walk takes: all of a tile from the
+    beam's first step to the tile's last one with dose."""
     from subsecondpbs_b200 import _lib as L
     from subsecondpbs_b200.cudaCalDoseRTD import DoseEngine
 
@@ -531,11 +533,14 @@ def _superpose_work(local, case, beam):
     st = eng.beam_stats()
     S, (X, Y) = st["tracer_steps"], st["superp_dims"]
     P = S * (Y // 8) * (X // 32)
-    keys, los, his = [], [], []
+    keys, los, his, walked = [], [], [], 0
     for layer in range(st["num_layers"]):
         code = eng.debug(L.PBS_DBG_TILE_BINS, layer, (P,), np.uint8)
         at = np.nonzero(((code & 0x80) != 0) & (code != 0xFF))[0]
         radius = _batched_radius(eng.layer_stats(layer)["tile_rad_counts"])[code[at] & 0x3F]
+        last = np.full(P // S, st["first_inside"] - 1)
+        np.maximum.at(last, at % (P // S), at // (P // S))
+        walked += 256 * int((last - st["first_inside"] + 1).sum())
 
         def tiles(which):
             v = eng.debug(which, layer, (S, Y, X)).reshape(S, Y // 8, 8, X // 32, 32).transpose(0, 1, 3, 2, 4)
@@ -556,7 +561,7 @@ def _superpose_work(local, case, beam):
     while True:
         left = hi > 0.0
         if not left.any():
-            return float(flops.sum()), int(item.size)
+            return float(flops.sum()), int(item.size), walked
         top = np.minimum(hi, 1.6 * lo)
         d = top / lo - 1.0
         J = 4 + 2 * (d > 0.075) + 2 * (d > 0.285)
@@ -706,7 +711,7 @@ def run_ours(args):
     # Roofline of the dominant kernel (superposition: the FP32 operations that it executes
     # against the FP32 pipe's rate) and per-stage HBM figures.
     sup_ms = float(np.mean(stage_acc["superpose"]))
-    executed, items = _superpose_work(local, case, beam)
+    executed, items, walked = _superpose_work(local, case, beam)
     achieved = executed / (sup_ms * 1e-3) / 1e12
     traffic = None
     tfile = ROOT / "profiles" / "superpose_traffic.json"
@@ -720,23 +725,22 @@ def run_ours(args):
     hbm_source = ("MEASURED_PEAKS.json hbm_gbs (measured copy bandwidth)" if "hbm_gbs" in peaks
                   else "fallback: 6.65 TB/s, an earlier copy-bandwidth measurement on this pool")
     rays = stats["ray_dims"][0] * stats["ray_dims"][1]
-    pad = stats["superp_dims"][0] * stats["superp_dims"][1]
     S = stats["tracer_steps"]
-    first = stats["first_inside"]
-    idd_steps = sum(max(eng.layer_stats(l)["after_last_step"] - first, 0) for l in range(stats["num_layers"]))
     tb = stats["transfer_start"], stats["transfer_max"]
     box = int(np.prod([max(tb[1][i] - tb[0][i] + 1, 0) for i in range(3)]))
     stage_ms = {k: float(np.mean(v)) for k, v in stage_acc.items()}
     stage_bytes = {
         "trace": 12.0 * rays * S,                     # density, density x radiation length, WEPL written
-        "idd": 20.0 * pad * idd_steps,                # those read, IDD + sigma written (tiles without a live ray are not)
+        "idd": 20.0 * walked,                         # those read, IDD + sigma written
         "transfer": 16.0 * box,                       # FP64 dose read-modify-write over the box
     }
+    # What holds each back from that rate (profiles/).
+    stage_bound = {"trace": "latency", "idd": "issue", "transfer": "latency"}
     roof_stages = []
     for k, b in stage_bytes.items():
         if stage_ms[k] > 0:
             gbs = b / (stage_ms[k] * 1e-3) / 1e9
-            roof_stages.append({"stage": k, "bound": "hbm", "achieved": round(gbs, 1), "peak": hbm_peak,
+            roof_stages.append({"stage": k, "bound": stage_bound[k], "achieved": round(gbs, 1), "peak": hbm_peak,
                                 "unit": "GB/s", "frac": round(gbs / hbm_peak, 4), "algorithmic_bytes": b,
                                 "peak_source": hbm_source})
 
