@@ -54,3 +54,33 @@ def test_slots_shared_by_two_contexts():
         e.close()
     assert np.array_equal(want[0], got[0]) and np.array_equal(want[1], got[1])
     assert not np.array_equal(want[0], want[1])
+
+
+def test_slots_shared_by_threads():
+    """Six contexts on six threads, more than there are slots to lend."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    case = phantoms.weq_case(ray_mm=0.5, n_layers=2)
+    base = np.array(case["beam"]["water_equivalence"], np.float32)
+
+    def beam(k):
+        v = base.copy()
+        v[9:] *= np.float32(1.0 - 0.02 * k)
+        return dict(case["beam"], water_equivalence=v)
+
+    def work(k):
+        eng = run_gpu(case, beams=[beam(k)], keep_debug=False)
+        first = eng.read_dose()
+        prepared = eng.prepare_beam(beam(k))
+        for _ in range(15):
+            eng.reset_dose()
+            eng.add_beam(prepared)
+        last = eng.read_dose()
+        eng.close()
+        return first, last
+
+    alone = [work(k)[0] for k in range(6)]
+    with ThreadPoolExecutor(6) as pool:
+        got = list(pool.map(work, range(6)))
+    for want, (first, last) in zip(alone, got):
+        assert np.array_equal(want, first) and np.array_equal(want, last)
